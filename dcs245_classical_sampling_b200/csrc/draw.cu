@@ -14,7 +14,7 @@
 //      |S_i - P_i| <= gamma_{i} P_i (Higham, Accuracy and Stability, Sec. 4.2), so if u lies
 //      outside the error intervals of both bin edges, numpy's index is the same index.
 //      Otherwise the block is flagged as a tie and an exact sequential FP64 pass (the same
-//      operation order as numpy's cumsum) decides — on the device, without host sync.  On
+//      operation order as numpy's cumsum, evaluated through integer maps) decides, without host sync.  On
 //      request (DCS_DRAW_SEQUENTIAL) that pass runs for every block, so that the reported CDF
 //      values are numpy's bit for bit (the production record rows derive a grid count from them);
 //   5. the 53-bit grid total-variation diagnostic of the reference.
@@ -68,35 +68,59 @@ constexpr int kPer = kChunk / kThreads;
 
 struct BlockState {  // per block scratch (device)
     dd total;
-    double total_plain;
     int64_t chunk;
     int32_t status;
-    int32_t nonfinite;
+    int32_t pad;
 };
 
-// sequential pass: one checkpoint (the running FP64 sum before the group) per 32 elements
-constexpr int kSeqLog = 5;
-__host__ __device__ constexpr size_t seq_groups(size_t n) { return (n + 31) >> kSeqLog; }
+// The sequential CDF as integer maps.  While the running FP64 sum S stays in one binade [2^e, 2^(e+1)) it
+// is k q with q = 2^(e-52), and S <- fl(S + w) adds to k a whole number that depends on w and, only
+// where w / q ends in exactly one half (ties go to even), on the parity of k.  So any stretch of
+// additions inside one binade is a map (parity of k) -> increment of k, two maps in a row are again
+// such a map, and stretches are composed in parallel, exactly.  A stretch is a sub-chunk of kSub elements
+// and a chunk; S of its ends is known beforehand to (n + 16) 2^-52 relative from the compensated
+// prefix sums (Higham, Accuracy and Stability, Sec. 4.2), which decides whether it lies in one binade.
+constexpr int kSub = 128;                       // elements per sub-chunk: 16 threads of kPer
+constexpr int kSubs = kChunk / kSub;            // sub-chunks per chunk
+constexpr int kSubThreads = kSub / kPer;
+constexpr int32_t kMapWalk = INT32_MIN;         // crosses (or may cross) a binade: add its weights one by one
+constexpr int32_t kMapNone = INT32_MIN + 1;     // all weights are zero: S does not change
+struct SeqMap {
+    long long d0, d1;  // increment of k for even / odd k
+    int32_t e;         // the binade's exponent, kMapWalk or kMapNone
+    int32_t pad;
+};
+struct SeqChunk {
+    SeqMap map;
+    double start;      // S before the chunk
+};
 
 // layout of the scratch area
 struct Layout {
-    size_t w, chunk_sum, state, tv_part, sq_part, ckpt, bytes;
+    size_t w, chunk_sum, state, tv_part, sq_part, chunk_map, sub_map, bytes;
 };
 __host__ __device__ constexpr Layout layout(int k, int nblocks) {
     const size_t n = (size_t)1 << k;
     const size_t nch = n >= (size_t)kChunk ? n / kChunk : 1;
+    const size_t nsub = n >= (size_t)kSub ? n / kSub : 1;
     Layout L{};
     L.w = 0;
-    L.chunk_sum = L.w + n * nblocks * sizeof(double);
+    L.chunk_sum = L.w + ((n * nblocks * sizeof(double) + 15) & ~(size_t)15);
     L.state = L.chunk_sum + nch * nblocks * sizeof(dd);
     L.tv_part = L.state + nblocks * sizeof(BlockState);
     L.sq_part = L.tv_part + nch * nblocks * sizeof(double);
-    L.ckpt = L.sq_part + nch * nblocks * sizeof(double);
-    L.bytes = L.ckpt + seq_groups(n) * nblocks * sizeof(double);
+    L.chunk_map = L.sq_part + nch * nblocks * sizeof(double);
+    L.sub_map = L.chunk_map + nch * nblocks * sizeof(SeqChunk);
+    L.bytes = L.sub_map + nsub * nblocks * sizeof(SeqMap);
     L.bytes = (L.bytes + 255) & ~(size_t)255;
     return L;
 }
 
+__device__ __forceinline__ dd shfl_up_dd(dd v, int off) {
+    return {__shfl_up_sync(0xffffffffu, v.hi, off), __shfl_up_sync(0xffffffffu, v.lo, off)};
+}
+
+// sum over the CTA (kThreads threads), the same value in every thread
 __device__ __forceinline__ dd block_sum_dd(dd v) {
     __shared__ dd red[kThreads / 32];
     for (int off = 16; off > 0; off >>= 1) {
@@ -105,21 +129,49 @@ __device__ __forceinline__ dd block_sum_dd(dd v) {
     }
     if ((threadIdx.x & 31) == 0) red[threadIdx.x >> 5] = v;
     __syncthreads();
-    if (threadIdx.x == 0) {
-        dd s = red[0];
-        for (int w = 1; w < kThreads / 32; ++w) s = dd_add(s, red[w]);
-        red[0] = s;
+    v = red[threadIdx.x & (kThreads / 32 - 1)];
+    for (int off = kThreads / 64; off > 0; off >>= 1) {
+        dd o{__shfl_xor_sync(0xffffffffu, v.hi, off), __shfl_xor_sync(0xffffffffu, v.lo, off)};
+        v = dd_add(v, o);
     }
     __syncthreads();
-    dd r = red[0];
-    __syncthreads();
-    return r;
+    return v;
 }
 
-// 1. weights + per-chunk double-double sums
+// Exclusive scan over the CTA's threads, on top of `carry`; `total` receives carry + the sum.  Two
+// shuffle scans (inside the warps, then over the warp sums in every warp) instead of one thread
+// walking the kThreads sums: a walk is kThreads dependent double-double additions.
+__device__ __forceinline__ dd block_scan_dd(dd v, dd carry, dd* total) {
+    __shared__ dd red[kThreads / 32];
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    dd inc = v;
+    for (int off = 1; off < 32; off <<= 1) {
+        const dd o = shfl_up_dd(inc, off);
+        if (lane >= off) inc = dd_add(o, inc);
+    }
+    if (lane == 31) red[warp] = inc;
+    __syncthreads();
+    dd s = lane < kThreads / 32 ? red[lane] : dd{0.0, 0.0};
+    if (lane == 0) s = dd_add(carry, s);
+    for (int off = 1; off < kThreads / 32; off <<= 1) {
+        const dd o = shfl_up_dd(s, off);
+        if (lane >= off) s = dd_add(o, s);
+    }
+    const int last = kThreads / 32 - 1;
+    *total = {__shfl_sync(0xffffffffu, s.hi, last), __shfl_sync(0xffffffffu, s.lo, last)};
+    const int from = warp ? warp - 1 : 0;
+    dd before{__shfl_sync(0xffffffffu, s.hi, from), __shfl_sync(0xffffffffu, s.lo, from)};
+    if (warp == 0) before = carry;
+    dd ex = shfl_up_dd(inc, 1);
+    if (lane == 0) ex = dd{0.0, 0.0};
+    __syncthreads();
+    return dd_add(before, ex);
+}
+
+// 1. weights + per-chunk double-double sums; part[] marks chunks with a nonfinite amplitude
 __global__ void __launch_bounds__(kThreads)
 k_weights(const double2* __restrict__ blocks, int k, double* __restrict__ w, dd* __restrict__ chunk_sum,
-          BlockState* __restrict__ state) {
+          double* __restrict__ part) {
     const int b = blockIdx.y;
     const uint64_t n = 1ull << k;
     const uint64_t start = (uint64_t)blockIdx.x * kChunk;
@@ -142,262 +194,172 @@ k_weights(const double2* __restrict__ blocks, int k, double* __restrict__ w, dd*
     const int anybad = __syncthreads_or(bad);
     if (threadIdx.x == 0) {
         chunk_sum[(uint64_t)b * gridDim.x + blockIdx.x] = s;
-        if (anybad) atomicOr(&state[b].nonfinite, 1);
+        part[(uint64_t)b * gridDim.x + blockIdx.x] = anybad ? 1.0 : 0.0;
     }
 }
 
-// 2. chunk scan (sequential over <= 2^k/2048 chunks) + chunk search, one thread per block
-__global__ void k_scan_locate(dd* __restrict__ chunk_sum, int nch, const double* __restrict__ uniforms,
-                              BlockState* __restrict__ state, dcs_draw_result* __restrict__ res) {
+// 2. chunk scan + chunk search, one CTA per block.  A 2^20 block has 512 chunks: one thread walking them
+//    took 69 us (a dependent load, store and addition per chunk), the scan takes about 5.
+__global__ void __launch_bounds__(kThreads)
+k_scan_locate(dd* __restrict__ chunk_sum, int nch, const double* __restrict__ uniforms,
+              BlockState* __restrict__ state, dcs_draw_result* __restrict__ res, const double* __restrict__ part) {
     const int b = blockIdx.x;
     dd* cs = chunk_sum + (uint64_t)b * nch;
+    __shared__ int at;
+    if (threadIdx.x == 0) at = 0;
     dd run{0.0, 0.0};
-    for (int c = 0; c < nch; ++c) {  // exclusive scan in place
-        const dd s = cs[c];
-        cs[c] = run;
-        run = dd_add(run, s);
+    int bad = 0;
+    for (int c0 = 0; c0 < nch; c0 += kThreads) {  // exclusive scan in place
+        const int c = c0 + threadIdx.x;
+        dd s{0.0, 0.0};
+        if (c < nch) {
+            s = cs[c];
+            bad |= part[(uint64_t)b * nch + c] != 0.0;
+        }
+        dd total;
+        const dd ex = block_scan_dd(s, run, &total);
+        if (c < nch) cs[c] = ex;
+        run = total;
     }
-    BlockState& st = state[b];
-    st.total = run;
+    const int nonfinite = __syncthreads_or(bad);
     const double u = uniforms[b];
-    dcs_draw_result& r = res[b];
-    memset(&r, 0, sizeof(r));
-    r.uniform = u;
-    r.index = -1;
-    if (st.nonfinite || !(u >= 0.0 && u < 1.0)) { r.status = DCS_E_ARG; st.status = DCS_E_ARG; return; }
-    if (!(run.hi > 0.0) || !isfinite(run.hi)) { r.status = DCS_E_CDF; st.status = DCS_E_CDF; return; }
-    const dd target = dd_mul(run, u);
-    // last chunk whose exclusive start is <= target
-    int lo = 0, hi = nch - 1;
-    while (lo < hi) {
-        const int mid = (lo + hi + 1) >> 1;
-        if (dd_lt(target, cs[mid])) hi = mid - 1; else lo = mid;
-    }
-    st.chunk = lo;
-    st.status = 0;
-}
-
-// 3. element search inside the chunk + certification (one CTA per block)
-__global__ void __launch_bounds__(kThreads)
-k_locate_elem(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, int nch,
-              BlockState* __restrict__ state, dcs_draw_result* __restrict__ res) {
-    const int b = blockIdx.x;
-    BlockState& st = state[b];
-    if (st.status) return;
-    const uint64_t n = 1ull << k;
-    const int64_t c = st.chunk;
-    const uint64_t start = (uint64_t)c * kChunk;
-    const double* wb = w + ((uint64_t)b << k);
-    const dd off = chunk_sum[(uint64_t)b * nch + c];
-    const dd T = st.total;
-    const double u = res[b].uniform;
-    const dd target = dd_mul(T, u);
-    // thread t owns kPer consecutive elements
-    __shared__ dd pre[kThreads];
-    double loc[kPer];
-    dd acc{0.0, 0.0};
-    for (int j = 0; j < kPer; ++j) {
-        const uint64_t i = start + (uint64_t)threadIdx.x * kPer + j;
-        loc[j] = i < n ? wb[i] : 0.0;
-        acc = dd_add(acc, loc[j]);
-    }
-    pre[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {  // exclusive scan of the 256 thread sums
-        dd run = off;
-        for (int t = 0; t < kThreads; ++t) {
-            const dd s = pre[t];
-            pre[t] = run;
-            run = dd_add(run, s);
-        }
+    int status = 0;
+    if (nonfinite || !(u >= 0.0 && u < 1.0)) status = DCS_E_ARG;
+    else if (!(run.hi > 0.0) || !isfinite(run.hi)) status = DCS_E_CDF;
+    if (!status) {
+        // last chunk whose exclusive start is <= target (every thread reads back its own stores)
+        const dd target = dd_mul(run, u);
+        int mine = 0;
+        for (int c = threadIdx.x; c < nch; c += kThreads)
+            if (!dd_lt(target, cs[c])) mine = c;
+        if (mine) atomicMax(&at, mine);
     }
     __syncthreads();
-    // each thread scans its own elements; the first i with P_i > target wins
-    dd run = pre[threadIdx.x];
-    int64_t found = -1;
-    dd p_before{0, 0}, p_at{0, 0};
-    for (int j = 0; j < kPer; ++j) {
-        const uint64_t i = start + (uint64_t)threadIdx.x * kPer + j;
-        if (i >= n) break;
-        const dd nxt = dd_add(run, loc[j]);
-        if (dd_lt(target, nxt) && loc[j] > 0.0) {
-            found = (int64_t)i;
-            p_before = run;
-            p_at = nxt;
-            break;
-        }
-        run = nxt;
-    }
-    __shared__ unsigned long long best;
-    if (threadIdx.x == 0) best = ~0ull;
-    __syncthreads();
-    if (found >= 0) atomicMin(&best, (unsigned long long)found);
-    __syncthreads();
-    if (found >= 0 && (unsigned long long)found == best) {
+    if (threadIdx.x == 0) {
+        BlockState& st = state[b];
+        st.total = run;
+        st.status = status;
+        st.chunk = at;
         dcs_draw_result& r = res[b];
-        // math.fsum rounds each sum to double before the division (sampling_protocol.py:67-69);
-        // a normalised double-double's high word is that rounding
-        const double lo = __ddiv_rn(p_before.hi, T.hi), hi = __ddiv_rn(p_at.hi, T.hi);
-        const double wi = loc[found - (int64_t)start - (int64_t)threadIdx.x * kPer];
-        r.index = found;
-        r.selected_weight = wi;
-        r.total_exact = T.hi;
-        r.total_cdf = r.total_exact;
-        r.cdf_lower_exact = lo;
-        r.cdf_upper_exact = hi;
-        r.cdf_lower = found ? lo : 0.0;
-        r.cdf_upper = ((uint64_t)found == n - 1) ? 1.0 : hi;
-        // certification against numpy's sequential cumsum (bound on each side + 4 ulp slack)
-        const double eps = 1.1102230246251565e-16;  // 2^-53
-        const double rel = ((double)found + (double)n + 8.0) * eps;
-        const bool low_ok = found == 0 || lo * (1.0 + rel) <= u;
-        const bool high_ok = ((uint64_t)found == n - 1) || hi * (1.0 - rel) > u;
-        r.tie = !(low_ok && high_ok);
-        r.status = 0;
-    }
-    if (threadIdx.x == 0 && best == ~0ull) {
-        // u*T beyond every accurate prefix (possible only within rounding of T): sequential path decides
-        res[b].tie = 1;
-        res[b].total_exact = T.hi;
+        memset(&r, 0, sizeof(r));
+        r.uniform = u;
+        r.index = -1;
+        r.status = status;
+        r.total_exact = status ? 0.0 : run.hi;
     }
 }
 
-// 4. exact sequential FP64 CDF (numpy's operation order), one warp per block: for blocks
-//    flagged as ties, or for every block when `force`.  Every lane runs the same dependent
-//    chain S <- S + w_i (the 32 weights of a group are loaded by the 32 lanes and broadcast by
-//    shuffles, the next 128 prefetched), so the chain is numpy's cumsum exactly.  Pass 1 gives
-//    S_n and a checkpoint before every 32-element group; the selected group is the last one
-//    whose starting value satisfies fl(start / S_n) <= u (fl(x / S_n) is non-decreasing in x),
-//    and pass 2 replays that group only.  The compensated interval of the selected index is
-//    checked against u as the reference's independent check does (sampling_protocol.py:67-72).
-__global__ void __launch_bounds__(32)
-k_sequential(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, int nch,
-             BlockState* __restrict__ state, dcs_draw_result* __restrict__ res, double* __restrict__ ckpt,
-             int force) {
-    const int b = blockIdx.x;
-    const int lane = threadIdx.x;
-    dcs_draw_result& r = res[b];
-    if (state[b].status || !(r.tie || force)) return;
-    const uint64_t n = 1ull << k;
-    const uint64_t ng = seq_groups(n);
-    const double* wb = w + ((uint64_t)b << k);
-    double* ck = ckpt + (uint64_t)b * ng;
-    // pass 1: S_n with checkpoints, four groups (128 weights) per iteration, the next four in flight
-    double S = 0.0;
-    double cur[4], nxt[4];
+// first map, then second
+__device__ __forceinline__ void map_then(long long& a0, long long& a1, long long b0, long long b1) {
+    a0 += (a0 & 1) ? b1 : b0;
+    a1 += ((a1 + 1) & 1) ? b1 : b0;
+}
+
+// The maps of one chunk's sub-chunks and of the chunk (all threads of the CTA): thread t owns the
+// weights loc[] of elements kPer t .. kPer t + kPer - 1 and `before`, the prefix sum before them.
+__device__ __forceinline__ void chunk_maps(const double (&loc)[kPer], double before, uint64_t n, uint64_t c,
+                                           uint64_t nch, SeqChunk* __restrict__ chunk_map,
+                                           SeqMap* __restrict__ sub_map) {
+    constexpr int kGroups = kThreads / kSubThreads;
+    __shared__ SeqMap sm[kGroups];
+    const int lane = threadIdx.x & 31;
+    double mine = 0.0;
 #pragma unroll
-    for (int q = 0; q < 4; ++q) {
-        const uint64_t i = (uint64_t)q * 32 + lane;
-        cur[q] = i < n ? wb[i] : 0.0;
+    for (int j = 0; j < kPer; ++j) mine += loc[j];
+    // ends of the sub-chunk (its kSubThreads threads are half a warp)
+    const int first = lane & ~(kSubThreads - 1);
+    const double lo = __shfl_sync(0xffffffffu, before, first);
+    const double hi = __shfl_sync(0xffffffffu, before + mine, first + kSubThreads - 1);
+    const unsigned some = __ballot_sync(0xffffffffu, mine > 0.0) >> first & ((1u << kSubThreads) - 1u);
+    const double rel = ((double)n + 16.0) * 2.220446049250313e-16;  // twice the bound, in ulps of 2^-53
+    const double s0 = lo * (1.0 - rel), s1 = hi * (1.0 + rel);
+    const int e0 = (__double2hiint(s0) >> 20) - 1023, e1 = (__double2hiint(s1) >> 20) - 1023;
+    const bool inside = some && e0 == e1 && e0 > -900 && e0 < 1000;
+    long long d0 = 0, d1 = 0;
+    if (inside) {
+        // increments from an even and from an odd k of the same binade: 2^e and 2^e + q
+        const double even = __hiloint2double((e0 + 1023) << 20, 0), odd = __hiloint2double((e0 + 1023) << 20, 1);
+        const double inv_q = __hiloint2double((1023 + 52 - e0) << 20, 0);
+#pragma unroll
+        for (int j = 0; j < kPer; ++j)
+            map_then(d0, d1, (long long)__dmul_rn(__dsub_rn(__dadd_rn(even, loc[j]), even), inv_q),
+                     (long long)__dmul_rn(__dsub_rn(__dadd_rn(odd, loc[j]), odd), inv_q));
     }
-    for (uint64_t g0 = 0; g0 < ng; g0 += 4) {
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            const uint64_t i = (g0 + 4 + q) * 32 + lane;
-            nxt[q] = i < n ? wb[i] : 0.0;
-        }
+    for (int off = 1; off < kSubThreads; off <<= 1) {
+        const long long o0 = __shfl_down_sync(0xffffffffu, d0, off), o1 = __shfl_down_sync(0xffffffffu, d1, off);
+        if (!((lane & (kSubThreads - 1)) & (2 * off - 1))) map_then(d0, d1, o0, o1);
+    }
+    if (lane == first) {
+        SeqMap m{d0, d1, inside ? e0 : (some ? kMapWalk : kMapNone), 0};
+        sm[threadIdx.x / kSubThreads] = m;
+        const uint64_t g = c * kSubs + threadIdx.x / kSubThreads;
+        if (g * kSub < n) sub_map[g] = m;
+    }
+    __syncthreads();
+    if (threadIdx.x < 32) {  // the chunk: one map if no sub-chunk leaves the binade of the others
+        const SeqMap m = lane < kSubs ? sm[lane] : SeqMap{0, 0, kMapNone, 0};
+        int e = m.e;
+        bool walk = e == kMapWalk;
+        long long c0 = m.d0, c1 = m.d1;
 #pragma unroll
-        for (int q = 0; q < 4; ++q) {
-            if (g0 + q < ng) {
-                if (lane == 0) ck[g0 + q] = S;
-                const uint64_t base = (g0 + q) * 32;
-#pragma unroll
-                for (int j = 0; j < 32; ++j) {
-                    const double v = __shfl_sync(0xffffffffu, cur[q], j);
-                    if (base + j < n) S = __dadd_rn(S, v);
-                }
+        for (int off = 1; off < kSubs; off <<= 1) {
+            const int oe = __shfl_down_sync(0xffffffffu, e, off);
+            const bool ow = __shfl_down_sync(0xffffffffu, (int)walk, off);
+            const long long o0 = __shfl_down_sync(0xffffffffu, c0, off), o1 = __shfl_down_sync(0xffffffffu, c1, off);
+            if (!(lane & (2 * off - 1))) {
+                walk = walk || ow || (e != kMapNone && oe != kMapNone && e != oe);
+                if (e == kMapNone) e = oe;
+                map_then(c0, c1, o0, o1);
             }
         }
-#pragma unroll
-        for (int q = 0; q < 4; ++q) cur[q] = nxt[q];
+        if (lane == 0) chunk_map[c].map = SeqMap{c0, c1, walk ? kMapWalk : e, 0};
     }
-    if (lane != 0) return;  // lane 0 wrote the checkpoints and finishes alone
-    if (!(S > 0.0) || !isfinite(S)) {
-        r.status = DCS_E_CDF;
-        return;
-    }
-    const double u = r.uniform;
-    // last group whose starting value's quotient is <= u (group 0 starts at 0)
-    uint64_t lo = 0, hi = ng - 1;
-    while (lo < hi) {
-        const uint64_t mid = (lo + hi + 1) >> 1;
-        if (__ddiv_rn(ck[mid], S) <= u) lo = mid; else hi = mid - 1;
-    }
-    // pass 2: replay the group; the last element's value is forced to 1 (numpy: cumulative[-1] = 1)
-    double run = ck[lo], prev = __ddiv_rn(run, S);
-    uint64_t idx = n - 1;
-    double upper = 1.0;
-    for (uint64_t i = lo * 32; i < n && i < (lo + 1) * 32; ++i) {
-        run = __dadd_rn(run, wb[i]);
-        const double ci = (i == n - 1) ? 1.0 : __ddiv_rn(run, S);
-        if (u < ci) { idx = i; upper = ci; break; }
-        prev = ci;
-    }
-    // compensated prefix before idx: the scan's chunk prefix plus the chunk's elements before idx
-    const uint64_t c0 = idx / kChunk;
-    dd pre = chunk_sum[(uint64_t)b * nch + c0];
-    for (uint64_t i = c0 * kChunk; i < idx; ++i) pre = dd_add(pre, wb[i]);
-    const dd at = dd_add(pre, wb[idx]);
-    const dd T = state[b].total;
-    r.cdf_lower = idx ? prev : 0.0;
-    r.cdf_upper = upper;
-    r.cdf_lower_exact = __ddiv_rn(pre.hi, T.hi);
-    r.cdf_upper_exact = __ddiv_rn(at.hi, T.hi);
-    r.index = (int64_t)idx;
-    r.total_cdf = S;
-    r.total_exact = T.hi;
-    r.selected_weight = wb[idx];
-    if (!(wb[idx] > 0.0)) r.status = DCS_E_CDF;
-    // the reference's independent check of the interval (a disagreement is an error, never a resample)
-    else if (!(r.cdf_lower_exact <= u && u < r.cdf_upper_exact)) r.status = DCS_E_CDF;
+    __syncthreads();
 }
 
-// 5. 53-bit grid TV and the sum of squared weights, per chunk partial sums (deterministic final
-//    sums in k_tv_final)
+// 3. per chunk: 53-bit grid TV and sum of squared weights (partial sums), in the located chunk the
+//    element search with its certification, and on request (maps) the sequential CDF's maps.  The three
+//    need the same prefix sums of the chunk's weights.
 __global__ void __launch_bounds__(kThreads)
-k_tv(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, int nch,
-     const BlockState* __restrict__ state, const dcs_draw_result* __restrict__ res, double* __restrict__ part,
-     double* __restrict__ sq_part) {
+k_chunk(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, int nch,
+        const BlockState* __restrict__ state, dcs_draw_result* __restrict__ res, double* __restrict__ part,
+        double* __restrict__ sq_part, SeqChunk* __restrict__ chunk_map, SeqMap* __restrict__ sub_map, int maps) {
     const int b = blockIdx.y;
     const int c = blockIdx.x;
     const uint64_t n = 1ull << k;
     if (state[b].status) return;
     const dd T = state[b].total;
-    const double mass = res[b].total_exact;
+    const double mass = T.hi;
     const uint64_t start = (uint64_t)c * kChunk;
     const double* wb = w + ((uint64_t)b << k);
-    __shared__ dd pre[kThreads];
     double loc[kPer];
     dd acc{0.0, 0.0};
+#pragma unroll
     for (int j = 0; j < kPer; ++j) {
         const uint64_t i = start + (uint64_t)threadIdx.x * kPer + j;
         loc[j] = i < n ? wb[i] : 0.0;
         acc = dd_add(acc, loc[j]);
     }
-    pre[threadIdx.x] = acc;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        dd run = chunk_sum[(uint64_t)b * nch + c];
-        for (int t = 0; t < kThreads; ++t) {
-            const dd s = pre[t];
-            pre[t] = run;
-            run = dd_add(run, s);
-        }
-    }
-    __syncthreads();
-    dd run = pre[threadIdx.x];
+    dd total;
+    const dd before = block_scan_dd(acc, chunk_sum[(uint64_t)b * nch + c], &total);
+    if (maps)
+        chunk_maps(loc, before.hi, n, c, nch, chunk_map + (uint64_t)b * nch,
+                   sub_map + (uint64_t)b * (n >= (uint64_t)kSub ? n / kSub : 1));
+    dd run = before;
     const double two53 = 9007199254740992.0;
     double prev_end = ceil(dd_div(run, T) * two53);
     if (start + (uint64_t)threadIdx.x * kPer == 0) prev_end = 0.0;
     double s = 0.0, q = 0.0;
+#pragma unroll
     for (int j = 0; j < kPer; ++j) {
         const uint64_t i = start + (uint64_t)threadIdx.x * kPer + j;
         if (i >= n) break;
         run = dd_add(run, loc[j]);
         const double ci = (i == n - 1) ? 1.0 : dd_div(run, T);
         const double end = ceil(ci * two53);
-        s += fabs((end - prev_end) / two53 - loc[j] / mass);
         const double p = loc[j] / mass;
+        s += fabs((end - prev_end) / two53 - p);
         q = fma(p, p, q);
         prev_end = end;
     }
@@ -407,20 +369,259 @@ k_tv(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, int 
         part[(uint64_t)b * nch + c] = tot.hi + tot.lo;
         sq_part[(uint64_t)b * nch + c] = sq.hi + sq.lo;
     }
+    if (c != state[b].chunk) return;
+    // element search inside the located chunk: the first i with P_i > target wins
+    const double u = res[b].uniform;
+    const dd target = dd_mul(T, u);
+    int found = -1;
+    dd p_before{0, 0}, p_at{0, 0};
+    double wi = 0.0;
+    run = before;
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const dd nxt = dd_add(run, loc[j]);
+        if (found < 0 && loc[j] > 0.0 && dd_lt(target, nxt)) {
+            found = (int)threadIdx.x * kPer + j;
+            p_before = run;
+            p_at = nxt;
+            wi = loc[j];
+        }
+        run = nxt;
+    }
+    __shared__ int best;
+    if (threadIdx.x == 0) best = INT32_MAX;
+    __syncthreads();
+    if (found >= 0) atomicMin(&best, found);
+    __syncthreads();
+    dcs_draw_result& r = res[b];
+    if (found >= 0 && found == best) {
+        const uint64_t i = start + found;
+        // math.fsum rounds each sum to double before the division (sampling_protocol.py:67-69);
+        // a normalised double-double's high word is that rounding
+        const double lo = __ddiv_rn(p_before.hi, T.hi), hi = __ddiv_rn(p_at.hi, T.hi);
+        r.index = (int64_t)i;
+        r.selected_weight = wi;
+        r.total_exact = T.hi;
+        r.total_cdf = r.total_exact;
+        r.cdf_lower_exact = lo;
+        r.cdf_upper_exact = hi;
+        r.cdf_lower = i ? lo : 0.0;
+        r.cdf_upper = (i == n - 1) ? 1.0 : hi;
+        // certification against numpy's sequential cumsum (bound on each side + 4 ulp slack)
+        const double eps = 1.1102230246251565e-16;  // 2^-53
+        const double rel = ((double)i + (double)n + 8.0) * eps;
+        const bool low_ok = i == 0 || lo * (1.0 + rel) <= u;
+        const bool high_ok = (i == n - 1) || hi * (1.0 - rel) > u;
+        r.tie = !(low_ok && high_ok);
+        r.status = 0;
+    }
+    if (threadIdx.x == 0 && best == INT32_MAX) {
+        // u*T beyond every accurate prefix (possible only within rounding of T): sequential path decides
+        r.tie = 1;
+        r.total_exact = T.hi;
+    }
 }
 
-__global__ void k_tv_final(const double* __restrict__ part, const double* __restrict__ sq_part, int nch,
-                           const BlockState* __restrict__ state, dcs_draw_result* __restrict__ res, int nblocks) {
-    const int b = blockIdx.x * blockDim.x + threadIdx.x;
-    if (b >= nblocks) return;
-    if (state[b].status) { res[b].status = state[b].status; return; }
+// S after a stretch with map m, or false when S is not where the map holds (the weights are then added
+// one by one): S of one binade is an integer in its bit pattern, so the increment is an integer addition.
+__device__ __forceinline__ bool seq_apply(long long& S, const SeqMap& m) {
+    if (m.e == kMapNone) return true;
+    const long long t = S + ((S & 1) ? m.d1 : m.d0);
+    if ((int)(S >> 52) - 1023 != m.e || (int)(t >> 52) - 1023 != m.e) return false;  // kMapWalk: never equal
+    S = t;
+    return true;
+}
+// S after the weights [i0, i1) added one by one (one warp, the same S in every lane; i1 - i0 <= kSub);
+// out: optional array for S after each
+__device__ __forceinline__ double seq_walk(const double* __restrict__ wb, uint64_t i0, uint64_t i1, double S,
+                                           double* out) {
+    const int lane = threadIdx.x & 31;
+    double v[kSub / 32];
+#pragma unroll
+    for (int q = 0; q < kSub / 32; ++q) {
+        const uint64_t i = i0 + q * 32 + lane;
+        v[q] = i < i1 ? wb[i] : 0.0;  // adding zero changes nothing
+    }
+#pragma unroll
+    for (int q = 0; q < kSub / 32; ++q) {
+        if (i0 + q * 32 >= i1) break;
+        double keep = 0.0;
+#pragma unroll
+        for (int j = 0; j < 32; ++j) {
+            S = __dadd_rn(S, __shfl_sync(0xffffffffu, v[q], j));
+            if (j == lane) keep = S;
+        }
+        if (out) out[q * 32 + lane] = keep;
+    }
+    return S;
+}
+
+// S after chunk c from S before it (one warp); stop >= 0: only up to the start of sub-chunk `stop`
+__device__ __forceinline__ double seq_chunk(const double* __restrict__ wb, uint64_t n, uint64_t c,
+                                            const SeqMap* __restrict__ sub_map, double S, double* sub_start) {
+    const int lane = threadIdx.x & 31;
+    const uint64_t g0 = c * kSubs;
+    SeqMap mine{0, 0, kMapNone, 0};
+    if (lane < kSubs && (g0 + lane) * kSub < n) mine = sub_map[g0 + lane];
+    for (int j = 0; j < kSubs; ++j) {
+        if ((g0 + j) * kSub >= n) break;
+        if (sub_start && lane == 0) sub_start[j] = S;
+        SeqMap m;
+        m.d0 = __shfl_sync(0xffffffffu, mine.d0, j);
+        m.d1 = __shfl_sync(0xffffffffu, mine.d1, j);
+        m.e = __shfl_sync(0xffffffffu, mine.e, j);
+        long long bits = __double_as_longlong(S);
+        const uint64_t i0 = (g0 + j) * kSub;
+        if (seq_apply(bits, m)) S = __longlong_as_double(bits);
+        else S = seq_walk(wb, i0, i0 + kSub < n ? i0 + kSub : n, S, nullptr);
+    }
+    return S;
+}
+
+// 4. totals of the chunk sums, and the exact sequential FP64 CDF (numpy's operation order) for blocks
+//    flagged as ties, or for every block when `force` (one CTA per block).  Warp 0 carries S from chunk
+//    to chunk by the maps; chunks that cross a binade (about log2 of the block size of them) go through their
+//    sub-chunks' maps, and the one or two sub-chunks that cross are added up one weight after the other.
+//    The chain of n dependent additions this replaces took 10.9 ms for 2^20 weights; carrying S over 512
+//    chunks with 10 crossings takes about 30 us.  The selected chunk (and sub-chunk) is the last one whose
+//    starting value satisfies fl(start / S_n) <= u (fl(x / S_n) is non-decreasing in x), and only the
+//    selected sub-chunk is replayed.  The compensated interval of the selected index is checked
+//    against u as the reference's independent check does (sampling_protocol.py:67-72).
+__global__ void __launch_bounds__(kThreads)
+k_finish(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, int nch,
+         const BlockState* __restrict__ state, dcs_draw_result* __restrict__ res, const double* __restrict__ part,
+         const double* __restrict__ sq_part, SeqChunk* __restrict__ chunk_map, SeqMap* __restrict__ sub_map,
+         int force) {
+    const int b = blockIdx.x;
+    const int lane = threadIdx.x & 31;
+    dcs_draw_result& r = res[b];
+    if (state[b].status) return;
     double s = 0.0, q = 0.0;
-    for (int c = 0; c < nch; ++c) {
+    for (int c = threadIdx.x; c < nch; c += kThreads) {
         s += part[(uint64_t)b * nch + c];
         q += sq_part[(uint64_t)b * nch + c];
     }
-    res[b].tv53 = 0.5 * s;
-    res[b].weight_l2 = q;
+    const dd ts = block_sum_dd(dd{s, 0.0}), tq = block_sum_dd(dd{q, 0.0});
+    if (threadIdx.x == 0) {
+        r.tv53 = 0.5 * (ts.hi + ts.lo);
+        r.weight_l2 = tq.hi + tq.lo;
+    }
+    if (!(r.tie || force)) return;
+    const uint64_t n = 1ull << k;
+    const double* wb = w + ((uint64_t)b << k);
+    const dd* cs = chunk_sum + (uint64_t)b * nch;
+    SeqChunk* cm = chunk_map + (uint64_t)b * nch;
+    SeqMap* sb = sub_map + (uint64_t)b * (n >= (uint64_t)kSub ? n / kSub : 1);
+    __shared__ double s_total, sub_start[kSubs], seq[kSub];
+    __shared__ int at;
+    if (!force) {  // a tie found by the search: the maps were not made with the chunk sums
+        for (int c = 0; c < nch; ++c) {
+            double loc[kPer];
+            dd acc{0.0, 0.0};
+#pragma unroll
+            for (int j = 0; j < kPer; ++j) {
+                const uint64_t i = (uint64_t)c * kChunk + (uint64_t)threadIdx.x * kPer + j;
+                loc[j] = i < n ? wb[i] : 0.0;
+                acc = dd_add(acc, loc[j]);
+            }
+            dd total;
+            const dd before = block_scan_dd(acc, cs[c], &total);
+            chunk_maps(loc, before.hi, n, c, nch, cm, sb);
+        }
+    }
+    if (threadIdx.x == 0) at = 0;
+    __syncthreads();
+    if (threadIdx.x < 32) {
+        double S = 0.0;
+        for (int c0 = 0; c0 < nch; c0 += 32) {
+            SeqMap mine{0, 0, kMapNone, 0};
+            if (c0 + lane < nch) mine = cm[c0 + lane].map;
+            double started = 0.0;
+            const int cnt = nch - c0 < 32 ? nch - c0 : 32;
+            for (int j = 0; j < cnt; ++j) {
+                if (j == lane) started = S;
+                SeqMap m;
+                m.d0 = __shfl_sync(0xffffffffu, mine.d0, j);
+                m.d1 = __shfl_sync(0xffffffffu, mine.d1, j);
+                m.e = __shfl_sync(0xffffffffu, mine.e, j);
+                long long bits = __double_as_longlong(S);
+                if (seq_apply(bits, m)) S = __longlong_as_double(bits);
+                else S = seq_chunk(wb, n, c0 + j, sb, S, nullptr);
+            }
+            if (c0 + lane < nch) cm[c0 + lane].start = started;
+        }
+        if (lane == 0) s_total = S;
+    }
+    __syncthreads();
+    const double S = s_total;
+    if (!(S > 0.0) || !isfinite(S)) {
+        if (threadIdx.x == 0) r.status = DCS_E_CDF;
+        return;
+    }
+    const double u = r.uniform;
+    // last chunk whose starting value's quotient is <= u (chunk 0 starts at 0)
+    int mine = 0;
+    for (int c = threadIdx.x; c < nch; c += kThreads)
+        if (__ddiv_rn(cm[c].start, S) <= u) mine = c;
+    if (mine) atomicMax(&at, mine);
+    __syncthreads();
+    const uint64_t c = at;
+    __shared__ int64_t s_idx;
+    if (threadIdx.x < 32) {
+        seq_chunk(wb, n, c, sb, cm[c].start, sub_start);
+        __syncwarp();
+        const bool is = lane < kSubs && (c * kSubs + lane) * kSub < n && __ddiv_rn(sub_start[lane], S) <= u;
+        const unsigned m = __ballot_sync(0xffffffffu, is);
+        const int j = m ? 31 - __clz(m) : 0;
+        // replay the sub-chunk; the last element's value is forced to 1 (numpy: cumulative[-1] = 1)
+        const uint64_t i0 = (c * kSubs + j) * kSub, i1 = i0 + kSub < n ? i0 + kSub : n;
+        const double S0 = sub_start[j];
+        seq_walk(wb, i0, i1, S0, seq);
+        __syncwarp();
+        int hit = kSub;
+#pragma unroll
+        for (int p = kSub / 32 - 1; p >= 0; --p) {
+            const uint64_t i = i0 + p * 32 + lane;
+            if (i < i1 && u < ((i == n - 1) ? 1.0 : __ddiv_rn(seq[p * 32 + lane], S))) hit = p * 32 + lane;
+        }
+        for (int off = 16; off > 0; off >>= 1) hit = min(hit, __shfl_xor_sync(0xffffffffu, hit, off));
+        if (lane == 0) {
+            const uint64_t idx = hit < kSub ? i0 + hit : n - 1;
+            double prev = 0.0, upper = 1.0;
+            if (hit < kSub) {
+                prev = __ddiv_rn(hit ? seq[hit - 1] : S0, S);
+                upper = (idx == n - 1) ? 1.0 : __ddiv_rn(seq[hit], S);
+            } else {
+                prev = __ddiv_rn(seq[i1 - 1 - i0], S);
+            }
+            s_idx = (int64_t)idx;
+            r.cdf_lower = idx ? prev : 0.0;
+            r.cdf_upper = upper;
+        }
+    }
+    __syncthreads();
+    const uint64_t idx = (uint64_t)s_idx;
+    // compensated prefix before idx: the scan's chunk prefix plus the chunk's elements before idx
+    const uint64_t ci = idx / kChunk;
+    dd acc{0.0, 0.0};
+#pragma unroll
+    for (int j = 0; j < kPer; ++j) {
+        const uint64_t i = ci * kChunk + (uint64_t)threadIdx.x * kPer + j;
+        if (i < idx) acc = dd_add(acc, wb[i]);
+    }
+    const dd pre = dd_add(cs[ci], block_sum_dd(acc));
+    if (threadIdx.x) return;
+    const double wi = wb[idx];
+    const dd T = state[b].total;
+    r.cdf_lower_exact = __ddiv_rn(pre.hi, T.hi);
+    r.cdf_upper_exact = __ddiv_rn(dd_add(pre, wi).hi, T.hi);
+    r.index = (int64_t)idx;
+    r.total_cdf = S;
+    r.total_exact = T.hi;
+    r.selected_weight = wi;
+    if (!(wi > 0.0)) r.status = DCS_E_CDF;
+    // the reference's independent check of the interval (a disagreement is an error, never a resample)
+    else if (!(r.cdf_lower_exact <= u && u < r.cdf_upper_exact)) r.status = DCS_E_CDF;
 }
 
 // ---------------------------------------------------------------- audit overlap
@@ -472,24 +673,19 @@ int enqueue_draw(const double* blocks, int k, int nblocks, const double* uniform
     BlockState* st = (BlockState*)(base + L.state);
     double* part = (double*)(base + L.tv_part);
     double* sq = (double*)(base + L.sq_part);
-    double* ck = (double*)(base + L.ckpt);
+    SeqChunk* cm = (SeqChunk*)(base + L.chunk_map);
+    SeqMap* sm = (SeqMap*)(base + L.sub_map);
     const uint64_t n = 1ull << k;
     const int nch = (int)(n >= (uint64_t)kChunk ? n / kChunk : 1);
-    // the scratch keeps the previous call's contents: the per-block state must start at zero
-    cudaError_t e = cudaMemsetAsync(st, 0, nblocks * sizeof(BlockState), s);
-    if (e != cudaSuccess) return dcs_host::check_cuda(e, "dcs_draw memset");
-    k_weights<<<dim3(nch, nblocks), kThreads, 0, s>>>((const double2*)blocks, k, w, cs, st);
+    const int force = (flags & DCS_DRAW_SEQUENTIAL) ? 1 : 0;
+    k_weights<<<dim3(nch, nblocks), kThreads, 0, s>>>((const double2*)blocks, k, w, cs, part);
     DCS_CHECK_LAUNCH("k_weights");
-    k_scan_locate<<<nblocks, 1, 0, s>>>(cs, nch, uniforms, st, results);
+    k_scan_locate<<<nblocks, kThreads, 0, s>>>(cs, nch, uniforms, st, results, part);
     DCS_CHECK_LAUNCH("k_scan_locate");
-    k_locate_elem<<<nblocks, kThreads, 0, s>>>(w, k, cs, nch, st, results);
-    DCS_CHECK_LAUNCH("k_locate_elem");
-    k_sequential<<<nblocks, 32, 0, s>>>(w, k, cs, nch, st, results, ck, (flags & DCS_DRAW_SEQUENTIAL) ? 1 : 0);
-    DCS_CHECK_LAUNCH("k_sequential");
-    k_tv<<<dim3(nch, nblocks), kThreads, 0, s>>>(w, k, cs, nch, st, results, part, sq);
-    DCS_CHECK_LAUNCH("k_tv");
-    k_tv_final<<<(nblocks + 31) / 32, 32, 0, s>>>(part, sq, nch, st, results, nblocks);
-    DCS_CHECK_LAUNCH("k_tv_final");
+    k_chunk<<<dim3(nch, nblocks), kThreads, 0, s>>>(w, k, cs, nch, st, results, part, sq, cm, sm, force);
+    DCS_CHECK_LAUNCH("k_chunk");
+    k_finish<<<nblocks, kThreads, 0, s>>>(w, k, cs, nch, st, results, part, sq, cm, sm, force);
+    DCS_CHECK_LAUNCH("k_finish");
     return DCS_OK;
 }
 }  // namespace
@@ -515,8 +711,8 @@ extern "C" int dcs_overlap(const double* ref, const double* ap, uint64_t len, do
         dcs_host::set_error("dcs_overlap: invalid arguments");
         return DCS_E_ARG;
     }
-    const int parts = 256;
     cudaStream_t s = (cudaStream_t)stream;
+    const int parts = 256;
     k_overlap<<<parts, kThreads, 0, s>>>((const double2*)ref, (const double2*)ap, len, (dd*)scratch);
     DCS_CHECK_LAUNCH("k_overlap");
     k_overlap_final<<<1, 32, 0, s>>>((const dd*)scratch, parts, out);
