@@ -625,15 +625,29 @@ k_finish(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, 
 }
 
 // ---------------------------------------------------------------- audit overlap
+constexpr int kOverlapParts = kThreads;  // partial sums, one CTA each: 16 KiB of scratch
+
 __global__ void __launch_bounds__(kThreads)
 k_overlap(const double2* __restrict__ ref, const double2* __restrict__ ap, uint64_t len, dd* __restrict__ part) {
+    constexpr int kIn = 4;  // entries in flight per thread: one at a time left the loads' latency exposed
     dd rr{0, 0}, aa{0, 0}, re{0, 0}, im{0, 0};
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += (uint64_t)gridDim.x * blockDim.x) {
-        const double2 r = ref[i], a = ap[i];
-        rr = dd_add(rr, r.x * r.x + r.y * r.y);
-        aa = dd_add(aa, a.x * a.x + a.y * a.y);
-        re = dd_add(re, r.x * a.x + r.y * a.y);   // <ref, ap> = sum conj(ref) * ap
-        im = dd_add(im, r.x * a.y - r.y * a.x);
+    const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < len; i += kIn * stride) {
+        double2 r[kIn], a[kIn];
+#pragma unroll
+        for (int j = 0; j < kIn; ++j)
+            if (i + j * stride < len) {
+                r[j] = ref[i + j * stride];
+                a[j] = ap[i + j * stride];
+            }
+#pragma unroll
+        for (int j = 0; j < kIn; ++j)
+            if (i + j * stride < len) {
+                rr = dd_add(rr, r[j].x * r[j].x + r[j].y * r[j].y);
+                aa = dd_add(aa, a[j].x * a[j].x + a[j].y * a[j].y);
+                re = dd_add(re, r[j].x * a[j].x + r[j].y * a[j].y);   // <ref, ap> = sum conj(ref) * ap
+                im = dd_add(im, r[j].x * a[j].y - r[j].y * a[j].x);
+            }
     }
     rr = block_sum_dd(rr);
     aa = block_sum_dd(aa);
@@ -647,12 +661,14 @@ k_overlap(const double2* __restrict__ ref, const double2* __restrict__ ap, uint6
     }
 }
 
-__global__ void k_overlap_final(const dd* __restrict__ part, int nparts, double* __restrict__ out) {
-    const int q = threadIdx.x;
-    if (q >= 4) return;
-    dd s{0, 0};
-    for (int p = 0; p < nparts; ++p) s = dd_add(s, part[4 * p + q]);
-    out[q] = s.hi + s.lo;
+// A thread per partial sum (four threads walking the 256 of them took 24 us, the first pass 9).
+__global__ void __launch_bounds__(kThreads)
+k_overlap_final(const dd* __restrict__ part, double* __restrict__ out) {
+#pragma unroll
+    for (int q = 0; q < 4; ++q) {
+        const dd s = block_sum_dd(part[4 * threadIdx.x + q]);
+        if (threadIdx.x == 0) out[q] = s.hi + s.lo;
+    }
 }
 
 }  // namespace
@@ -712,10 +728,9 @@ extern "C" int dcs_overlap(const double* ref, const double* ap, uint64_t len, do
         return DCS_E_ARG;
     }
     cudaStream_t s = (cudaStream_t)stream;
-    const int parts = 256;
-    k_overlap<<<parts, kThreads, 0, s>>>((const double2*)ref, (const double2*)ap, len, (dd*)scratch);
+    k_overlap<<<kOverlapParts, kThreads, 0, s>>>((const double2*)ref, (const double2*)ap, len, (dd*)scratch);
     DCS_CHECK_LAUNCH("k_overlap");
-    k_overlap_final<<<1, 32, 0, s>>>((const dd*)scratch, parts, out);
+    k_overlap_final<<<1, kThreads, 0, s>>>((const dd*)scratch, out);
     DCS_CHECK_LAUNCH("k_overlap_final");
     return DCS_OK;
 }
