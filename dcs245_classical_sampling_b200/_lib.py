@@ -26,7 +26,7 @@ STEP_DTYPE = np.dtype([
 ])
 PARAM_DTYPE = np.dtype([("f0r", "<f8"), ("f0i", "<f8"), ("f1r", "<f8"), ("f1i", "<f8"),
                         ("ov", "<i4"), ("y", "<i4")])
-SCALE_DTYPE = np.dtype([("logscale", "<f8"), ("exponent_sum", "<i8"), ("flags", "<u4"), ("pad", "<u4"),
+SCALE_DTYPE = np.dtype([("logscale", "<f8"), ("exponent_sum", "<i8"), ("flags", "<u4"), ("table_exp", "<i4"),
                         ("phase", "<f8")])
 GROUP_DTYPE = np.dtype([
     ("first", "<i4"), ("count", "<i4"), ("tile_dim", "<i4"), ("low_bits", "<i4"),
@@ -71,6 +71,7 @@ SIGNATURES = {
     "dcs_slice_steps_batched": (_I, [_I, _P, _U64, _P, _P, _U64, _I, _I, _I, _P, _P, _I, _P]),
     "dcs_fused_groups": (_I, [_P, _P, _I, _P, _I, _P, _P, _I, _I, _P, _P, _P]),
     "dcs_fused_runs": (_I, [_P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P]),
+    "dcs_tile_groups": (_I, [_I, _P, _U64, _P, _I, _P, _I, _P, _P, _U64, _P, _U64, _P, _I, _P]),
     "dcs_accumulate_batched": (_I, [_I, _P, _U64, _I, _P, _I, _P, _P, _P, _P, _I, _D, _P, _P, _U64, _P, _I, _I,
                                     _P]),
     "dcs_block_tail": (_I, [_P, _I, _P, _P, _I, _P]),

@@ -49,7 +49,12 @@ k_accumulate(const S* __restrict__ table, uint64_t table_stride, const __grid_co
             uint32_t i = 0;
             for (int j = 0; j < tm.tr; ++j) i |= (uint32_t)(__popc(sv & tm.linv[j]) & 1) << j;
             const uint64_t c = deposit(i, tm.runs, tm.nruns);
-            const double2 v = entry_f64(table[(uint64_t)it * table_stride + c]);
+            double2 v = entry_f64(table[(uint64_t)it * table_stride + c]);
+            if (sc.table_exp) {  // exact
+                const double p2 = ldexp(1.0, -sc.table_exp);
+                v.x *= p2;
+                v.y *= p2;
+            }
             const double m = exp(sc.logscale - log_shift);
             double cr = coefs[2 * it] * m, ci = coefs[2 * it + 1] * m;
             if (sc.phase != 0.0) {  // step factors divided out by the plan-specialised kernels

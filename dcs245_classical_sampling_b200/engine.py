@@ -14,7 +14,9 @@ Execution modes (``alloc(..., mode=...)``):
   launch (the reference's control flow, ``kernel_opt/inplace_gpu.py:107-124``);
 * ``"device"`` — the renormalisation stays on the device; all steps of all slices are
   enqueued without host synchronisation, several slices (work items) per launch when the
-  HBM budget allows (default);
+  HBM budget allows (default).  complex64 and complex128 tables take up to 24 steps per launch,
+  tile by tile in shared memory (csrc/tiles.cu); binary16 tables, and step weights outside
+  ``TILE_WEIGHT_RANGE``, one step per launch;
 * ``"fused"``  — like ``device`` but several vertex steps per pass over the table
   (coset-tiled fused kernels; complex128 tables run the plan-specialised register-run kernels
   compiled in FP64, which is how the complex128 audit recontraction runs at full size).
@@ -44,6 +46,20 @@ FP64_FUSED_CONFIG = {"max_dim": 12, "low": 3, "max_steps": 24, "variant": 12, "p
 # shapes tried in order when a group of the plan fits no run of that shape (small plans)
 FP64_FALLBACK_CONFIGS = ({"low": 4, "grouping": "greedy"}, {"variant": 4}, {"variant": 4, "low": 4, "grouping": "greedy"},
                          {"variant": 4, "low": 2}, {"variant": 4, "low": 1, "grouping": "greedy"})
+
+
+TILE_STEPS = 24  # steps of a tile group: the most that one launch takes
+# Step weights that a tile group may run without a renormalisation inside: the larger weight of a free
+# step (the selected one of a fixed step) in [2^-3, 2^2].  A step then grows the largest entry by 2^4
+# at most, 24 of them by 2^96, inside the FP32 range.
+TILE_WEIGHT_RANGE = (0.125, 4.0)
+
+
+def tile_dim(maxslots):
+    """log2 of the tile entries of device mode's tile groups for tables of 2^maxslots entries: 12 where
+    the whole table is one tile or there are tiles for many SMs (2^22 entries, 16 slices: 1763 us
+    against 2680 with 11), 11 between (2^16 entries, a slice: 149 against 154 us with 12)."""
+    return 12 if maxslots <= 12 or maxslots >= 18 else 11
 
 
 def device_steps(steps):
@@ -292,6 +308,9 @@ class InplaceConditionalBlockGPU:
             self.jit_group_cfg = {int(g): tuple(c) for g, c in (cfg.get("group_cfg") or {}).items()}
             self.fplan = self._build_fplan()
             self.items = 1
+        # device mode: groups of steps per launch over shared-memory tiles (binary16 tables round after
+        # every step with that step's scale, so they keep one launch per step)
+        self.tplan = self._build_tplan() if mode == "device" and not half else None
         self.entry_bytes = entry
         self.table_dtype = torch.float16 if half else tdtype
         self.items_cap = self.items
@@ -377,6 +396,13 @@ class InplaceConditionalBlockGPU:
                              threads=getattr(self, "jit_threads", 256),
                              group_cfg=getattr(self, "jit_group_cfg", None))
         return fp
+
+    def _build_tplan(self, dim=None, low=3):
+        """The tile groups of device mode (csrc/tiles.cu): tiles of at most 2^dim entries."""
+        from .fused import build_fused_plan
+        if dim is None:
+            dim = tile_dim(self.plan.maxslots)
+        return build_fused_plan(self.plan, max_dim=dim, low=low, max_steps=TILE_STEPS)
 
     def set_fused_config(self, jit=None, minb=None, threads=None, group_cfg=None, **cfg):
         """Rebuild the fused plan with another tile shape (max_dim, low, max_steps, variant, pairs,
@@ -480,10 +506,12 @@ class InplaceConditionalBlockGPU:
                 begin.append(begin[-1] + sum(1 for it in chunk if it[0] == bb))
             chunks.append((c0, len(chunk), blocks_in[0], len(blocks_in), len(begin_all)))
             begin_all.extend(begin)
-        unit_ok = [all(self.unit_weights_ok(it[2]) for it in work[c0:c0 + cn]) if self.mode == "fused" else True
-                   for c0, cn, _, _, _ in chunks]
-        host_params = (np.concatenate([it[2] for it in work]) if n else
-                       np.zeros(1, _lib.PARAM_DTYPE)).view(np.int64)
+        all_params = np.concatenate([it[2] for it in work]) if n else np.zeros(1, _lib.PARAM_DTYPE)
+        if self.mode == "fused":
+            unit_ok = [all(self.unit_weights_ok(it[2]) for it in work[c0:c0 + cn]) for c0, cn, _, _, _ in chunks]
+        else:  # one look at the whole batch
+            unit_ok = [n == 0 or self.weights_ok(all_params.reshape(n, -1))] * len(chunks)
+        host_params = all_params.view(np.int64)
         coefs = np.zeros(2 * max(1, n), np.float64)
         xors = np.zeros(max(1, n), np.uint64)
         for i, (_, c, _, xo) in enumerate(work):
@@ -501,6 +529,21 @@ class InplaceConditionalBlockGPU:
                 "dev": dev,
                 "pinned": pinned, "params": dev[:o1], "coefs": dev[o1:o2].view(torch.float64),
                 "xors": dev[o2:o3], "begin": dev[o3:].to(torch.int32), "h2d_bytes": blob.nbytes}
+
+    def weights_ok(self, params):
+        """Whether an item's step weights can run the kernels of several steps per launch of this mode
+        (generated kernels, tile groups); else its batch runs the library kernels / single steps."""
+        if self.mode == "fused":
+            return self.unit_weights_ok(params)
+        return self.tile_weights_ok(params) if self.tplan is not None else True
+
+    def tile_weights_ok(self, params):
+        """Whether step weights (dcs_param arrays, the plan's steps on the last axis) stay inside
+        TILE_WEIGHT_RANGE."""
+        a0 = np.hypot(params["f0r"], params["f0i"])
+        a1 = np.hypot(params["f1r"], params["f1i"])
+        big = np.where(self.free_steps, np.maximum(a0, a1), np.where(params["y"] != 0, a1, a0))
+        return bool(np.all((big >= TILE_WEIGHT_RANGE[0]) & (big <= TILE_WEIGHT_RANGE[1])))
 
     def unit_weights_ok(self, params):
         """Whether an item's step weights (a dcs_param array) can run the plan-specialised kernels,
@@ -538,6 +581,13 @@ class InplaceConditionalBlockGPU:
                 if np.all(m2 == 0):
                     break  # the remaining steps act on zero tables (the reference returns None here)
             return
+        if self.tplan is not None and unit_ok:
+            f = self.tplan
+            _lib.check(lib.dcs_tile_groups(
+                self.dcode, _lib.ptr(self.table), self.table_stride, self.dsteps.ctypes.data, self.nsteps,
+                f.groups.ctypes.data, len(f.groups), f.tile_steps.ctypes.data, params_ptr, self.nsteps,
+                _lib.ptr(self.maxbits), nm, _lib.ptr(self.scale), n_items, st))
+            return
         _lib.check(lib.dcs_slice_steps_batched(
             self.dcode, _lib.ptr(self.table), self.table_stride, self.dsteps.ctypes.data, params_ptr,
             self.nsteps, self.nsteps, 0, self.nsteps, _lib.ptr(self.maxbits), _lib.ptr(self.scale), n_items, st))
@@ -554,8 +604,10 @@ class InplaceConditionalBlockGPU:
         out.zero_()
         for ci, (c0, cn, b0, nb, boff) in enumerate(prep["chunks"]):
             self._reset_items(cn)
-            self._run_steps(_lib.ptr(prep["params"]) + c0 * self.nsteps * entry, cn, prep["unit_ok"][ci])
-            launches += len(self.fplan.groups) if self.mode == "fused" else self.nsteps
+            ok = prep["unit_ok"][ci]
+            self._run_steps(_lib.ptr(prep["params"]) + c0 * self.nsteps * entry, cn, ok)
+            launches += (len(self.fplan.groups) if self.mode == "fused" else
+                         len(self.tplan.groups) if self.tplan is not None and ok else self.nsteps)
             flat = out[b0:b0 + nb].view(torch.float64)
             _lib.check(lib.dcs_accumulate_batched(
                 self.dcode, _lib.ptr(self.table), self.table_stride, self.plan.terminal_rank,

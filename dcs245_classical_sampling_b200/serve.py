@@ -95,7 +95,8 @@ class DeviceCircuit:
         for b in (0, 1):
             rows["f0r"][b::2], rows["f0i"][b::2] = fsel[:, 4 * b], fsel[:, 4 * b + 1]
             rows["f1r"][b::2], rows["f1i"][b::2] = fsel[:, 4 * b + 2], fsel[:, 4 * b + 3]
-        self.unit_ok = all(engine.unit_weights_ok(rows[b::2]) for b in (0, 1))
+        rows["y"] = np.hypot(rows["f0r"], rows["f0i"]) <= 1e-12  # the value that a fixed step's row selects
+        self.unit_ok = all(engine.weights_ok(rows[b::2]) for b in (0, 1))
         self.nsteps, self.nfixed = S, nfixed
         dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)
         self.fsel = dev(fsel)
@@ -298,7 +299,9 @@ class CircuitRunner:
         nm = eng._nmax() + 1
         for c0, cn, b0, nb, boff in chunks:
             eng._reset_items(cn)
-            eng._run_steps(_lib.ptr(self.d_params) + c0 * eng.nsteps * entry, cn)
+            # (fused mode: weights that the generated kernels cannot take have switched them off)
+            eng._run_steps(_lib.ptr(self.d_params) + c0 * eng.nsteps * entry, cn,
+                           self.dc.unit_ok or self.mode == "fused")
             _lib.check(lib.dcs_accumulate_batched(
                 eng.dcode, _lib.ptr(eng.table), eng.table_stride, eng.plan.terminal_rank,
                 eng.term_runs.ctypes.data, eng.term_nruns, eng.tbasis.ctypes.data,

@@ -104,7 +104,7 @@ typedef struct dcs_scale {
     double logscale;
     int64_t exponent_sum;
     uint32_t flags; /* bit 0: a nonfinite maximum was seen; bit 1: the table became zero */
-    uint32_t pad;
+    int32_t table_exp; /* the entries are the table's times 2^-table_exp (dcs_tile_groups; else 0) */
     double phase;   /* radians: the argument of the step factors the plan-specialised kernels divide
                        out of the weights (the table is e^{logscale + i phase} times its entries) */
 } dcs_scale;
@@ -275,6 +275,20 @@ int dcs_fused_groups(void *table, const dcs_step *steps, int nsteps, const dcs_g
 int dcs_fused_runs(void *table, const dcs_step *steps, int nsteps, const dcs_group *groups, int ngroups,
                    const dcs_tile_step *tile_steps, const dcs_tile_run *tile_runs, const dcs_param *params,
                    int g0, int ng, uint64_t *maxbits, dcs_scale *scale, void *stream);
+
+/* The same passes for `nitems` work items that share the plan, on complex64 or complex128 tables, with the
+ * per-step kernel's formulas (the entries, and in complex64 the scale record, have the bits of
+ * dcs_slice_steps_batched up to table_exp): groups
+ * [0, ngroups) in order, tiles of at most 2^12 entries.  Item i uses table + i*table_stride entries,
+ * params + i*param_stride, maxbits + i*maxbits_stride (word s + 1 receives the max of step s, for
+ * complex128 of a group's last step s only; word 0 holds the bits of 1.0) and scale + i (all zero on entry).  The table is renormalised once per group, so
+ * the weights of a group must not overflow or underflow the storage precision; the power of two that
+ * a complex64 table still has is in table_exp.  Steps 0 .. nsteps - 1
+ * in groups that follow one another; steps, groups, tile_steps: host arrays. */
+int dcs_tile_groups(int dtype, void *table, uint64_t table_stride, const dcs_step *steps, int nsteps,
+                    const dcs_group *groups, int ngroups, const dcs_tile_step *tile_steps, const dcs_param *params,
+                    uint64_t param_stride, uint64_t *maxbits, uint64_t maxbits_stride, dcs_scale *scale, int nitems,
+                    void *stream);
 
 /* Plan-specialised group kernels (no reference counterpart: the reference's kernels are fixed
  * sources compiled once).  A fused plan with register runs is turned into one CUDA kernel per
