@@ -192,6 +192,142 @@ class SliceParams:
         return count, out
 
 
+class DeviceCircuit:
+    """Static tables of one circuit for dcs_build_items (from the engine's host bookkeeping)."""
+
+    MAX_QUBITS = 64  # dcs_build_items takes a prefix as a 64-bit mask
+
+    def __init__(self, engine, device):
+        sp = engine.params
+        p = engine.plan
+        S = sp.nsteps
+        fsel = np.zeros((S, 8), np.float64)
+        xq = np.full(S, -1, np.int32)
+        fixidx = np.full(S, -1, np.int32)
+        ffull_ref = sp.full_vectors(np.zeros(p.n, np.int64))  # reference vertices do not depend on x
+        for j in range(S):
+            q = int(sp.keep[sp.vert[j]])
+            if q < p.n:
+                for b in (0, 1):
+                    row = sp.U[q, b]
+                    fsel[j, 4 * b:4 * b + 4] = [row[0].real, row[0].imag, row[1].real, row[1].imag]
+                xq[j] = q
+            else:
+                f = ffull_ref[q]
+                fsel[j, 0:4] = fsel[j, 4:8] = [f[0].real, f[0].imag, f[1].real, f[1].imag]
+        for a, j in enumerate(sp.fixed_pos):
+            fixidx[j] = a
+        nfixed = len(sp.fixed_pos)
+        fwords = (S + 31) // 32
+        F = np.zeros((max(1, nfixed), fwords), np.uint32)
+        for a in range(nfixed):
+            for t in np.flatnonzero(sp.F[a]):
+                F[a, t >> 5] |= np.uint32(1 << (t & 31))
+        tail = np.array([int(x) for x in sp.tail] + [0], np.uint64)
+        # slices: x-independent coefficients (slices are reference vertices) and flips
+        _, items = sp.items(np.zeros(p.n, np.uint8))
+        # items skip zero coefficients; recover each kept slice's flips from its bits
+        flips, coefs, freeflips = [], [], []
+        ff = ffull_ref
+        for bits in itertools.product((0, 1), repeat=sp.nslice):
+            bits = np.array(bits, np.int64)
+            coef = complex(np.prod([ff[s][b] for s, b in zip(p.slices, bits)])) if sp.nslice else 1 + 0j
+            par = sum(int(bits[p.slices.index(a)]) * int(bits[p.slices.index(b)]) for a, b in p.slice_edges)
+            coef *= (-1) ** par
+            if not coef:
+                continue
+            fl = (bits @ sp.nbr) & 1 if sp.nslice else np.zeros(p.N, np.int64)
+            flips.append(fl[sp.vert].astype(np.uint8))
+            coefs.append(coef)
+            freeflips.append(sum(int(fl[q]) << jj for jj, q in enumerate(sp.open_red)))
+        self.nslices = len(coefs)
+        assert self.nslices == len(items)
+        # the plan-specialised kernels divide f0 out of the free steps' weights: every weight row
+        # a prefix can select (slices flip only f1) must pass the engine's check
+        rows = np.zeros(2 * S, _lib.PARAM_DTYPE)
+        for b in (0, 1):
+            rows["f0r"][b::2], rows["f0i"][b::2] = fsel[:, 4 * b], fsel[:, 4 * b + 1]
+            rows["f1r"][b::2], rows["f1i"][b::2] = fsel[:, 4 * b + 2], fsel[:, 4 * b + 3]
+        rows["y"] = np.hypot(rows["f0r"], rows["f0i"]) <= 1e-12  # the value that a fixed step's row selects
+        self.unit_ok = all(engine.weights_ok(rows[b::2]) for b in (0, 1))
+        self.nsteps, self.nfixed = S, nfixed
+        dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)
+        self.fsel = dev(fsel)
+        self.xq = dev(xq)
+        self.fixidx = dev(fixidx)
+        self.flip = dev(np.stack(flips).astype(np.uint8))
+        self.F = dev(F)
+        self.tail = dev(tail.view(np.int64))
+        self.coef = dev(np.array([[c.real, c.imag] for c in coefs], np.float64).reshape(-1))
+        self.freeflip = dev(np.array(freeflips, np.uint64).view(np.int64))
+        self.closed = dev(np.array([q for q in range(p.n) if q not in set(p.open_full)], np.int32))
+
+    @classmethod
+    def of(cls, engine):
+        """The tables of an engine's circuit, or None where dcs_build_items cannot build its items: more
+        qubits than a mask has bits, or no slice with a nonzero coefficient."""
+        if engine.n > cls.MAX_QUBITS or not engine.params.nsteps:
+            return None
+        return cls(engine, engine.device) if engine.params.items(np.zeros(engine.n, np.uint8))[1] else None
+
+    def build(self, lib, xbits, nsamples, params, coefs, xors, stream):
+        _lib.check(lib.dcs_build_items(
+            _lib.ptr(self.fsel), _lib.ptr(self.xq), _lib.ptr(self.fixidx), _lib.ptr(self.flip), _lib.ptr(self.F),
+            _lib.ptr(self.tail), _lib.ptr(self.coef), _lib.ptr(self.freeflip), self.nsteps, self.nfixed,
+            self.nslices, _lib.ptr(xbits), nsamples, _lib.ptr(params), _lib.ptr(coefs), _lib.ptr(xors), stream))
+
+
+def prefix_masks(x_list, n):
+    """The prefixes' first n bits as 64-bit masks (bit q of data vertex q), or None where one of them
+    is not n or more values 0 / 1 (the host bookkeeping then says what it makes of it)."""
+    if n > DeviceCircuit.MAX_QUBITS or not len(x_list):
+        return None
+    try:
+        x = np.asarray([np.asarray(v)[:n] for v in x_list])
+    except (ValueError, TypeError, IndexError):
+        return None
+    if x.ndim != 2 or x.shape[1] != n or x.dtype.kind not in "bui" or x.min(initial=0) < 0 or x.max(initial=0) > 1:
+        return None
+    bits = np.zeros((len(x), 64), np.uint8)
+    bits[:, :n] = x
+    return np.packbits(bits, axis=1, bitorder="little").view(np.uint64).reshape(-1)
+
+
+def item_chunks(nblocks, nslices, cap):
+    """Launch chunks of at most cap work items (nslices per block, in block order): a list of (first item,
+    items, first block, blocks, offset of the chunk's item ranges), and the ranges."""
+    chunks, begins = [], []
+    for c0 in range(0, nblocks * nslices, cap):
+        cn = min(cap, nblocks * nslices - c0)
+        b0, b1 = c0 // nslices, (c0 + cn - 1) // nslices
+        chunks.append((c0, cn, b0, b1 - b0 + 1, len(begins)))
+        begins.extend([0] + [min((b + 1) * nslices, c0 + cn) - c0 for b in range(b0, b1 + 1)])
+    return chunks, begins
+
+
+def device_batch(engine, masks):
+    """The work items of whole prefixes (masks), built on the device by dcs_build_items: one upload of the
+    masks and the chunks' block ranges, no host work per item."""
+    B, L = len(masks), engine.dc.nslices
+    n = B * L
+    chunks, begins = item_chunks(B, L, engine.items)
+    words = (len(begins) + 1) // 2
+    pinned = torch.empty(B + words, dtype=torch.int64).pin_memory()
+    host = pinned.numpy()
+    host[:B] = masks.view(np.int64)
+    host[B:].view(np.int32)[:len(begins)] = begins
+    o1 = n * engine.dc.nsteps * (_lib.PARAM_DTYPE.itemsize // 8)
+    o2, o3 = o1 + 2 * n, o1 + 3 * n
+    dev = torch.empty(o3 + B + words, dtype=torch.int64, device=engine.device)
+    dev[o3:].copy_(pinned, non_blocking=True)
+    params, coefs, xors = dev[:o1], dev[o1:o2].view(torch.float64), dev[o2:o3]
+    engine.dc.build(engine.lib, dev[o3:], B, params, coefs, xors, engine._stream())
+    return {"n_items": n, "chunks": chunks, "unit_ok": [True] * len(chunks),
+            "counts": [1 << len(engine.plan.slices)] * B, "nblocks": B, "dev": dev, "pinned": pinned,
+            "params": params, "coefs": coefs, "xors": xors, "begin": dev[o3 + B:].view(torch.int32),
+            "h2d_bytes": pinned.numel() * 8}
+
+
 class DeviceBlock(torch.Tensor):
     """What ``block`` returns: the complex128 block as a CUDA tensor that host code can copy the
     way the reference's worker copies CuPy arrays (``host = cp.asnumpy(v)``,
@@ -343,6 +479,7 @@ class InplaceConditionalBlockGPU:
             u[q] = [m[0, 0].real, m[0, 0].imag, m[0, 1].real, m[0, 1].imag,
                     m[1, 0].real, m[1, 0].imag, m[1, 1].real, m[1, 1].imag]
         self.u_open = u
+        self.dc = DeviceCircuit.of(self)
         self._alloc = True
         self.buf = True
 
@@ -483,10 +620,16 @@ class InplaceConditionalBlockGPU:
             self.table.view(self.items, self.table_stride)[:n_items, 0] = 1
 
     def prepare(self, x_list, w=None, part=0, parts=1):
-        """Host bookkeeping for a batch of prefixes and ONE host->device upload.
+        """The work items of a batch of prefixes, on the device.
 
         Work items are the (prefix, slice) pairs with a nonzero slice coefficient, in prefix
-        order then slice order; they run `self.items` at a time."""
+        order then slice order; they run `self.items` at a time.  Whole batches with the default
+        reference bras are built there from the prefix masks (dcs_build_items); otherwise the host
+        builds them and uploads them once."""
+        if w is None and parts == 1 and part == 0 and self.dc is not None and self.dc.unit_ok:
+            masks = prefix_masks(x_list, self.n)
+            if masks is not None:
+                return device_batch(self, masks)
         work, counts = [], []
         for b, x in enumerate(x_list):
             cnt, items = self.params.items(x, w, part, parts)

@@ -21,7 +21,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .engine import DeviceBlock, SliceParams, pack_runs
+from .engine import DeviceBlock, DeviceCircuit, SliceParams, device_batch, pack_runs, prefix_masks
 from .plan import build_block_plan, build_gather_plan
 
 
@@ -104,23 +104,26 @@ class ConditionalBlockGPU:
             u[q] = [m[0, 0].real, m[0, 0].imag, m[0, 1].real, m[0, 1].imag,
                     m[1, 0].real, m[1, 0].imag, m[1, 1].real, m[1, 1].imag]
         self.u_open = u
+        self.dc = DeviceCircuit.of(self)
         self._alloc = True
 
-    def _stream(self):
-        return torch.cuda.current_stream(self.device).cuda_stream
+    def weights_ok(self, params):
+        """Every step weight runs the gather kernel."""
+        return True
 
-    def block(self, x_bits, w=None, part=0, parts=1):
-        """Scaled conditional amplitudes of one prefix (conditional_block_gpu.py:128-177)."""
-        if not self._alloc:
-            self.alloc()
-        start = time.perf_counter()
+    def _prepare(self, x_bits, w, part, parts):
+        """The block's work items on the device: (slices evaluated, chunks of (items, params, coefs,
+        xors, item range) as device addresses, what keeps them alive)."""
+        if w is None and part == 0 and parts == 1 and self.dc is not None:
+            masks = prefix_masks([x_bits], self.n)
+            if masks is not None:
+                p = device_batch(self, masks)
+                entry = _lib.PARAM_DTYPE.itemsize * len(self.steps)
+                return p["counts"][0], [(cn, _lib.ptr(p["params"]) + c0 * entry, _lib.ptr(p["coefs"]) + 16 * c0,
+                                         _lib.ptr(p["xors"]) + 8 * c0, _lib.ptr(p["begin"]) + 4 * boff)
+                                        for c0, cn, _, _, boff in p["chunks"]], p
         count, items = self.params.items(x_bits, w, part, parts)
-        lib, st = self.lib, self._stream()
-        out = torch.zeros((1, 1 << self.k), dtype=torch.complex128, device=self.device)
-        flags = torch.zeros(self.items, dtype=torch.int64, device=self.device)
-        S = len(self.steps)
-        final = self.tab[S & 1]  # step s reads table s % 2
-        sw = _lib.SCALE_DTYPE.itemsize // 8
+        chunks, keep = [], []
         for c0 in range(0, len(items), self.items):
             chunk = items[c0:c0 + self.items]
             cn = len(chunk)
@@ -131,19 +134,39 @@ class ConditionalBlockGPU:
                                                     np.array([0, cn], np.int64)])).to(self.device)
             o1, o2, o3 = host.size, host.size + coefs.size, host.size + coefs.size + xors.size
             begin = blob[o3:].to(torch.int32)
+            keep.append((blob, begin))
+            chunks.append((cn, _lib.ptr(blob), _lib.ptr(blob) + 8 * o1, _lib.ptr(blob) + 8 * o2, _lib.ptr(begin)))
+        return count, chunks, keep
+
+    def _stream(self):
+        return torch.cuda.current_stream(self.device).cuda_stream
+
+    def block(self, x_bits, w=None, part=0, parts=1):
+        """Scaled conditional amplitudes of one prefix (conditional_block_gpu.py:128-177)."""
+        if not self._alloc:
+            self.alloc()
+        start = time.perf_counter()
+        count, chunks, keep = self._prepare(x_bits, w, part, parts)
+        lib, st = self.lib, self._stream()
+        out = torch.zeros((1, 1 << self.k), dtype=torch.complex128, device=self.device)
+        flags = torch.zeros(self.items, dtype=torch.int64, device=self.device)
+        S = len(self.steps)
+        final = self.tab[S & 1]  # step s reads table s % 2
+        sw = _lib.SCALE_DTYPE.itemsize // 8
+        for cn, d_params, d_coefs, d_xors, d_begin in chunks:
             mb = self.maxbits[: cn * self.nm].view(cn, self.nm)
             mb.zero_()
             mb[:, 0] = self.one_bits
             self.scale[: cn * sw].zero_()
             self.tab[0].view(self.items, self.stride)[:cn, 0] = 1  # empty environment (gpu_kernel.py:132)
             _lib.check(lib.dcs_gather_steps(self.dcode, _lib.ptr(self.tab[0]), _lib.ptr(self.tab[1]), self.stride,
-                                            self.dsteps.ctypes.data, _lib.ptr(self.words), _lib.ptr(blob), S, 0, S,
+                                            self.dsteps.ctypes.data, _lib.ptr(self.words), d_params, S, 0, S,
                                             _lib.ptr(self.maxbits), self.nm, _lib.ptr(self.scale), cn, st))
             _lib.check(lib.dcs_accumulate_batched(
                 self.dcode, _lib.ptr(final), self.stride, self.terminal_rank, self.term_runs.ctypes.data,
-                self.term_nruns, self.tbasis.ctypes.data, _lib.ptr(blob) + 8 * o2, _lib.ptr(blob) + 8 * o1,
-                _lib.ptr(begin), 1, self.params.shift, _lib.ptr(self.scale), _lib.ptr(self.maxbits[self.nm - 1:]),
-                self.nm, _lib.ptr(out.view(torch.float64)), self.k, cn, st))
+                self.term_nruns, self.tbasis.ctypes.data, d_xors, d_coefs, d_begin, 1, self.params.shift,
+                _lib.ptr(self.scale), _lib.ptr(self.maxbits[self.nm - 1:]), self.nm,
+                _lib.ptr(out.view(torch.float64)), self.k, cn, st))
             flags[:cn] |= self.scale[: cn * sw].view(cn, sw)[:, 2]
         _lib.check(lib.dcs_block_tail(_lib.ptr(out), self.k, self.adj_hi.ctypes.data, self.u_open.ctypes.data, 1, st))
         if bool(((flags & 1) != 0).any()):

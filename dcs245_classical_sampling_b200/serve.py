@@ -37,83 +37,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .engine import InplaceConditionalBlockGPU
-
-
-class DeviceCircuit:
-    """Static tables of one circuit for dcs_build_items (from the engine's host bookkeeping)."""
-
-    def __init__(self, engine, device):
-        sp = engine.params
-        p = engine.plan
-        S = sp.nsteps
-        fsel = np.zeros((S, 8), np.float64)
-        xq = np.full(S, -1, np.int32)
-        fixidx = np.full(S, -1, np.int32)
-        ffull_ref = sp.full_vectors(np.zeros(p.n, np.int64))  # reference vertices do not depend on x
-        for j in range(S):
-            q = int(sp.keep[sp.vert[j]])
-            if q < p.n:
-                for b in (0, 1):
-                    row = sp.U[q, b]
-                    fsel[j, 4 * b:4 * b + 4] = [row[0].real, row[0].imag, row[1].real, row[1].imag]
-                xq[j] = q
-            else:
-                f = ffull_ref[q]
-                fsel[j, 0:4] = fsel[j, 4:8] = [f[0].real, f[0].imag, f[1].real, f[1].imag]
-        for a, j in enumerate(sp.fixed_pos):
-            fixidx[j] = a
-        nfixed = len(sp.fixed_pos)
-        fwords = (S + 31) // 32
-        F = np.zeros((max(1, nfixed), fwords), np.uint32)
-        for a in range(nfixed):
-            for t in np.flatnonzero(sp.F[a]):
-                F[a, t >> 5] |= np.uint32(1 << (t & 31))
-        tail = np.array([int(x) for x in sp.tail] + [0], np.uint64)
-        # slices: x-independent coefficients (slices are reference vertices) and flips
-        _, items = sp.items(np.zeros(p.n, np.uint8))
-        # items skip zero coefficients; recover each kept slice's flips from its bits
-        import itertools
-        flips, coefs, freeflips = [], [], []
-        ff = ffull_ref
-        for bits in itertools.product((0, 1), repeat=sp.nslice):
-            bits = np.array(bits, np.int64)
-            coef = complex(np.prod([ff[s][b] for s, b in zip(p.slices, bits)])) if sp.nslice else 1 + 0j
-            par = sum(int(bits[p.slices.index(a)]) * int(bits[p.slices.index(b)]) for a, b in p.slice_edges)
-            coef *= (-1) ** par
-            if not coef:
-                continue
-            fl = (bits @ sp.nbr) & 1 if sp.nslice else np.zeros(p.N, np.int64)
-            flips.append(fl[sp.vert].astype(np.uint8))
-            coefs.append(coef)
-            freeflips.append(sum(int(fl[q]) << jj for jj, q in enumerate(sp.open_red)))
-        self.nslices = len(coefs)
-        assert self.nslices == len(items)
-        # the plan-specialised kernels divide f0 out of the free steps' weights: every weight row
-        # a prefix can select (slices flip only f1) must pass the engine's check
-        rows = np.zeros(2 * S, _lib.PARAM_DTYPE)
-        for b in (0, 1):
-            rows["f0r"][b::2], rows["f0i"][b::2] = fsel[:, 4 * b], fsel[:, 4 * b + 1]
-            rows["f1r"][b::2], rows["f1i"][b::2] = fsel[:, 4 * b + 2], fsel[:, 4 * b + 3]
-        rows["y"] = np.hypot(rows["f0r"], rows["f0i"]) <= 1e-12  # the value that a fixed step's row selects
-        self.unit_ok = all(engine.weights_ok(rows[b::2]) for b in (0, 1))
-        self.nsteps, self.nfixed = S, nfixed
-        dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)
-        self.fsel = dev(fsel)
-        self.xq = dev(xq)
-        self.fixidx = dev(fixidx)
-        self.flip = dev(np.stack(flips).astype(np.uint8))
-        self.F = dev(F)
-        self.tail = dev(tail.view(np.int64))
-        self.coef = dev(np.array([[c.real, c.imag] for c in coefs], np.float64).reshape(-1))
-        self.freeflip = dev(np.array(freeflips, np.uint64).view(np.int64))
-        self.closed = dev(np.array([q for q in range(p.n) if q not in set(p.open_full)], np.int32))
-
-    def build(self, lib, xbits, nsamples, params, coefs, xors, stream):
-        _lib.check(lib.dcs_build_items(
-            _lib.ptr(self.fsel), _lib.ptr(self.xq), _lib.ptr(self.fixidx), _lib.ptr(self.flip), _lib.ptr(self.F),
-            _lib.ptr(self.tail), _lib.ptr(self.coef), _lib.ptr(self.freeflip), self.nsteps, self.nfixed,
-            self.nslices, _lib.ptr(xbits), nsamples, _lib.ptr(params), _lib.ptr(coefs), _lib.ptr(xors), stream))
+from .engine import DeviceCircuit, InplaceConditionalBlockGPU, item_chunks
 
 
 class TablePool:
@@ -228,7 +152,7 @@ class CircuitRunner:
                           external_table=pool is not None)
         self.item_bytes = self.engine.table_item_bytes()
         self.lib = _lib.load()
-        self.dc = DeviceCircuit(self.engine, self.device)
+        self.dc = self.engine.dc or DeviceCircuit(self.engine, self.device)
         assert self.dc.nslices == L
         if self.mode == "fused" and self.engine.jit and not self.dc.unit_ok:
             self.engine.set_fused_config(jit=False)  # weights the plan-specialised kernels cannot take
@@ -273,16 +197,7 @@ class CircuitRunner:
 
     def _chunks(self, n):
         """Launch chunks of engine.items work items and, per chunk, the item ranges of its blocks."""
-        L, cap = self.dc.nslices, self.engine.items
-        items = n * L
-        chunks, begins = [], []
-        for c0 in range(0, items, cap):
-            cn = min(cap, items - c0)
-            b0, b1 = c0 // L, (c0 + cn - 1) // L
-            bl = [0] + [min((b + 1) * L, c0 + cn) - c0 for b in range(b0, b1 + 1)]
-            chunks.append((c0, cn, b0, b1 - b0 + 1, len(begins)))
-            begins.extend(bl)
-        return chunks, begins
+        return item_chunks(n, self.dc.nslices, self.engine.items)
 
     def _device_work(self, n, chunks):
         """Every device step of a batch of n samples after the id upload, on self.stream, with
