@@ -71,6 +71,8 @@ SIGNATURES = {
     "dcs_slice_steps_batched": (_I, [_I, _P, _U64, _P, _P, _U64, _I, _I, _I, _P, _P, _I, _P]),
     "dcs_fused_groups": (_I, [_P, _P, _I, _P, _I, _P, _P, _I, _I, _P, _P, _P]),
     "dcs_fused_runs": (_I, [_P, _P, _I, _P, _I, _P, _P, _P, _I, _I, _P, _P, _P]),
+    "dcs_begin_items": (_I, [_I, _P, _U64, _P, _U64, _P, _I, _P]),
+    "dcs_collect_flags": (_I, [_P, _P, _I, _P]),
     "dcs_tile_groups": (_I, [_I, _P, _U64, _P, _I, _P, _I, _P, _P, _U64, _P, _U64, _P, _I, _P]),
     "dcs_accumulate_batched": (_I, [_I, _P, _U64, _I, _P, _I, _P, _P, _P, _P, _I, _D, _P, _P, _U64, _P, _I, _I,
                                     _P]),

@@ -267,6 +267,27 @@ int launch_step(M* table, uint64_t table_stride, const dcs_step& st, int s, cons
     return DCS_E_ARG;
 }
 
+// Initial state of a batch's work items, one CTA per item: the empty environment (entry 0 = 1), the maxima
+// (word 0 = the bits of 1, the others 0) and the scale.  One launch instead of four fills.
+template <class M>
+__global__ void __launch_bounds__(256)
+k_begin(M* __restrict__ table, uint64_t table_stride, M one, unsigned long long* __restrict__ maxbits,
+        uint64_t maxbits_stride, unsigned long long one_bits, dcs_scale* __restrict__ scale) {
+    const int item = blockIdx.x;
+    unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
+    for (uint64_t i = threadIdx.x; i < maxbits_stride; i += 256) mb[i] = i ? 0ull : one_bits;
+    if (threadIdx.x == 0) {
+        table[(uint64_t)item * table_stride] = one;
+        scale[item] = dcs_scale{0.0, 0, 0u, 0, 0.0};
+    }
+}
+
+__global__ void __launch_bounds__(256)
+k_collect_flags(const dcs_scale* __restrict__ scale, int64_t* __restrict__ flags, int nitems) {
+    const int i = blockIdx.x * 256 + threadIdx.x;
+    if (i < nitems) flags[i] |= (int64_t)scale[i].flags;
+}
+
 int validate_step(const dcs_step& st, int s) {
     if (st.kind < 0 || st.kind > 7) { dcs_host::set_error("step %d: kind %d out of range", s, st.kind); return DCS_E_ARG; }
     if (st.m < 0 || st.m > DCS_MAX_SLOTS) { dcs_host::set_error("step %d: m=%d out of range", s, st.m); return DCS_E_ARG; }
@@ -354,4 +375,40 @@ extern "C" int dcs_slice_steps(int dtype, void* table, const dcs_step* steps, co
                                int first, int count, uint64_t* maxbits, dcs_scale* scale, void* stream) {
     return dcs_slice_steps_batched(dtype, table, 0, steps, params, 0, nsteps, first, count, maxbits, scale, 1,
                                    stream);
+}
+
+extern "C" int dcs_begin_items(int dtype, void* table, uint64_t table_stride, uint64_t* maxbits,
+                               uint64_t maxbits_stride, dcs_scale* scale, int nitems, void* stream) {
+    if (!table || !maxbits || !scale || nitems < 1 || maxbits_stride < 1) {
+        dcs_host::set_error("dcs_begin_items: invalid arguments");
+        return DCS_E_ARG;
+    }
+    cudaStream_t st = (cudaStream_t)stream;
+    unsigned long long* mb = (unsigned long long*)maxbits;
+    constexpr unsigned long long one32 = 0x3f800000ull, one64 = 0x3ff0000000000000ull;  // 1.0f, 1.0
+    if (dtype == DCS_C64)
+        k_begin<<<nitems, 256, 0, st>>>((float2*)table, table_stride, make_float2(1.f, 0.f), mb, maxbits_stride, one32,
+                                        scale);
+    else if (dtype == DCS_C128)
+        k_begin<<<nitems, 256, 0, st>>>((double2*)table, table_stride, make_double2(1.0, 0.0), mb, maxbits_stride, one64,
+                                        scale);
+    else if (dtype == DCS_H16)
+        k_begin<<<nitems, 256, 0, st>>>((ushort2*)table, table_stride, make_ushort2(0x3c00, 0), mb, maxbits_stride,
+                                        one64, scale);  // binary16 1
+    else {
+        dcs_host::set_error("dcs_begin_items: unknown dtype %d", dtype);
+        return DCS_E_ARG;
+    }
+    DCS_CHECK_LAUNCH("k_begin launch");
+    return DCS_OK;
+}
+
+extern "C" int dcs_collect_flags(const dcs_scale* scale, int64_t* flags, int nitems, void* stream) {
+    if (!scale || !flags || nitems < 1) {
+        dcs_host::set_error("dcs_collect_flags: invalid arguments");
+        return DCS_E_ARG;
+    }
+    k_collect_flags<<<(nitems + 255) / 256, 256, 0, (cudaStream_t)stream>>>(scale, flags, nitems);
+    DCS_CHECK_LAUNCH("k_collect_flags launch");
+    return DCS_OK;
 }

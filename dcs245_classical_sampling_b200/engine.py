@@ -606,18 +606,11 @@ class InplaceConditionalBlockGPU:
     def _stream(self):
         return torch.cuda.current_stream(self.device).cuda_stream
 
-    def _reset_items(self, n_items):
-        mb = self._mb()
-        mb[:n_items].zero_()
-        mb[:n_items, 0] = self.one_bits
-        self._sc()[:n_items].zero_()
-        # empty environment = 1 at address 0 of every item (inplace_gpu.py:108)
-        if getattr(self, "half", False):
-            t = self.table.view(self.items, self.table_stride, 2)
-            t[:n_items, 0, 0] = 1
-            t[:n_items, 0, 1] = 0
-        else:
-            self.table.view(self.items, self.table_stride)[:n_items, 0] = 1
+    def _reset_items(self, n_items, st=None):
+        """The empty environment (1 at address 0 of every item, inplace_gpu.py:108), the maxima and the scale."""
+        _lib.check(self.lib.dcs_begin_items(self.dcode, _lib.ptr(self.table), self.table_stride,
+                                            _lib.ptr(self.maxbits), self._nmax() + 1, _lib.ptr(self.scale), n_items,
+                                            self._stream() if st is None else st))
 
     def prepare(self, x_list, w=None, part=0, parts=1):
         """The work items of a batch of prefixes, on the device.
@@ -696,8 +689,9 @@ class InplaceConditionalBlockGPU:
         a0 = np.hypot(p["f0r"], p["f0i"])
         return bool(np.all(a0 > 0) and np.all(np.hypot(p["f1r"], p["f1i"]) <= 2.0 ** 32 * a0))
 
-    def _run_steps(self, params_ptr, n_items, unit_ok=True):
-        lib, st = self.lib, self._stream()
+    def _run_steps(self, params_ptr, n_items, unit_ok=True, st=None):
+        lib = self.lib
+        st = self._stream() if st is None else st
         nm = self._nmax() + 1
         if self.mode == "fused":
             f = self.fplan
@@ -740,30 +734,33 @@ class InplaceConditionalBlockGPU:
         every work item, accumulation, tail.  No host synchronisation (except in "plain" mode).
         flags: optional (self.items,) int64 device tensor that collects the items' scale flags
         (bit 0: a nonfinite table).  Returns the number of library kernel launches."""
-        lib = self.lib
+        lib, st = self.lib, self._stream()
         nm = self._nmax() + 1
         entry = _lib.PARAM_DTYPE.itemsize
         launches = 0
         out.zero_()
+        d_params, d_coefs, d_xors, d_begin = (_lib.ptr(prep[k]) for k in ("params", "coefs", "xors", "begin"))
         for ci, (c0, cn, b0, nb, boff) in enumerate(prep["chunks"]):
-            self._reset_items(cn)
+            self._reset_items(cn, st)
             ok = prep["unit_ok"][ci]
-            self._run_steps(_lib.ptr(prep["params"]) + c0 * self.nsteps * entry, cn, ok)
+            self._run_steps(d_params + c0 * self.nsteps * entry, cn, ok, st)
             launches += (len(self.fplan.groups) if self.mode == "fused" else
                          len(self.tplan.groups) if self.tplan is not None and ok else self.nsteps)
-            flat = out[b0:b0 + nb].view(torch.float64)
             _lib.check(lib.dcs_accumulate_batched(
                 self.dcode, _lib.ptr(self.table), self.table_stride, self.plan.terminal_rank,
                 self.term_runs.ctypes.data, self.term_nruns, self.tbasis.ctypes.data,
-                _lib.ptr(prep["xors"]) + 8 * c0, _lib.ptr(prep["coefs"]) + 16 * c0,
-                _lib.ptr(prep["begin"]) + 4 * boff, nb, self.params.shift, _lib.ptr(self.scale),
-                _lib.ptr(self.maxbits[nm - 1:]), nm, _lib.ptr(flat), self.k, cn, self._stream()))
-            launches += 2
+                d_xors + 8 * c0, d_coefs + 16 * c0,
+                d_begin + 4 * boff, nb, self.params.shift, _lib.ptr(self.scale),
+                _lib.ptr(self.maxbits) + 8 * (nm - 1), nm, _lib.ptr(out) + (b0 << (self.k + 4)), self.k, cn, st))
+            launches += 3
             if flags is not None:
-                flags[:cn] |= self._sc()[:cn, 2]
+                if flags.dtype != torch.int64 or not flags.is_cuda or not flags.is_contiguous() or flags.numel() < cn:
+                    raise ValueError("flags must be a contiguous int64 device tensor of engine.items elements")
+                _lib.check(lib.dcs_collect_flags(_lib.ptr(self.scale), _lib.ptr(flags), cn, st))
+                launches += 1
         _lib.check(lib.dcs_block_tail(_lib.ptr(out), self.k, self.adj_hi.ctypes.data, self.u_open.ctypes.data,
-                                      prep["nblocks"], self._stream()))
-        launches += 2 if self.k <= 12 else 4
+                                      prep["nblocks"], st))
+        launches += 1 if self.k <= 12 else 4
         return launches
 
     def _flags_tensor(self):

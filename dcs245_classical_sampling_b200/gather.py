@@ -152,26 +152,22 @@ class ConditionalBlockGPU:
         flags = torch.zeros(self.items, dtype=torch.int64, device=self.device)
         S = len(self.steps)
         final = self.tab[S & 1]  # step s reads table s % 2
-        sw = _lib.SCALE_DTYPE.itemsize // 8
         for cn, d_params, d_coefs, d_xors, d_begin in chunks:
-            mb = self.maxbits[: cn * self.nm].view(cn, self.nm)
-            mb.zero_()
-            mb[:, 0] = self.one_bits
-            self.scale[: cn * sw].zero_()
-            self.tab[0].view(self.items, self.stride)[:cn, 0] = 1  # empty environment (gpu_kernel.py:132)
+            # empty environment (gpu_kernel.py:132)
+            _lib.check(lib.dcs_begin_items(self.dcode, _lib.ptr(self.tab[0]), self.stride, _lib.ptr(self.maxbits), self.nm,
+                                           _lib.ptr(self.scale), cn, st))
             _lib.check(lib.dcs_gather_steps(self.dcode, _lib.ptr(self.tab[0]), _lib.ptr(self.tab[1]), self.stride,
                                             self.dsteps.ctypes.data, _lib.ptr(self.words), d_params, S, 0, S,
                                             _lib.ptr(self.maxbits), self.nm, _lib.ptr(self.scale), cn, st))
             _lib.check(lib.dcs_accumulate_batched(
                 self.dcode, _lib.ptr(final), self.stride, self.terminal_rank, self.term_runs.ctypes.data,
                 self.term_nruns, self.tbasis.ctypes.data, d_xors, d_coefs, d_begin, 1, self.params.shift,
-                _lib.ptr(self.scale), _lib.ptr(self.maxbits[self.nm - 1:]), self.nm,
+                _lib.ptr(self.scale), _lib.ptr(self.maxbits) + 8 * (self.nm - 1), self.nm,
                 _lib.ptr(out.view(torch.float64)), self.k, cn, st))
-            flags[:cn] |= self.scale[: cn * sw].view(cn, sw)[:, 2]
+            _lib.check(lib.dcs_collect_flags(_lib.ptr(self.scale), _lib.ptr(flags), cn, st))
         _lib.check(lib.dcs_block_tail(_lib.ptr(out), self.k, self.adj_hi.ctypes.data, self.u_open.ctypes.data, 1, st))
-        if bool(((flags & 1) != 0).any()):
+        if np.any(flags.cpu().numpy() & 1):
             raise ArithmeticError("Nonfinite prefix table")
-        torch.cuda.current_stream(self.device).synchronize()
         meta = {"seconds": time.perf_counter() - start, "part": part, "parts": parts, "slices_evaluated": count,
                 "prefix_dtype": "complex128" if self.use_fp64 else "complex64", "rmax": self.rmax,
                 "terminal_rank": self.terminal_rank, "work_per_slice": self.work, "open_vertices": self.open_full,

@@ -248,6 +248,13 @@ int dcs_slice_steps_batched(int dtype, void *table, uint64_t table_stride, const
                             const dcs_param *params, uint64_t param_stride, int nsteps, int first, int count,
                             uint64_t *maxbits, dcs_scale *scale, int nitems, void *stream);
 
+/* Initial state of `nitems` work items: entry 0 of table + i*table_stride = 1 (the empty environment), words
+ * of maxbits + i*maxbits_stride zero but for word 0 (the bits of 1.0), scale + i zero. */
+int dcs_begin_items(int dtype, void *table, uint64_t table_stride, uint64_t *maxbits, uint64_t maxbits_stride,
+                    dcs_scale *scale, int nitems, void *stream);
+/* flags[i] |= scale[i].flags (device memory). */
+int dcs_collect_flags(const dcs_scale *scale, int64_t *flags, int nitems, void *stream);
+
 /* Gather-form steps [s0, s0 + count) on two tables of nitems work items each (item i at
  * i * stride entries): step s0 reads table_a and writes table_b, the next reads table_b, and so on,
  * so the result is in table_b for odd count.  Replaces the host loop of the reference's
