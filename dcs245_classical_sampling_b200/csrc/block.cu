@@ -89,12 +89,80 @@ struct TailParams {
     int k;
 };
 
+constexpr int kTailLog = 12;  // 4096 complex128 = 64 KiB of shared memory per tile
+enum { kTailWht = 0, kTailPhaseU = 1, kTailU = 2, kTailAll = 3 };
+
+// 16-byte entries, eight of them per 128-byte row of banks: the XOR keeps the eight lanes of an access apart both
+// when they hold neighbours and when each holds a run of eight
+__device__ __forceinline__ int swz(int i) { return i ^ ((i >> 3) & 7); }
+
+// sign of the open-edge phase at index ad
+__device__ __forceinline__ bool open_phase(uint32_t ad, const TailParams& tp) {
+    uint32_t par = 0;
+    for (int q = 0; q < tp.k; ++q)
+        if ((ad >> q) & 1) par ^= ad & tp.adj_hi[q];
+    return __popc(par) & 1;
+}
+
+// NB consecutive tile bits from bit j on, one after the other, on 2^NB entries per thread
+template <int NB, bool U>
+__device__ __forceinline__ void tail_round(double2* sh, int tsize, int j, int q0, const TailParams& tp, bool phase) {
+    constexpr int N = 1 << NB;
+    for (int g = threadIdx.x; g < (tsize >> NB); g += blockDim.x) {
+        const int i0 = ((g >> j) << (j + NB)) | (g & ((1 << j) - 1));
+        double2 x[N];
+#pragma unroll
+        for (int e = 0; e < N; ++e) {
+            x[e] = sh[swz(i0 | e << j)];
+            if (U && phase && open_phase((uint32_t)(i0 | e << j), tp)) x[e] = make_double2(-x[e].x, -x[e].y);
+        }
+#pragma unroll
+        for (int b = 0; b < NB; ++b) {
+            const double* m = tp.u[q0 + b];
+#pragma unroll
+            for (int e = 0; e < N; ++e) {
+                if (e >> b & 1) continue;
+                const double2 x0 = x[e], x1 = x[e | 1 << b];
+                if constexpr (U) {
+                    x[e] = make_double2(m[0] * x0.x - m[1] * x0.y + m[2] * x1.x - m[3] * x1.y,
+                                        m[0] * x0.y + m[1] * x0.x + m[2] * x1.y + m[3] * x1.x);
+                    x[e | 1 << b] = make_double2(m[4] * x0.x - m[5] * x0.y + m[6] * x1.x - m[7] * x1.y,
+                                                 m[4] * x0.y + m[5] * x0.x + m[6] * x1.y + m[7] * x1.x);
+                } else {
+                    x[e] = make_double2(x0.x + x1.x, x0.y + x1.y);
+                    x[e | 1 << b] = make_double2(x0.x - x1.x, x0.y - x1.y);
+                }
+            }
+        }
+#pragma unroll
+        for (int e = 0; e < N; ++e) sh[swz(i0 | e << j)] = x[e];
+    }
+    __syncthreads();
+}
+
+// tile bits [lo, hi), three per round (one round trip through shared memory for three of them); `a`: the tile
+// bits below it are the physical bits, the others start at physical bit b_lo
+template <bool U>
+__device__ __forceinline__ void tail_bits(double2* sh, int tsize, int lo, int hi, int a, int b_lo, const TailParams& tp,
+                                          bool phase) {
+    for (int j = lo; j < hi;) {
+        const int q0 = j < a ? j : b_lo + (j - a);  // physical bit
+        const int nb = hi - j < 3 ? hi - j : 3;
+        if (nb == 3) tail_round<3, U>(sh, tsize, j, q0, tp, phase);
+        else if (nb == 2) tail_round<2, U>(sh, tsize, j, q0, tp, phase);
+        else tail_round<1, U>(sh, tsize, j, q0, tp, phase);
+        phase = false;
+        j += nb;
+    }
+}
+
 // Apply per-bit 2x2 transforms over the tile bits [tb_lo, tb_hi) of tiles made of
-// physical bits [0, a) (contiguous) and [b_lo, b_hi).  mode 0: Walsh-Hadamard;
-// mode 1: multiply by the open-edge phase on load, then U_open.
+// physical bits [0, a) (contiguous) and [b_lo, b_hi).  kTailWht: Walsh-Hadamard; kTailPhaseU: multiply by
+// the open-edge phase on load, then U_open; kTailU: U_open; kTailAll (one tile per block): all of it.
+template <int MODE>
 __global__ void __launch_bounds__(512)
 k_tail(double2* __restrict__ total, const __grid_constant__ TailParams tp, int a, int b_lo, int b_hi, int tb_lo,
-       int tb_hi, int mode) {
+       int tb_hi) {
     extern __shared__ double2 sh[];
     const int k = tp.k;
     const int tile_log = a + (b_hi - b_lo);
@@ -113,56 +181,30 @@ k_tail(double2* __restrict__ total, const __grid_constant__ TailParams tp, int a
         const uint64_t hi = (uint64_t)t >> a;
         return gbase | lo | (hi << b_lo);
     };
+#pragma unroll 4
     for (int t = threadIdx.x; t < tsize; t += blockDim.x) {
         const uint64_t ad = addr(t);
         double2 x = v[ad];
-        if (mode == 1) {
-            int par = 0;
-            for (int q = 0; q < k; ++q)
-                if ((ad >> q) & 1) par ^= __popc((uint32_t)ad & tp.adj_hi[q]) & 1;
-            if (par) { x.x = -x.x; x.y = -x.y; }
-        }
-        sh[t] = x;
+        if (MODE == kTailPhaseU && open_phase((uint32_t)ad, tp)) x = make_double2(-x.x, -x.y);
+        sh[swz(t)] = x;
     }
     __syncthreads();
-    for (int j = tb_lo; j < tb_hi; ++j) {
-        const int q = j < a ? j : b_lo + (j - a);  // physical bit
-        const int half = tsize >> 1;
-        const double* m = tp.u[q];
-        for (int h = threadIdx.x; h < half; h += blockDim.x) {
-            const int lo_part = h & ((1 << j) - 1);
-            const int t0 = ((h >> j) << (j + 1)) | lo_part;
-            const int t1 = t0 | (1 << j);
-            const double2 x0 = sh[t0], x1 = sh[t1];
-            double2 y0, y1;
-            if (mode == 0) {
-                y0 = make_double2(x0.x + x1.x, x0.y + x1.y);
-                y1 = make_double2(x0.x - x1.x, x0.y - x1.y);
-            } else {
-                y0 = make_double2(m[0] * x0.x - m[1] * x0.y + m[2] * x1.x - m[3] * x1.y,
-                                  m[0] * x0.y + m[1] * x0.x + m[2] * x1.y + m[3] * x1.x);
-                y1 = make_double2(m[4] * x0.x - m[5] * x0.y + m[6] * x1.x - m[7] * x1.y,
-                                  m[4] * x0.y + m[5] * x0.x + m[6] * x1.y + m[7] * x1.x);
-            }
-            sh[t0] = y0;
-            sh[t1] = y1;
-        }
-        __syncthreads();
-    }
-    for (int t = threadIdx.x; t < tsize; t += blockDim.x) v[addr(t)] = sh[t];
+    if constexpr (MODE == kTailWht || MODE == kTailAll) tail_bits<false>(sh, tsize, tb_lo, tb_hi, a, b_lo, tp, false);
+    if constexpr (MODE != kTailWht) tail_bits<true>(sh, tsize, tb_lo, tb_hi, a, b_lo, tp, MODE == kTailAll);
+#pragma unroll 4
+    for (int t = threadIdx.x; t < tsize; t += blockDim.x) v[addr(t)] = sh[swz(t)];
 }
 
-constexpr int kTailLog = 12;  // 4096 complex128 = 64 KiB of shared memory per tile
-
-int tail_pass(double2* total, const TailParams& tp, int a, int b_lo, int b_hi, int tb_lo, int tb_hi, int mode,
-              int nblocks, cudaStream_t st) {
+template <int MODE>
+int tail_pass(double2* total, const TailParams& tp, int a, int b_lo, int b_hi, int tb_lo, int tb_hi, int nblocks,
+              cudaStream_t st) {
     const int tile_log = a + (b_hi - b_lo);
     const uint64_t tiles = (uint64_t)nblocks << (tp.k - tile_log);
     if (tiles > 0x7fffffffull) {
         dcs_host::set_error("dcs_block_tail: too many tiles");
         return DCS_E_ARG;
     }
-    const int threads = tile_log >= 10 ? 512 : (1 << (tile_log > 5 ? tile_log - 1 : 5));
+    const int threads = tile_log >= kTailLog ? 512 : 1 << (tile_log > 8 ? tile_log - 3 : 5);  // eight entries each
     int dev = 0;
     if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
         dcs_host::set_error("dcs_block_tail: no current device");
@@ -170,13 +212,14 @@ int tail_pass(double2* total, const TailParams& tp, int a, int b_lo, int b_hi, i
     }
     static int attr_set[64] = {0};
     if (!attr_set[dev]) {
-        cudaError_t e = cudaFuncSetAttribute(k_tail, cudaFuncAttributeMaxDynamicSharedMemorySize,
+        cudaError_t e = cudaFuncSetAttribute(k_tail<MODE>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                              (int)(sizeof(double2) << kTailLog));
         if (e != cudaSuccess) return dcs_host::check_cuda(e, "k_tail smem attribute");
         attr_set[dev] = 1;
     }
-    k_tail<<<(unsigned)tiles, threads, sizeof(double2) << tile_log, st>>>(total, tp, a, b_lo, b_hi, tb_lo, tb_hi,
-                                                                         mode);
+    // (a swizzled index stays inside its row of eight)
+    const size_t smem = sizeof(double2) << (tile_log > 3 ? tile_log : 3);
+    k_tail<MODE><<<(unsigned)tiles, threads, smem, st>>>(total, tp, a, b_lo, b_hi, tb_lo, tb_hi);
     DCS_CHECK_LAUNCH("k_tail launch");
     return DCS_OK;
 }
@@ -290,23 +333,20 @@ extern "C" int dcs_block_tail(double* total, int k, const uint32_t* adj_hi, cons
     cudaStream_t st = (cudaStream_t)stream;
     double2* v = (double2*)total;
     int rc;
-    if (k <= kTailLog) {
-        // one tile per block: all bits at once
-        if ((rc = tail_pass(v, tp, k, k, k, 0, k, 0, nblocks, st))) return rc;
-        if ((rc = tail_pass(v, tp, k, k, k, 0, k, 1, nblocks, st))) return rc;
-        return DCS_OK;
-    }
-    // low tile: bits [0, L); high tile: 3 contiguous low bits + bits [L, k)
-    const int L = kTailLog - 3 > k - 3 ? k - 3 : kTailLog;
-    const int hb = k - L;  // high bits
-    if (hb + 3 > kTailLog) {
+    if (k <= kTailLog)  // one tile per block: everything in one pass
+        return tail_pass<kTailAll>(v, tp, k, k, k, 0, k, nblocks, st);
+    // low tile: bits [0, L); high tile: 3 contiguous low bits + bits [L, k).  The two sizes are as near as they
+    // get, so that a 2^17 block has 128 tiles in every pass: with 2^12-entry low tiles it had 32, and a
+    // shared-memory round trip per bit, and took 39 us for the four passes.
+    int L = (k + 3) / 2;
+    if (L < k + 3 - kTailLog) L = k + 3 - kTailLog;
+    if (L > kTailLog) {
         dcs_host::set_error("dcs_block_tail: k=%d too large for the two-pass tail", k);
         return DCS_E_ARG;
     }
-    if ((rc = tail_pass(v, tp, L, L, L, 0, L, 0, nblocks, st))) return rc;
-    if ((rc = tail_pass(v, tp, 3, L, k, 3, 3 + hb, 0, nblocks, st))) return rc;
-    if ((rc = tail_pass(v, tp, L, L, L, 0, L, 1, nblocks, st))) return rc;
-    // second U pass must not re-apply the phase: mode 2 == U without phase
-    if ((rc = tail_pass(v, tp, 3, L, k, 3, 3 + hb, 2, nblocks, st))) return rc;
-    return DCS_OK;
+    const int hb = k - L;  // high bits
+    if ((rc = tail_pass<kTailWht>(v, tp, L, L, L, 0, L, nblocks, st))) return rc;
+    if ((rc = tail_pass<kTailWht>(v, tp, 3, L, k, 3, 3 + hb, nblocks, st))) return rc;
+    if ((rc = tail_pass<kTailPhaseU>(v, tp, L, L, L, 0, L, nblocks, st))) return rc;
+    return tail_pass<kTailU>(v, tp, 3, L, k, 3, 3 + hb, nblocks, st);
 }
