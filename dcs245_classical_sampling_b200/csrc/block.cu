@@ -24,37 +24,41 @@ struct TermMap {
     int nruns, tr, nchecks, k;
 };
 
+// What an item adds, the same for every entry of its block.
+struct ItemTerm {
+    double cr, ci, p2;  // coefficient; power of two that its table still has
+    uint64_t xor_;
+    int on;
+};
+
 template <class S>
 __global__ void __launch_bounds__(256)
 k_accumulate(const S* __restrict__ table, uint64_t table_stride, const __grid_constant__ TermMap tm,
              const uint64_t* __restrict__ xors, const double* __restrict__ coefs, const int32_t* __restrict__ item_begin,
              double log_shift, dcs_scale* __restrict__ scale, const unsigned long long* __restrict__ maxbits_final,
-             uint64_t mstride, double2* __restrict__ total) {
+             uint64_t mstride, int is64, double2* __restrict__ total) {
     // grid.y = output block; items item_begin[b] .. item_begin[b+1]-1 belong to block b
+    constexpr int kTerms = 64;  // items whose terms sit in shared memory at a time
+    __shared__ ItemTerm terms[kTerms];
     const int blk = blockIdx.y;
     const int i0 = item_begin[blk], i1 = item_begin[blk + 1];
     double2* out = total + ((uint64_t)blk << tm.k);
     const uint64_t n = 1ull << tm.k;
-    for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
-        double2 acc = out[t];
-        for (int it = i0; it < i1; ++it) {
+    for (int c0 = i0; c0 < i1; c0 += kTerms) {
+        const int cn = i1 - c0 < kTerms ? i1 - c0 : kTerms;
+        __syncthreads();
+        // an exponential and a sine per item and CTA; per item and entry they were most of the kernel
+        if ((int)threadIdx.x < cn) {
+            const int it = c0 + threadIdx.x;
             const dcs_scale sc = scale[it];
             const unsigned long long mf = maxbits_final[(uint64_t)it * mstride];
-            if (sc.flags & 3u) continue;  // zero table (skipped slice) or nonfinite (reported)
-            if (mf == 0) continue;        // the last step produced an all-zero table
-            const uint32_t sv = (uint32_t)(t ^ xors[it]);
-            bool in = true;
-            for (int r = 0; r < tm.nchecks; ++r) in &= !(__popc(sv & tm.check[r]) & 1);
-            if (!in) continue;
-            uint32_t i = 0;
-            for (int j = 0; j < tm.tr; ++j) i |= (uint32_t)(__popc(sv & tm.linv[j]) & 1) << j;
-            const uint64_t c = deposit(i, tm.runs, tm.nruns);
-            double2 v = entry_f64(table[(uint64_t)it * table_stride + c]);
-            if (sc.table_exp) {  // exact
-                const double p2 = ldexp(1.0, -sc.table_exp);
-                v.x *= p2;
-                v.y *= p2;
-            }
+            const double m2 = is64 ? __longlong_as_double((long long)mf) : (double)__uint_as_float((uint32_t)mf);
+            ItemTerm t;
+            // a zero table (skipped slice: at some step, or after the last one) or a nonfinite one adds nothing
+            t.on = !(sc.flags & 3u) && mf != 0 && isfinite(m2);
+            // the reference checks every step's max, including the last (every other reader of the flags in
+            // this launch takes the maximum itself)
+            if (blockIdx.x == 0 && !isfinite(m2)) scale[it].flags = sc.flags | 1u;
             const double m = exp(sc.logscale - log_shift);
             double cr = coefs[2 * it] * m, ci = coefs[2 * it + 1] * m;
             if (sc.phase != 0.0) {  // step factors divided out by the plan-specialised kernels
@@ -64,22 +68,34 @@ k_accumulate(const S* __restrict__ table, uint64_t table_stride, const __grid_co
                 ci = cr * sp + ci * cp;
                 cr = r;
             }
-            const double vr = v.x, vi = v.y;
-            acc.x += vr * cr - vi * ci;
-            acc.y += vr * ci + vi * cr;
+            t.cr = cr;
+            t.ci = ci;
+            t.p2 = ldexp(1.0, -sc.table_exp);
+            t.xor_ = xors[it];
+            terms[threadIdx.x] = t;
         }
-        out[t] = acc;
+        __syncthreads();
+        for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
+            double2 acc = out[t];
+            for (int q = 0; q < cn; ++q) {
+                const ItemTerm& term = terms[q];
+                if (!term.on) continue;
+                const uint32_t sv = (uint32_t)(t ^ term.xor_);
+                bool in = true;
+                for (int r = 0; r < tm.nchecks; ++r) in &= !(__popc(sv & tm.check[r]) & 1);
+                if (!in) continue;
+                uint32_t i = 0;
+                for (int j = 0; j < tm.tr; ++j) i |= (uint32_t)(__popc(sv & tm.linv[j]) & 1) << j;
+                const uint64_t c = deposit(i, tm.runs, tm.nruns);
+                const double2 v = entry_f64(table[(uint64_t)(c0 + q) * table_stride + c]);
+                const double vr = v.x * term.p2, vi = v.y * term.p2;  // exact
+                // (roundings fixed: the draws' 53-bit distances depend on every bit of a block)
+                acc.x = __dadd_rn(acc.x, __fma_rn(vr, term.cr, -__dmul_rn(vi, term.ci)));
+                acc.y = __dadd_rn(acc.y, __fma_rn(vi, term.cr, __dmul_rn(vr, term.ci)));
+            }
+            out[t] = acc;
+        }
     }
-}
-
-// flags for nonfinite final maxima (the reference checks every step's max, including the last)
-__global__ void k_final_flags(const unsigned long long* __restrict__ maxbits_final, uint64_t mstride, int is64,
-                              dcs_scale* __restrict__ scale, int nitems) {
-    const int it = blockIdx.x * blockDim.x + threadIdx.x;
-    if (it >= nitems) return;
-    const unsigned long long b = maxbits_final[(uint64_t)it * mstride];
-    const double m2 = is64 ? __longlong_as_double((long long)b) : (double)__uint_as_float((uint32_t)b);
-    if (!isfinite(m2)) scale[it].flags |= 1u;
 }
 
 // ---------------------------------------------------------------- tail
@@ -286,11 +302,6 @@ extern "C" int dcs_accumulate_batched(int dtype, const void* table, uint64_t tab
     int rc = build_termmap(tm, tr, terminal_runs, nruns, tbasis, k);
     if (rc) return rc;
     cudaStream_t st = (cudaStream_t)stream;
-    if (nitems > 0) {
-        k_final_flags<<<(nitems + 127) / 128, 128, 0, st>>>((const unsigned long long*)maxbits_final, mstride,
-                                                            dtype == DCS_C128, scale, nitems);
-        DCS_CHECK_LAUNCH("k_final_flags launch");
-    }
     const uint64_t n = 1ull << k;
     uint64_t bx = (n + 255) / 256;
     const uint64_t cap = (uint64_t)dcs_host::sm_count() * 8;
@@ -299,15 +310,15 @@ extern "C" int dcs_accumulate_batched(int dtype, const void* table, uint64_t tab
     if (dtype == DCS_C64)
         k_accumulate<float2><<<grid, 256, 0, st>>>((const float2*)table, table_stride, tm, xors, coefs, item_begin,
                                                    log_shift, scale, (const unsigned long long*)maxbits_final, mstride,
-                                                   (double2*)total);
+                                                   0, (double2*)total);
     else if (dtype == DCS_C128)
         k_accumulate<double2><<<grid, 256, 0, st>>>((const double2*)table, table_stride, tm, xors, coefs, item_begin,
                                                     log_shift, scale, (const unsigned long long*)maxbits_final,
-                                                    mstride, (double2*)total);
+                                                    mstride, 1, (double2*)total);
     else if (dtype == DCS_H16)
         k_accumulate<ushort2><<<grid, 256, 0, st>>>((const ushort2*)table, table_stride, tm, xors, coefs, item_begin,
                                                     log_shift, scale, (const unsigned long long*)maxbits_final,
-                                                    mstride, (double2*)total);
+                                                    mstride, 0, (double2*)total);
     else {
         dcs_host::set_error("dcs_accumulate: unknown dtype %d", dtype);
         return DCS_E_ARG;

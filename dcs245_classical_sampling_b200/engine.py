@@ -752,7 +752,7 @@ class InplaceConditionalBlockGPU:
                 d_xors + 8 * c0, d_coefs + 16 * c0,
                 d_begin + 4 * boff, nb, self.params.shift, _lib.ptr(self.scale),
                 _lib.ptr(self.maxbits) + 8 * (nm - 1), nm, _lib.ptr(out) + (b0 << (self.k + 4)), self.k, cn, st))
-            launches += 3
+            launches += 2
             if flags is not None:
                 if flags.dtype != torch.int64 or not flags.is_cuda or not flags.is_contiguous() or flags.numel() < cn:
                     raise ValueError("flags must be a contiguous int64 device tensor of engine.items elements")
