@@ -91,6 +91,14 @@ template <class R> __device__ __forceinline__ R bits_to_m2(unsigned long long b)
 template <> __device__ __forceinline__ float bits_to_m2<float>(unsigned long long b) { return __uint_as_float((uint32_t)b); }
 template <> __device__ __forceinline__ double bits_to_m2<double>(unsigned long long b) { return __longlong_as_double((long long)b); }
 
+// Launches that depend on the one before them in their stream (launch_after): the kernel may start while that one
+// still runs, does what needs none of its results, and waits here until it has finished and its writes are
+// visible.  Every kernel launched so waits before it ends, so a finished kernel means that all before it in
+// the chain have finished, too.
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;\n" ::: "memory"); }
+// Lets the next such launch begin as soon as every CTA of this one has started (or ended).
+__device__ __forceinline__ void let_next_start() { asm volatile("griddepcontrol.launch_dependents;\n" ::: "memory"); }
+
 // exponent e of frexp(sqrt(m2)) (0 for m2 == 0 or nonfinite), computed as the reference's
 // host loop does: maximum = sqrt(m2) in FP64, e = frexp(maximum)[1]
 __device__ __forceinline__ int scale_exponent(double m2) {
@@ -128,6 +136,22 @@ namespace dcs_host {
 void set_error(const char* fmt, ...);
 int check_cuda(cudaError_t e, const char* what);
 int sm_count();
+
+// A launch whose kernel calls after_previous(): it may start before the previous launch in the stream ends.
+template <class... K, class... A>
+cudaError_t launch_after(void (*kernel)(K...), dim3 grid, dim3 block, size_t smem, cudaStream_t stream, A... args) {
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = grid;
+    cfg.blockDim = block;
+    cfg.dynamicSmemBytes = smem;
+    cfg.stream = stream;
+    cudaLaunchAttribute attr = {};
+    attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr.val.programmaticStreamSerializationAllowed = 1;
+    cfg.attrs = &attr;
+    cfg.numAttrs = 1;
+    return cudaLaunchKernelEx(&cfg, kernel, static_cast<K>(args)...);
+}
 }  // namespace dcs_host
 
 #define DCS_CHECK_LAUNCH(what)                                                      \

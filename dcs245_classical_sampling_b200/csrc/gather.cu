@@ -20,9 +20,10 @@ constexpr int kThreads = 256;
 constexpr int kMaxTableWords = 8 * 256;  // up to 64-bit outputs
 constexpr int kMaxCombos = 64;
 
+// (Ein is what the launch before writes, which may still run when this one starts: no read-only loads of it)
 template <class S>
 __global__ void __launch_bounds__(kThreads)
-k_gather(const S* __restrict__ Ein, S* __restrict__ Eout, uint64_t stride, const __grid_constant__ dcs_gather_step st,
+k_gather(const S* Ein, S* Eout, uint64_t stride, const __grid_constant__ dcs_gather_step st,
          const uint64_t* __restrict__ words, int s, const dcs_param* __restrict__ params, uint64_t param_stride,
          unsigned long long* __restrict__ maxbits, uint64_t maxbits_stride, dcs_scale* __restrict__ scale) {
     using R = typename Store<S>::R;
@@ -31,6 +32,11 @@ k_gather(const S* __restrict__ Ein, S* __restrict__ Eout, uint64_t stride, const
     const int item = blockIdx.y;
     const S* E = Ein + (uint64_t)item * stride;
     S* out = Eout + (uint64_t)item * stride;
+    let_next_start();
+    // the step's tables are the plan's: nothing in the stream writes them
+    for (int i = threadIdx.x; i < st.nbytes * 256; i += kThreads) T[i] = words[st.table_off + i];
+    for (int i = threadIdx.x; i < st.ncombos; i += kThreads) C[i] = words[st.combo_off + i];
+    after_previous();
     const dcs_param p = params[(uint64_t)item * param_stride + s];
     unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
     const double m2prev = (double)bits_to_m2<R>(mb[s]);
@@ -43,8 +49,6 @@ k_gather(const S* __restrict__ Ein, S* __restrict__ Eout, uint64_t stride, const
         if (!isfinite(m2prev)) sp->flags |= 1u;
         else if (m2prev == 0.0) sp->flags |= 2u;
     }
-    for (int i = threadIdx.x; i < st.nbytes * 256; i += kThreads) T[i] = words[st.table_off + i];
-    for (int i = threadIdx.x; i < st.ncombos; i += kThreads) C[i] = words[st.combo_off + i];
     __syncthreads();
     const uint64_t mask = st.r_in >= 64 ? ~0ull : ((1ull << st.r_in) - 1ull);
     const uint64_t n_out = 1ull << st.r_out;
@@ -96,10 +100,12 @@ int run_steps(void* a, void* b, uint64_t stride, const dcs_gather_step* steps, c
         const uint64_t want = (n_out + kThreads - 1) / kThreads;
         const unsigned grid = (unsigned)(want < (uint64_t)sms * 8 ? want : (uint64_t)sms * 8);
         const int k = s - s0;
-        k_gather<S><<<dim3(grid, n_items), kThreads, 0, stream>>>(bufs[k & 1], bufs[(k & 1) ^ 1], stride, st, words, s,
-                                                                 params, param_stride, maxbits, maxbits_stride,
-                                                                 scale);
-        DCS_CHECK_LAUNCH("k_gather");
+        const int rc = dcs_host::check_cuda(
+            dcs_host::launch_after(k_gather<S>, dim3(grid, n_items), dim3(kThreads), 0, stream, bufs[k & 1],
+                                   bufs[(k & 1) ^ 1], stride, st, words, s, params, param_stride, maxbits, maxbits_stride,
+                                   scale),
+            "k_gather");
+        if (rc) return rc;
     }
     return DCS_OK;
 }

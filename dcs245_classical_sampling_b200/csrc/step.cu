@@ -32,25 +32,7 @@ k_step(M* __restrict__ table, uint64_t table_stride, const __grid_constant__ dcs
     constexpr int NT = 256;  // threads per block (the launch uses exactly this)
     constexpr int LU = ORB == 8 ? 3 : (ORB == 4 ? 2 : 1);
     static_assert((1 << LU) == ORB, "ORB is a power of two");
-    const int item = blockIdx.y;
-    M* E = table + (uint64_t)item * table_stride;
-    const dcs_param p = params[(uint64_t)item * param_stride + s];
-    unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
-    const double m2prev = (double)bits_to_m2<R>(mb[s]);
-    const int e = scale_exponent(m2prev);
-    const R sc = (R)ldexp(1.0, -e);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
-        dcs_scale* sp = scale + item;
-        sp->logscale += (double)e * 0.69314718055994530942;  // ln 2, as the reference's e*log(2.)
-        sp->exponent_sum += e;
-        if (!isfinite(m2prev)) sp->flags |= 1u;
-        else if (m2prev == 0.0) sp->flags |= 2u;
-    }
-    // the power-of-two scale is folded into the weights: (f * 2^-e) * v == (f * v) * 2^-e exactly
-    // (outside the subnormal range), and the scaled weights drop two multiplies per output
-    const S f0 = cscale(Store<S>::make((R)p.f0r, (R)p.f0i), sc);
-    const S f1 = cscale(Store<S>::make((R)p.f1r, (R)p.f1i), sc);
-    const int y = p.y;
+    let_next_start();
     const uint64_t norbits = 1ull << st.m;
     const bool ident = st.nruns == 0 || (st.nruns == 1 && st.runs[0] == ((uint32_t)st.m << 16));
     const uint64_t beta = st.beta, K = st.K, Ka = st.Ka, pbit = st.pivot_bit;
@@ -74,8 +56,29 @@ k_step(M* __restrict__ table, uint64_t table_stride, const __grid_constant__ dcs
             if (u >> b & 1) d |= du[b];
         pu |= par(d) << u;
     }
-    const int st_ov = p.ov ^ par(dt);           // sign of c = parity(base) ^ bit u of pu ^ st_ov
+    const int pdt = par(dt);
     const int pK = par(K), pKa = par(Ka);       // sign(c ^ K) = sign(c) ^ pK, likewise for Ka
+    after_previous();
+    const int item = blockIdx.y;
+    M* E = table + (uint64_t)item * table_stride;
+    const dcs_param p = params[(uint64_t)item * param_stride + s];
+    unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
+    const double m2prev = (double)bits_to_m2<R>(mb[s]);
+    const int e = scale_exponent(m2prev);
+    const R sc = (R)ldexp(1.0, -e);
+    if (blockIdx.x == 0 && threadIdx.x == 0) {
+        dcs_scale* sp = scale + item;
+        sp->logscale += (double)e * 0.69314718055994530942;  // ln 2, as the reference's e*log(2.)
+        sp->exponent_sum += e;
+        if (!isfinite(m2prev)) sp->flags |= 1u;
+        else if (m2prev == 0.0) sp->flags |= 2u;
+    }
+    // the power-of-two scale is folded into the weights: (f * 2^-e) * v == (f * v) * 2^-e exactly
+    // (outside the subnormal range), and the scaled weights drop two multiplies per output
+    const S f0 = cscale(Store<S>::make((R)p.f0r, (R)p.f0i), sc);
+    const S f1 = cscale(Store<S>::make((R)p.f1r, (R)p.f1i), sc);
+    const int y = p.y;
+    const int st_ov = p.ov ^ pdt;               // sign of c = parity(base) ^ bit u of pu ^ st_ov
     Q lm = 0;
     constexpr uint64_t chunk = (uint64_t)NT * ORB;
     for (uint64_t base = (uint64_t)blockIdx.x * chunk; base < norbits; base += (uint64_t)gridDim.x * chunk) {
@@ -240,10 +243,9 @@ int launch_kind(M* table, uint64_t table_stride, const dcs_step& st, int s, cons
     if (blocks > cap) blocks = cap;
     if (blocks < 1) blocks = 1;
     dim3 grid((unsigned)blocks, (unsigned)nitems);
-    k_step<S, KIND, ORB, M><<<grid, kThreads, 0, stream>>>(table, table_stride, st, s, params, param_stride,
-                                                           maxbits, mstride, scale);
-    DCS_CHECK_LAUNCH("k_step launch");
-    return DCS_OK;
+    return dcs_host::check_cuda(dcs_host::launch_after(k_step<S, KIND, ORB, M>, grid, dim3(kThreads), 0, stream, table,
+                                                       table_stride, st, s, params, param_stride, maxbits, mstride, scale),
+                                "k_step launch");
 }
 
 template <class S, class M = S>

@@ -211,6 +211,7 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     S* E = table + (uint64_t)item * table_stride;
     unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
 
+    let_next_start();
     for (int i = threadIdx.x; i < A.count * kTab; i += NT) {
         const TileStep& st = A.st[i / kTab];
         const uint32_t j = i % kTab;
@@ -225,6 +226,7 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
             if ((h >> i) & 1) a ^= A.basis[i];
         hi_tab[h] = a;
     }
+    after_previous();  // the tables above are the plan's
     const int e = scale_exponent((double)bits_to_m2<R>(mb[A.first]));
     if (blockIdx.x == 0 && threadIdx.x < 32) {
         const int lo = kStepMax<S> ? A.prev_first + 1 : A.first;
@@ -410,10 +412,10 @@ int launch_group(S* table, uint64_t table_stride, const TileArgs& A, const dcs_p
             grid = (grid + each - 1) / each;
         }
     }
-    k_tiles<S, NT><<<dim3((unsigned)grid, (unsigned)nitems), NT, smem, st>>>(table, table_stride, A, params, param_stride,
-                                                                            maxbits, maxbits_stride, scale);
-    DCS_CHECK_LAUNCH("k_tiles launch");
-    return DCS_OK;
+    return dcs_host::check_cuda(dcs_host::launch_after(k_tiles<S, NT>, dim3((unsigned)grid, (unsigned)nitems), dim3(NT), smem,
+                                                       st, table, table_stride, A, params, param_stride, maxbits,
+                                                       maxbits_stride, scale),
+                                "k_tiles launch");
 }
 
 template <class S>
