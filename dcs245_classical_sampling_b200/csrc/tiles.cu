@@ -34,7 +34,8 @@ using namespace dcs;
 namespace {
 
 constexpr int kMaxSteps = 24;
-constexpr int kMaxDim = 12;  // 32 KiB (complex64) or 64 KiB per tile
+constexpr int kMaxDim = 12;   // 32 KiB (complex64) or 64 KiB per tile
+constexpr int kHalfDim = 13;  // binary16 tables: 32 KiB
 
 struct TileStep {
     uint64_t beta, cskip;
@@ -78,7 +79,7 @@ template <class S> struct Weights {
 };
 
 // whether every step's maximum is taken (else the group's)
-template <class S> constexpr bool kStepMax = sizeof(S) == 8;
+template <class M> constexpr bool kStepMax = sizeof(M) <= 8;
 
 constexpr uint32_t kSign = 0x80000000u;
 // +-1 by bit 31 of x
@@ -93,8 +94,8 @@ template <class S> __device__ __forceinline__ S flip(S a, uint32_t m) { return c
 
 // Words per step of the spread tables: 16 for bits 0-3 of the thread, then its other bits, then the orbit
 // slots of a thread.
-template <int NT> struct Tab {
-    static constexpr int kHi = 16, kOrb = kHi + NT / 16, kWords = kOrb + (1 << kMaxDim) / NT;
+template <int NT, int DIM = kMaxDim> struct Tab {
+    static constexpr int kHi = 16, kOrb = kHi + NT / 16, kWords = kOrb + (1 << DIM) / NT;
 };
 
 // One vertex step over the active orbit representatives of the tile.  Representatives are the tile
@@ -104,12 +105,13 @@ template <int NT> struct Tab {
 // gives an orbit's offset and sign.  (Spreading and counting bits per orbit took 31 instructions per entry
 // and step instead of 20.)  Signs enter as factors +-1 of a fused multiply-add, which round as the
 // addition of the negated value does.
-template <class S, int KIND, int NT>
-__device__ __forceinline__ typename Store<S>::R run_step(unsigned char* __restrict__ sh, int T, const TileStep& st,
+template <class S, int KIND, int NT, class M = S>
+__device__ __forceinline__ typename Mem<S, M>::Q run_step(unsigned char* __restrict__ sh, int T, const TileStep& st,
                                                          const uint32_t* __restrict__ tab, const Weights<S>& w,
                                                          uint32_t cs, int y) {
     using R = typename Store<S>::R;
-    constexpr int SH = sizeof(S) == 8 ? 3 : 4;
+    using IO = Mem<S, M>;
+    constexpr int SH = sizeof(M) == 4 ? 2 : (sizeof(M) == 8 ? 3 : 4);
     const int nrep = T >> st.nins;
     if ((int)threadIdx.x >= nrep) return 0;
     const uint32_t tp = tab[threadIdx.x & 15] ^ tab[Tab<NT>::kHi + (threadIdx.x >> 4)] ^ (cs << 31);
@@ -122,11 +124,11 @@ __device__ __forceinline__ typename Store<S>::R run_step(unsigned char* __restri
     const S fy = y ? f1 : f0;  // a fixed step: the weight that its value selects
     const R gy = y ? gK : (R)1;
     const uint32_t my = y ? kSign : 0u;
-    auto ld = [&](uint32_t o) { return *reinterpret_cast<const S*>(sh + o); };
-    R lm = 0;
+    auto ld = [&](uint32_t o) { return IO::ld(*reinterpret_cast<const M*>(sh + o)); };
+    typename IO::Q lm = 0;
     auto stv = [&](uint32_t o, S v) {
-        *reinterpret_cast<S*>(sh + o) = v;
-        if constexpr (kStepMax<S>) lm = fmax(lm, v.x * v.x + v.y * v.y);
+        const typename IO::Q q = IO::st(reinterpret_cast<M*>(sh + o), 0, v);
+        if constexpr (kStepMax<M>) lm = fmax(lm, q);
     };
 #pragma unroll 4
     for (int u = 0; u < niter; ++u) {
@@ -191,6 +193,27 @@ __device__ __forceinline__ int add_exponents(const unsigned long long* mb, int l
     return sum;
 }
 
+// The spread tables of every step, and the table addresses of the tile's high coordinates.
+template <int NT, int DIM, int SH>
+__device__ __forceinline__ void fill_tables(const TileArgs& A, uint32_t (*tab)[Tab<NT, DIM>::kWords], uint64_t* hi_tab) {
+    constexpr int kTab = Tab<NT, DIM>::kWords, kHi = Tab<NT, DIM>::kHi, kOrb = Tab<NT, DIM>::kOrb;
+    const uint32_t in_tile = (1u << A.tile_dim) - 1u;
+    for (int i = threadIdx.x; i < A.count * kTab; i += NT) {
+        const TileStep& st = A.st[i / kTab];
+        const uint32_t j = i % kTab;
+        uint32_t o = j < kHi ? j : j < kOrb ? (j - kHi) << 4 : (j - kOrb) * NT;
+        for (int q = 0; q < st.nins; ++q) o = insert0(o, st.ins[q]);
+        o &= in_tile;  // bits past the tile belong to idle threads and orbit slots
+        tab[i / kTab][j] = (o << SH) | (uint32_t)(__popc(o & st.tbeta) << 31);
+    }
+    for (int h = threadIdx.x; h < (1 << (A.tile_dim - A.low_bits)); h += NT) {
+        uint64_t a = 0;
+        for (int i = 0; i < A.tile_dim - A.low_bits; ++i)
+            if ((h >> i) & 1) a ^= A.basis[i];
+        hi_tab[h] = a;
+    }
+}
+
 template <class S, int NT>
 __global__ void __launch_bounds__(NT, (sizeof(S) == 8 ? 1280 : 768) / NT)
 k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ TileArgs A,
@@ -199,8 +222,7 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     using R = typename Store<S>::R;
     constexpr int SH = sizeof(S) == 8 ? 3 : 4;
     extern __shared__ __align__(16) unsigned char smem[];
-    constexpr int kTab = Tab<NT>::kWords, kHi = Tab<NT>::kHi, kOrb = Tab<NT>::kOrb;
-    __shared__ uint32_t tab[kMaxSteps][kTab];
+    __shared__ uint32_t tab[kMaxSteps][Tab<NT>::kWords];
     __shared__ Weights<S> fw[kMaxSteps];
     __shared__ int ovy[kMaxSteps];
     __shared__ uint32_t smax[kMaxSteps];  // per step: the CTA's maximum |x|^2 (max_key)
@@ -212,20 +234,7 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
 
     let_next_start();
-    for (int i = threadIdx.x; i < A.count * kTab; i += NT) {
-        const TileStep& st = A.st[i / kTab];
-        const uint32_t j = i % kTab;
-        uint32_t o = j < kHi ? j : j < kOrb ? (j - kHi) << 4 : (j - kOrb) * NT;
-        for (int q = 0; q < st.nins; ++q) o = insert0(o, st.ins[q]);
-        o &= (uint32_t)(T - 1);  // bits past the tile belong to idle threads and orbit slots
-        tab[i / kTab][j] = (o << SH) | (uint32_t)(__popc(o & st.tbeta) << 31);
-    }
-    for (int h = threadIdx.x; h < (1 << (A.tile_dim - low)); h += NT) {
-        uint64_t a = 0;
-        for (int i = 0; i < A.tile_dim - low; ++i)
-            if ((h >> i) & 1) a ^= A.basis[i];
-        hi_tab[h] = a;
-    }
+    fill_tables<NT, kMaxDim, SH>(A, tab, hi_tab);
     after_previous();  // the tables above are the plan's
     const int e = scale_exponent((double)bits_to_m2<R>(mb[A.first]));
     if (blockIdx.x == 0 && threadIdx.x < 32) {
@@ -344,7 +353,86 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     if (threadIdx.x == 0) sp->table_exp = rest;
 }
 
-bool fill_args(TileArgs& A, const dcs_group* groups, int gi, int ngroups, const dcs_step* steps, int nsteps,
+// A group whose table is one tile, on binary16 tables with FP64 arithmetic (the half-storage tier): one CTA
+// per item.  Every step rounds what it stores, scaled by the exponent of the maximum before it, so the
+// scale is taken step by step here, too; the CTA holds the whole table, so its maximum is at hand.
+// One launch for up to 24 steps instead of a launch each: see run_half_groups.
+template <int NT>
+__global__ void __launch_bounds__(NT)
+k_tile_half(ushort2* __restrict__ table, uint64_t table_stride, const __grid_constant__ TileArgs A,
+            const dcs_param* __restrict__ params, uint64_t param_stride, unsigned long long* __restrict__ maxbits,
+            uint64_t maxbits_stride, dcs_scale* __restrict__ scale) {
+    extern __shared__ __align__(16) unsigned char smem[];
+    __shared__ uint32_t tab[kMaxSteps][Tab<NT, kHalfDim>::kWords];
+    __shared__ dcs_param prm[kMaxSteps];
+    __shared__ uint32_t smax[kMaxSteps];
+    const int item = blockIdx.y;
+    const int T = 1 << A.tile_dim;
+    const int low = A.low_bits;
+    uint64_t* hi_tab = reinterpret_cast<uint64_t*>(smem + ((size_t)T << 2));
+    ushort2* E = table + (uint64_t)item * table_stride;
+    unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
+    let_next_start();
+    fill_tables<NT, kHalfDim, 2>(A, tab, hi_tab);
+    after_previous();
+    if (threadIdx.x < A.count) {
+        prm[threadIdx.x] = params[(uint64_t)item * param_stride + A.first + threadIdx.x];
+        smax[threadIdx.x] = 0;
+    }
+    __syncthreads();
+    const uint64_t lowmask = (1ull << low) - 1;
+    const uint64_t base = deposit(0, A.coset_runs, A.ncoset_runs);
+    ushort2* sh = reinterpret_cast<ushort2*>(smem);
+    for (int t = threadIdx.x; t < T; t += NT) {
+        const uint64_t a = base ^ hi_tab[t >> low] ^ ((uint64_t)t & lowmask);
+        if (!(a & A.in_inactive)) sh[t] = E[a];
+    }
+    __syncthreads();
+    double m2 = __longlong_as_double((long long)mb[A.first]);
+    dcs_scale sc = scale[item];
+    for (int s = 0; s < A.count; ++s) {
+        const TileStep& st = A.st[s];
+        const dcs_param p = prm[s];
+        const int e = scale_exponent(m2);
+        sc.logscale += (double)e * 0.69314718055994530942;  // ln 2, as the reference's e*log(2.)
+        sc.exponent_sum += e;
+        if (!isfinite(m2)) sc.flags |= 1u;
+        else if (m2 == 0.0) sc.flags |= 2u;
+        const double f = ldexp(1.0, -e);
+        Weights<double2> w;
+        w.f0 = cscale(make_double2(p.f0r, p.f0i), f);
+        w.f1 = cscale(make_double2(p.f1r, p.f1i), f);
+        w.fp = zadd(w.f0, w.f1);
+        w.fm = zadd(w.f0, c2(-w.f1.x, -w.f1.y));
+        const uint32_t cs = (uint32_t)__popcll(base & st.beta) ^ (uint32_t)(p.ov & 1);
+        float lm = 0.f;
+        switch (st.kind) {
+#define DCS_CASE(K) \
+    case K: lm = run_step<double2, K, NT, ushort2>(smem, T, st, tab[s], w, cs, p.y & 1); break;
+            DCS_CASE(DCS_KIND_GROW)
+            DCS_CASE(DCS_KIND_MIX)
+            DCS_CASE(DCS_KIND_DIAG)
+            DCS_CASE(DCS_KIND_REPLACE)
+            DCS_CASE(DCS_KIND_FIXED)
+            DCS_CASE(DCS_KIND_FIXED_SHRINK)
+            DCS_CASE(DCS_KIND_SHRINK4)
+            DCS_CASE(DCS_KIND_SHRINK2)
+#undef DCS_CASE
+        }
+        const uint32_t key = __reduce_max_sync(0xffffffffu, __float_as_uint(lm));
+        if ((threadIdx.x & 31) == 0 && key) atomicMax(&smax[s], key);
+        __syncthreads();
+        m2 = (double)__uint_as_float(smax[s]);
+        if (threadIdx.x == 0) mb[A.first + s + 1] = max_bits(m2);
+    }
+    for (int t = threadIdx.x; t < T; t += NT) {
+        const uint64_t a = base ^ hi_tab[t >> low] ^ ((uint64_t)t & lowmask);
+        if (!(a & A.out_inactive)) E[a] = sh[t];
+    }
+    if (threadIdx.x == 0) scale[item] = sc;
+}
+
+bool fill_args(TileArgs& A, int max_dim, const dcs_group* groups, int gi, int ngroups, const dcs_step* steps, int nsteps,
                const dcs_tile_step* tile_steps) {
     const dcs_group& g = groups[gi];
     // the groups follow one another from the first step to the last
@@ -352,7 +440,7 @@ bool fill_args(TileArgs& A, const dcs_group* groups, int gi, int ngroups, const 
         (gi == ngroups - 1 && g.first + g.count != nsteps))
         return false;
     if (g.count < 1 || g.count > kMaxSteps || g.first < 0 || g.first + g.count > nsteps || g.tile_dim < 0 ||
-        g.tile_dim > kMaxDim || g.low_bits < 0 || g.low_bits > g.tile_dim || g.ncoset_runs < 0 ||
+        g.tile_dim > max_dim || g.low_bits < 0 || g.low_bits > g.tile_dim || g.ncoset_runs < 0 ||
         g.ncoset_runs > DCS_MAX_RUNS || g.coset_m < 0 || g.coset_m > DCS_MAX_SLOTS || g.tile_dim - g.low_bits > 16)
         return false;
     memset(&A, 0, sizeof(A));
@@ -430,7 +518,7 @@ int run_groups(S* table, uint64_t table_stride, const dcs_step* steps, int nstep
     }
     TileArgs A;
     for (int gi = 0; gi < ngroups; ++gi) {
-        if (!fill_args(A, groups, gi, ngroups, steps, nsteps, tile_steps)) {
+        if (!fill_args(A, kMaxDim, groups, gi, ngroups, steps, nsteps, tile_steps)) {
             dcs_host::set_error("dcs_tile_groups: malformed group %d", gi);
             return DCS_E_ARG;
         }
@@ -446,6 +534,48 @@ int run_groups(S* table, uint64_t table_stride, const dcs_step* steps, int nstep
     return DCS_OK;
 }
 
+// Binary16 tables: groups whose table is one tile in one launch, the others a launch per step.  A step's
+// launch is 5 us here, a step of a 2^12-entry tile in shared memory about 1: a 20-qubit block (60 steps, one
+// tile throughout) takes a quarter of the time, and a 48-qubit one starts its 208 steps with one launch for 24.
+int run_half_groups(ushort2* table, uint64_t table_stride, const dcs_step* steps, int nsteps, const dcs_group* groups,
+                    int ngroups, const dcs_tile_step* tile_steps, const dcs_param* params, uint64_t param_stride,
+                    uint64_t* maxbits, dcs_scale* scale, int nitems, cudaStream_t st) {
+    constexpr int NT = 512;
+    const uint64_t mstride = (uint64_t)nsteps + 1;
+    int dev = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= 64) {
+        dcs_host::set_error("dcs_tile_groups: no current device");
+        return DCS_E_CUDA;
+    }
+    static bool smem_set[64] = {false};
+    if (!smem_set[dev]) {
+        const cudaError_t e = cudaFuncSetAttribute(k_tile_half<NT>, cudaFuncAttributeMaxDynamicSharedMemorySize, 128 * 1024);
+        if (e != cudaSuccess) return dcs_host::check_cuda(e, "k_tile_half smem attribute");
+        smem_set[dev] = true;
+    }
+    TileArgs A;
+    for (int gi = 0; gi < ngroups; ++gi) {
+        const dcs_group& g = groups[gi];
+        int rc;
+        if (g.coset_m != 0 || g.tile_dim > kHalfDim) {
+            rc = dcs_slice_steps_batched(DCS_H16, table, table_stride, steps, params, param_stride, nsteps, g.first, g.count,
+                                         maxbits, scale, nitems, st);
+        } else {
+            if (!fill_args(A, kHalfDim, groups, gi, ngroups, steps, nsteps, tile_steps)) {
+                dcs_host::set_error("dcs_tile_groups: malformed group %d", gi);
+                return DCS_E_ARG;
+            }
+            const size_t smem = sizeof(ushort2) * ((size_t)1 << A.tile_dim) + sizeof(uint64_t) * ((size_t)1 << (A.tile_dim - A.low_bits));
+            rc = dcs_host::check_cuda(
+                dcs_host::launch_after(k_tile_half<NT>, dim3(1, (unsigned)nitems), dim3(NT), smem, st, table, table_stride, A,
+                                       params, param_stride, (unsigned long long*)maxbits, mstride, scale),
+                "k_tile_half launch");
+        }
+        if (rc) return rc;
+    }
+    return DCS_OK;
+}
+
 }  // namespace
 
 extern "C" int dcs_tile_groups(int dtype, void* table, uint64_t table_stride, const dcs_step* steps, int nsteps,
@@ -453,10 +583,14 @@ extern "C" int dcs_tile_groups(int dtype, void* table, uint64_t table_stride, co
                                const dcs_param* params, uint64_t param_stride, uint64_t* maxbits,
                                uint64_t maxbits_stride, dcs_scale* scale, int nitems, void* stream) {
     if (!table || !steps || !groups || !tile_steps || !params || !maxbits || !scale || ngroups < 0 || nitems < 1 ||
-        nitems > 65535 || maxbits_stride < (uint64_t)nsteps + 1 || (dtype != DCS_C64 && dtype != DCS_C128)) {
+        nitems > 65535 || maxbits_stride < (uint64_t)nsteps + 1 || (dtype != DCS_C64 && dtype != DCS_C128 && dtype != DCS_H16) ||
+        (dtype == DCS_H16 && maxbits_stride != (uint64_t)nsteps + 1)) {
         dcs_host::set_error("dcs_tile_groups: invalid arguments");
         return DCS_E_ARG;
     }
+    if (dtype == DCS_H16)
+        return run_half_groups((ushort2*)table, table_stride, steps, nsteps, groups, ngroups, tile_steps, params,
+                               param_stride, maxbits, scale, nitems, (cudaStream_t)stream);
     if (dtype == DCS_C64)
         return run_groups((float2*)table, table_stride, steps, nsteps, groups, ngroups, tile_steps, params, param_stride,
                           (unsigned long long*)maxbits, maxbits_stride, scale, nitems, (cudaStream_t)stream);

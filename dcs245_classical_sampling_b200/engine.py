@@ -15,8 +15,8 @@ Execution modes (``alloc(..., mode=...)``):
 * ``"device"`` — the renormalisation stays on the device; all steps of all slices are
   enqueued without host synchronisation, several slices (work items) per launch when the
   HBM budget allows (default).  complex64 and complex128 tables take up to 24 steps per launch,
-  tile by tile in shared memory (csrc/tiles.cu); binary16 tables, and step weights outside
-  ``TILE_WEIGHT_RANGE``, one step per launch;
+  tile by tile in shared memory (csrc/tiles.cu); step weights outside ``TILE_WEIGHT_RANGE``, and
+  binary16 tables of more than one tile, one step per launch;
 * ``"fused"``  — like ``device`` but several vertex steps per pass over the table
   (coset-tiled fused kernels; complex128 tables run the plan-specialised register-run kernels
   compiled in FP64, which is how the complex128 audit recontraction runs at full size).
@@ -53,6 +53,9 @@ TILE_STEPS = 24  # steps of a tile group: the most that one launch takes
 # step (the selected one of a fixed step) in [2^-3, 2^2].  A step then grows the largest entry by 2^4
 # at most, 24 of them by 2^96, inside the FP32 range.
 TILE_WEIGHT_RANGE = (0.125, 4.0)
+
+
+HALF_TILE_DIM = 13  # log2 of the largest binary16 table that one tile holds
 
 
 def tile_dim(maxslots):
@@ -445,8 +448,11 @@ class InplaceConditionalBlockGPU:
             self.fplan = self._build_fplan()
             self.items = 1
         # device mode: groups of steps per launch over shared-memory tiles (binary16 tables round after
-        # every step with that step's scale, so they keep one launch per step)
-        self.tplan = self._build_tplan() if mode == "device" and not half else None
+        # every step with that step's scale, so only tables of one tile take several)
+        self.tplan = self._build_tplan() if mode == "device" else None
+        # library launches of those groups (binary16 groups of more than one tile: one per step)
+        self.tile_launches = 0 if self.tplan is None else sum(
+            int(g["count"]) if half and g["coset_m"] else 1 for g in self.tplan.groups)
         self.entry_bytes = entry
         self.table_dtype = torch.float16 if half else tdtype
         self.items_cap = self.items
@@ -536,7 +542,10 @@ class InplaceConditionalBlockGPU:
 
     def _build_tplan(self, dim=None, low=3):
         """The tile groups of device mode (csrc/tiles.cu): tiles of at most 2^dim entries."""
-        from .fused import build_fused_plan
+        from .fused import build_fused_plan, one_tile_spans
+        if self.half:
+            dim = HALF_TILE_DIM if dim is None else dim
+            return build_fused_plan(self.plan, max_dim=dim, low=low, spans=one_tile_spans(self.plan.steps, dim, TILE_STEPS))
         if dim is None:
             dim = tile_dim(self.plan.maxslots)
         return build_fused_plan(self.plan, max_dim=dim, low=low, max_steps=TILE_STEPS)
@@ -671,7 +680,8 @@ class InplaceConditionalBlockGPU:
         (generated kernels, tile groups); else its batch runs the library kernels / single steps."""
         if self.mode == "fused":
             return self.unit_weights_ok(params)
-        return self.tile_weights_ok(params) if self.tplan is not None else True
+        # (binary16 tables renormalise after every step in both forms)
+        return self.tile_weights_ok(params) if self.tplan is not None and not self.half else True
 
     def tile_weights_ok(self, params):
         """Whether step weights (dcs_param arrays, the plan's steps on the last axis) stay inside
@@ -745,7 +755,7 @@ class InplaceConditionalBlockGPU:
             ok = prep["unit_ok"][ci]
             self._run_steps(d_params + c0 * self.nsteps * entry, cn, ok, st)
             launches += (len(self.fplan.groups) if self.mode == "fused" else
-                         len(self.tplan.groups) if self.tplan is not None and ok else self.nsteps)
+                         self.tile_launches if self.tplan is not None and ok else self.nsteps)
             _lib.check(lib.dcs_accumulate_batched(
                 self.dcode, _lib.ptr(self.table), self.table_stride, self.plan.terminal_rank,
                 self.term_runs.ctypes.data, self.term_nruns, self.tbasis.ctypes.data,

@@ -160,6 +160,25 @@ def group_steps(steps, max_dim=13, low=4, max_steps=MAX_GROUP_STEPS, max_extra=1
     return spans
 
 
+def one_tile_spans(steps, dim, max_steps):
+    """Spans (first, count): stretches of steps whose slots all fit one tile of 2^dim entries, as long as
+    they get, and single steps between them."""
+    spans, j = [], 0
+    while j < len(steps):
+        U, count = 0, 0
+        while j + count < len(steps) and count < max_steps:
+            st = steps[j + count]
+            U |= slot_mask(st.active_in) | slot_mask(st.active_out)
+            if orbit_kind(st)[0] == KIND_GROW:
+                U |= 1 << st.pivot
+            if bin(U).count("1") > dim:
+                break
+            count += 1
+        spans.append((j, max(count, 1)))
+        j += max(count, 1)
+    return spans
+
+
 def _feasible_ends(steps, i, max_dim, low, max_steps, max_extra):
     """Ends j of the groups [i, j) that group_steps' rules allow (span of the orbit vectors and
     low bits <= max_dim, at most max_steps steps, slot universe <= rank + max_extra)."""

@@ -290,7 +290,9 @@ int dcs_fused_runs(void *table, const dcs_step *steps, int nsteps, const dcs_gro
  * params + i*param_stride, maxbits + i*maxbits_stride (word s + 1 receives the max of step s, for
  * complex128 of a group's last step s only; word 0 holds the bits of 1.0) and scale + i (all zero on entry).  The table is renormalised once per group, so
  * the weights of a group must not overflow or underflow the storage precision; the power of two that
- * a complex64 table still has is in table_exp.  Steps 0 .. nsteps - 1
+ * a complex64 table still has is in table_exp.  DCS_H16: groups of one tile (2^13 entries at most) run
+ * in one launch with every step's own renormalisation, the others a launch per step; maxbits_stride is
+ * nsteps + 1.  Steps 0 .. nsteps - 1
  * in groups that follow one another; steps, groups, tile_steps: host arrays. */
 int dcs_tile_groups(int dtype, void *table, uint64_t table_stride, const dcs_step *steps, int nsteps,
                     const dcs_group *groups, int ngroups, const dcs_tile_step *tile_steps, const dcs_param *params,

@@ -10,7 +10,7 @@ CIRCUITS = [(3, 3, 2, 1, 0), (6, 6, 9, 3, 0), (10, 12, 30, 4, 1), (14, 15, 50, 5
             (24, 27, 100, 8, 2), (30, 33, 120, 10, 0), (34, 38, 150, 11, 0)]
 
 
-def _engine(shape, dtype, items):
+def _engine(shape, dtype, items, **kw):
     from dcs245_classical_sampling_b200.circuits import build_ring_instance
     from dcs245_classical_sampling_b200.engine import InplaceConditionalBlockGPU
     from dcs245_classical_sampling_b200.workloads import choose_reference_slices, sweep_order
@@ -20,7 +20,7 @@ def _engine(shape, dtype, items):
     order = sweep_order(inst, opened)
     ops = choose_reference_slices(inst["graph"], n, order, slices, opened)
     eng = InplaceConditionalBlockGPU(inst["graph"], inst["unitaries"], n, order, [list(o) for o in ops], opened)
-    eng.alloc(dtype, mode="device", items=items)
+    eng.alloc(dtype, mode="device", items=items, **kw)
     return eng
 
 
@@ -51,6 +51,20 @@ def test_tile_groups_equal_steps(shape, dtype, items):
             # complex128: up to 40 steps' e ln 2 (below 100 together) summed per group, 100 ulps of exp's
             # argument; products and sums are the same, so a block that cancels to rounding noise is, too
             assert np.linalg.norm(g - v) <= 1e-12 * np.linalg.norm(v)
+
+
+@pytest.mark.parametrize("items", [1, 5])
+@pytest.mark.parametrize("shape", CIRCUITS, ids=lambda s: f"{s[0]}q")
+def test_half_tiles_equal_steps(shape, items):
+    """Binary16 tables: stretches of steps on one tile in one launch, the same bits (every step rounds)."""
+    eng = _engine(shape, np.complex64, items, storage="float16")
+    rng = np.random.default_rng(shape[0])
+    xs = [rng.integers(0, 2, shape[0]).astype(np.uint8) for _ in range(4)]
+    for plan in (eng.tplan, eng._build_tplan(6, 2), eng._build_tplan(11, 1)):
+        assert plan.spans[-1][0] + plan.spans[-1][1] == eng.nsteps
+        eng.tplan = plan
+        got, want = _both(eng, xs)
+        assert np.array_equal(got, want)
 
 
 def test_weights_outside_the_range_take_single_steps():
