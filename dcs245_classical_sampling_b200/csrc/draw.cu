@@ -52,12 +52,13 @@ __device__ __forceinline__ dd dd_mul(dd a, double b) {  // Dekker product with F
     const double e = fma(a.hi, b, -p);
     return fast_two_sum(p, __dadd_rn(e, __dmul_rn(a.lo, b)));
 }
-__device__ __forceinline__ double dd_div(dd a, dd b) {  // a / b to ~1 ulp
-    if (b.hi == 0.0) return 0.0;
-    const double q = a.hi / b.hi;
+// a / b for b != 0, inv = 1 / b.hi: a first quotient, and the exact remainder's (double-double long division, as
+// in Hida, Li and Bailey's library), which is 2^-52 of it, so that neither needs a division of its own
+__device__ __forceinline__ double dd_div(dd a, dd b, double inv) {
+    const double q = a.hi * inv;
     const dd qb = dd_mul(b, q);
     const dd r = dd_add(a, dd{-qb.hi, -qb.lo});
-    return q + r.hi / b.hi;
+    return fma(r.hi, inv, q);
 }
 __device__ __forceinline__ bool dd_lt(dd a, dd b) { return a.hi < b.hi || (a.hi == b.hi && a.lo < b.lo); }
 
@@ -277,13 +278,13 @@ __device__ __forceinline__ void chunk_maps(const double (&loc)[kPer], double bef
     const bool inside = some && e0 == e1 && e0 > -900 && e0 < 1000;
     long long d0 = 0, d1 = 0;
     if (inside) {
-        // increments from an even and from an odd k of the same binade: 2^e and 2^e + q
+        // increments from an even and from an odd k of the same binade, 2^e and 2^e + q (inside a binade an
+        // increment of k is one of the bit pattern)
         const double even = __hiloint2double((e0 + 1023) << 20, 0), odd = __hiloint2double((e0 + 1023) << 20, 1);
-        const double inv_q = __hiloint2double((1023 + 52 - e0) << 20, 0);
 #pragma unroll
         for (int j = 0; j < kPer; ++j)
-            map_then(d0, d1, (long long)__dmul_rn(__dsub_rn(__dadd_rn(even, loc[j]), even), inv_q),
-                     (long long)__dmul_rn(__dsub_rn(__dadd_rn(odd, loc[j]), odd), inv_q));
+            map_then(d0, d1, __double_as_longlong(__dadd_rn(even, loc[j])) - __double_as_longlong(even),
+                     __double_as_longlong(__dadd_rn(odd, loc[j])) - __double_as_longlong(odd));
     }
 #pragma unroll
     for (int off = 1; off < kSubThreads; off <<= 1) {
@@ -348,7 +349,8 @@ k_chunk(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, i
                    sub_map + (uint64_t)b * (n >= (uint64_t)kSub ? n / kSub : 1));
     dd run = before;
     const double two53 = 9007199254740992.0;
-    double prev_end = ceil(dd_div(run, T) * two53);
+    const double inv = 1.0 / T.hi;  // T.hi > 0
+    double prev_end = ceil(dd_div(run, T, inv) * two53);
     if (start + (uint64_t)threadIdx.x * kPer == 0) prev_end = 0.0;
     double s = 0.0, q = 0.0;
 #pragma unroll
@@ -356,7 +358,7 @@ k_chunk(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, i
         const uint64_t i = start + (uint64_t)threadIdx.x * kPer + j;
         if (i >= n) break;
         run = dd_add(run, loc[j]);
-        const double ci = (i == n - 1) ? 1.0 : dd_div(run, T);
+        const double ci = (i == n - 1) ? 1.0 : dd_div(run, T, inv);
         const double end = ceil(ci * two53);
         const double p = loc[j] / mass;
         s += fabs((end - prev_end) / two53 - p);
@@ -422,68 +424,171 @@ k_chunk(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, i
     }
 }
 
-// S after a stretch with map m, or false when S is not where the map holds (the weights are then added
-// one by one): S of one binade is an integer in its bit pattern, so the increment is an integer addition.
-__device__ __forceinline__ bool seq_apply(long long& S, const SeqMap& m) {
-    if (m.e == kMapNone) return true;
-    const long long t = S + ((S & 1) ? m.d1 : m.d0);
-    if ((int)(S >> 52) - 1023 != m.e || (int)(t >> 52) - 1023 != m.e) return false;  // kMapWalk: never equal
-    S = t;
-    return true;
-}
-// S after the weights [i0, i1) added one by one (one warp, the same S in every lane; i1 - i0 <= kSub);
-// out: optional array for S after each
-__device__ __forceinline__ double seq_walk(const double* __restrict__ wb, uint64_t i0, uint64_t i1, double S,
-                                           double* out) {
+// Inclusive scan of maps over a warp's lanes (lane 0 first): d0 / d1 become the increments from before lane 0.
+__device__ __forceinline__ void map_scan(long long& d0, long long& d1) {
     const int lane = threadIdx.x & 31;
-    double v[kSub / 32];
+    if (__all_sync(0xffffffffu, d0 == d1)) {  // no ties, as almost always: a sum (a third of the general scan's time)
 #pragma unroll
-    for (int q = 0; q < kSub / 32; ++q) {
-        const uint64_t i = i0 + q * 32 + lane;
-        v[q] = i < i1 ? wb[i] : 0.0;  // adding zero changes nothing
-    }
-#pragma unroll
-    for (int q = 0; q < kSub / 32; ++q) {
-        if (i0 + q * 32 >= i1) break;
-        double keep = 0.0;
-#pragma unroll
-        for (int j = 0; j < 32; ++j) {
-            S = __dadd_rn(S, __shfl_sync(0xffffffffu, v[q], j));
-            if (j == lane) keep = S;
+        for (int off = 1; off < 32; off <<= 1) {
+            const long long a = __shfl_up_sync(0xffffffffu, d0, off);
+            if (lane >= off) d0 += a;
         }
-        if (out) out[q * 32 + lane] = keep;
+        d1 = d0;
+        return;
     }
-    return S;
+#pragma unroll
+    for (int off = 1; off < 32; off <<= 1) {
+        long long a0 = __shfl_up_sync(0xffffffffu, d0, off), a1 = __shfl_up_sync(0xffffffffu, d1, off);
+        map_then(a0, a1, d0, d1);
+        if (lane >= off) {
+            d0 = a0;
+            d1 = a1;
+        }
+    }
+}
+__device__ __forceinline__ int exponent_of(long long bits) { return (int)(bits >> 52) - 1023; }
+
+// S (its bit pattern, the same in every lane) through the maps of lanes pos .. stop - 1, the longest run whose
+// maps hold for S's binade; returns stop <= cnt.  `start` receives S before the lane's stretch for lanes pos ..
+// stop.  S of one binade is an integer in its bit pattern, so an increment is an integer addition.
+__device__ __forceinline__ int seq_run(long long& S, const SeqMap& m, int pos, int cnt, double& start) {
+    const int lane = threadIdx.x & 31;
+    const int es = exponent_of(S);
+    const bool here = lane >= pos && lane < cnt;
+    const unsigned bad = __ballot_sync(0xffffffffu, here && m.e != kMapNone && m.e != es);  // kMapWalk: always
+    int stop = bad ? __ffs(bad) - 1 : cnt;
+    long long d0 = 0, d1 = 0;
+    if (here && lane < stop && m.e != kMapNone) {
+        d0 = m.d0;
+        d1 = m.d1;
+    }
+    map_scan(d0, d1);
+    const long long after = S + ((S & 1) ? d1 : d0);
+    long long before = __shfl_up_sync(0xffffffffu, after, 1);
+    if (lane == 0) before = S;
+    // (maps are made only where S cannot leave the binade; were it to, the stretch would be walked)
+    const unsigned left = __ballot_sync(0xffffffffu, here && lane < stop && m.e != kMapNone && exponent_of(after) != es);
+    if (left) stop = __ffs(left) - 1;
+    if (lane >= pos && lane <= stop) start = __longlong_as_double(before);
+    if (stop > pos) S = __shfl_sync(0xffffffffu, after, stop - 1);
+    return stop;
 }
 
-// S after chunk c from S before it (one warp); stop >= 0: only up to the start of sub-chunk `stop`
+// S after the weights [i0, i1) of one sub-chunk (one warp, the same S in every lane); out: optional array for S after
+// each.  Four consecutive weights per lane; their maps in S's binade are scanned, the first weight that leaves the
+// binade is added itself, and the rest goes on in the new one: two scans where 128 dependent additions (2600
+// cycles) were.
+__device__ __forceinline__ double seq_walk(const double* __restrict__ wb, uint64_t i0, uint64_t i1, double S0, double* out) {
+    constexpr int kOwn = kSub / 32;
+    const int lane = threadIdx.x & 31;
+    const int n = (int)(i1 - i0);
+    double v[kOwn];
+#pragma unroll
+    for (int r = 0; r < kOwn; ++r) {
+        const int i = lane * kOwn + r;
+        v[r] = i < n ? wb[i0 + i] : 0.0;  // adding zero changes nothing
+    }
+    int pos = 0;
+    if (i0 == 0) {  // the sum of the first few weights leaves a binade with nearly every one
+        const int lim = n < 16 ? n : 16;
+        for (; pos < lim; ++pos) {
+            double w = v[0];
+#pragma unroll
+            for (int r = 1; r < kOwn; ++r)
+                if (r == (pos & (kOwn - 1))) w = v[r];
+            S0 = __dadd_rn(S0, __shfl_sync(0xffffffffu, w, pos / kOwn));
+            if (out && lane == 0) out[pos] = S0;
+        }
+    }
+    long long S = __double_as_longlong(S0);
+    while (pos < n) {
+        const int es = exponent_of(S);
+        int at = pos;  // the weight to add itself
+        if (es > -900 && es < 1000) {
+            const double even = __hiloint2double((es + 1023) << 20, 0), odd = __hiloint2double((es + 1023) << 20, 1);
+            long long c0[kOwn], c1[kOwn], d0 = 0, d1 = 0;
+#pragma unroll
+            for (int r = 0; r < kOwn; ++r) {
+                if (lane * kOwn + r >= pos)
+                    map_then(d0, d1, __double_as_longlong(__dadd_rn(even, v[r])) - __double_as_longlong(even),
+                             __double_as_longlong(__dadd_rn(odd, v[r])) - __double_as_longlong(odd));
+                c0[r] = d0;
+                c1[r] = d1;
+            }
+            map_scan(d0, d1);
+            long long e0 = __shfl_up_sync(0xffffffffu, d0, 1), e1 = __shfl_up_sync(0xffffffffu, d1, 1);
+            if (lane == 0) e0 = e1 = 0;
+            const long long before = S + ((S & 1) ? e1 : e0);  // before the lane's weights
+            long long k[kOwn];
+            int first = kOwn;
+#pragma unroll
+            for (int r = kOwn - 1; r >= 0; --r) {
+                k[r] = before + ((before & 1) ? c1[r] : c0[r]);
+                const int i = lane * kOwn + r;
+                if (i >= pos && i < n && (v[r] >= even || exponent_of(k[r]) != es)) first = r;
+            }
+            const unsigned any = __ballot_sync(0xffffffffu, first < kOwn);
+            const int who = any ? __ffs(any) - 1 : 31;
+            const int r0 = __shfl_sync(0xffffffffu, first, who);
+            at = any ? who * kOwn + r0 : n;
+            if (out) {
+#pragma unroll
+                for (int r = 0; r < kOwn; ++r) {
+                    const int i = lane * kOwn + r;
+                    if (i >= pos && i < at && i < n) out[i] = __longlong_as_double(k[r]);
+                }
+            }
+            // S before the weight `at` (after all of them when there is none)
+            long long prev = before;
+#pragma unroll
+            for (int r = 0; r < kOwn; ++r)
+                if (r < r0) prev = k[r];
+            S = __shfl_sync(0xffffffffu, prev, who);
+        }
+        if (at < n) {
+            double w = 0.0;
+#pragma unroll
+            for (int r = 0; r < kOwn; ++r)
+                if (r == (at & (kOwn - 1))) w = v[r];
+            w = __shfl_sync(0xffffffffu, w, at / kOwn);
+            const double s = __dadd_rn(__longlong_as_double(S), w);
+            if (out && lane == 0) out[at] = s;
+            S = __double_as_longlong(s);
+        }
+        pos = at + 1;
+    }
+    return __longlong_as_double(S);
+}
+
+// S after chunk c from S before it (one warp); sub_start: optional array for S before each of its sub-chunks
 __device__ __forceinline__ double seq_chunk(const double* __restrict__ wb, uint64_t n, uint64_t c,
-                                            const SeqMap* __restrict__ sub_map, double S, double* sub_start) {
+                                            const SeqMap* __restrict__ sub_map, double S0, double* sub_start) {
     const int lane = threadIdx.x & 31;
     const uint64_t g0 = c * kSubs;
+    const uint64_t left = ((n - c * kChunk) + kSub - 1) / kSub;
+    const int cnt = left < kSubs ? (int)left : kSubs;
     SeqMap mine{0, 0, kMapNone, 0};
-    if (lane < kSubs && (g0 + lane) * kSub < n) mine = sub_map[g0 + lane];
-    for (int j = 0; j < kSubs; ++j) {
-        if ((g0 + j) * kSub >= n) break;
-        if (sub_start && lane == 0) sub_start[j] = S;
-        SeqMap m;
-        m.d0 = __shfl_sync(0xffffffffu, mine.d0, j);
-        m.d1 = __shfl_sync(0xffffffffu, mine.d1, j);
-        m.e = __shfl_sync(0xffffffffu, mine.e, j);
-        long long bits = __double_as_longlong(S);
-        const uint64_t i0 = (g0 + j) * kSub;
-        if (seq_apply(bits, m)) S = __longlong_as_double(bits);
-        else S = seq_walk(wb, i0, i0 + kSub < n ? i0 + kSub : n, S, nullptr);
+    if (lane < cnt) mine = sub_map[g0 + lane];
+    long long S = __double_as_longlong(S0);
+    double start = 0.0;
+    for (int pos = 0; pos < cnt;) {
+        const int stop = seq_run(S, mine, pos, cnt, start);
+        if (stop < cnt) {
+            const uint64_t i0 = (g0 + stop) * kSub;
+            S = __double_as_longlong(seq_walk(wb, i0, i0 + kSub < n ? i0 + kSub : n, __longlong_as_double(S), nullptr));
+        }
+        pos = stop + 1;
     }
-    return S;
+    if (sub_start && lane < cnt) sub_start[lane] = start;
+    return __longlong_as_double(S);
 }
 
 // 4. totals of the chunk sums, and the exact sequential FP64 CDF (numpy's operation order) for blocks
-//    flagged as ties, or for every block when `force` (one CTA per block).  Warp 0 carries S from chunk
-//    to chunk by the maps; chunks that cross a binade (about log2 of the block size of them) go through their
-//    sub-chunks' maps, and the one or two sub-chunks that cross are added up one weight after the other.
-//    The chain of n dependent additions this replaces took 10.9 ms for 2^20 weights; carrying S over 512
-//    chunks with 10 crossings takes about 30 us.  The selected chunk (and sub-chunk) is the last one whose
+//    flagged as ties, or for every block when `force` (one CTA per block).  Warp 0 carries S over runs of
+//    chunks by scanning their maps; chunks that cross a binade (about log2 of the block size of them) go through
+//    their sub-chunks' maps, and the one or two sub-chunks that cross through their weights'.
+//    The chain of n dependent additions this replaces took 10.9 ms for 2^20 weights; chunk by chunk, with
+//    dependent additions in the sub-chunks that cross, the kernel took 93 us, so 53.  The selected chunk (and sub-chunk) is the last one whose
 //    starting value satisfies fl(start / S_n) <= u (fl(x / S_n) is non-decreasing in x), and only the
 //    selected sub-chunk is replayed.  The compensated interval of the selected index is checked
 //    against u as the reference's independent check does (sampling_protocol.py:67-72).
@@ -532,25 +637,23 @@ k_finish(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, 
     if (threadIdx.x == 0) at = 0;
     __syncthreads();
     if (threadIdx.x < 32) {
-        double S = 0.0;
+        long long S = 0;
+        SeqMap next{0, 0, kMapNone, 0};
+        if (lane < nch) next = cm[lane].map;
         for (int c0 = 0; c0 < nch; c0 += 32) {
-            SeqMap mine{0, 0, kMapNone, 0};
-            if (c0 + lane < nch) mine = cm[c0 + lane].map;
-            double started = 0.0;
+            const SeqMap mine = next;
+            if (c0 + 32 + lane < nch) next = cm[c0 + 32 + lane].map;  // on its way while these are scanned
+            double start = 0.0;
             const int cnt = nch - c0 < 32 ? nch - c0 : 32;
-            for (int j = 0; j < cnt; ++j) {
-                if (j == lane) started = S;
-                SeqMap m;
-                m.d0 = __shfl_sync(0xffffffffu, mine.d0, j);
-                m.d1 = __shfl_sync(0xffffffffu, mine.d1, j);
-                m.e = __shfl_sync(0xffffffffu, mine.e, j);
-                long long bits = __double_as_longlong(S);
-                if (seq_apply(bits, m)) S = __longlong_as_double(bits);
-                else S = seq_chunk(wb, n, c0 + j, sb, S, nullptr);
+            for (int pos = 0; pos < cnt;) {
+                const int stop = seq_run(S, mine, pos, cnt, start);
+                if (stop < cnt)
+                    S = __double_as_longlong(seq_chunk(wb, n, c0 + stop, sb, __longlong_as_double(S), nullptr));
+                pos = stop + 1;
             }
-            if (c0 + lane < nch) cm[c0 + lane].start = started;
+            if (c0 + lane < nch) cm[c0 + lane].start = start;
         }
-        if (lane == 0) s_total = S;
+        if (lane == 0) s_total = __longlong_as_double(S);
     }
     __syncthreads();
     const double S = s_total;
