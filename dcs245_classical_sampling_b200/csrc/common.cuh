@@ -108,6 +108,15 @@ __device__ __forceinline__ int scale_exponent(double m2) {
     return e;
 }
 
+// The same from the exponent alone, without the square root: m2 in [2^E, 2^(E+1)) has sqrt(m2) in
+// [2^floor(E/2), 2^(floor(E/2)+1)).  For m2 whose square root is not within half an ulp of a power of two from
+// below, as every float and every double with 32 zero low bits; subnormal m2 take the general way.
+__device__ __forceinline__ int scale_exponent_fast(double m2) {
+    const int h = __double2hiint(m2) >> 20;  // m2 >= 0
+    if (h == 0 || h == 0x7ff) return scale_exponent(m2);
+    return ((h - 1023) >> 1) + 1;
+}
+
 // block-wide max of an unsigned 64-bit value; result valid in thread 0
 __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v) {
     __shared__ unsigned long long red[32];

@@ -534,9 +534,9 @@ int run_groups(S* table, uint64_t table_stride, const dcs_step* steps, int nstep
     return DCS_OK;
 }
 
-// Binary16 tables: groups whose table is one tile in one launch, the others a launch per step.  A step's
-// launch is 5 us here, a step of a 2^12-entry tile in shared memory about 1: a 20-qubit block (60 steps, one
-// tile throughout) takes a quarter of the time, and a 48-qubit one starts its 208 steps with one launch for 24.
+// Binary16 tables: groups whose table is one tile in one launch, the others a launch per step.  A block with a
+// launch per step / so: 16 qubits (31 steps, 2 launches) 301 / 191 us, 24 qubits (72, 3) 452 / 230, 32 qubits
+// (97, 25; 2^16 entries at the largest) 583 / 377.
 int run_half_groups(ushort2* table, uint64_t table_stride, const dcs_step* steps, int nsteps, const dcs_group* groups,
                     int ngroups, const dcs_tile_step* tile_steps, const dcs_param* params, uint64_t param_stride,
                     uint64_t* maxbits, dcs_scale* scale, int nitems, cudaStream_t st) {
