@@ -33,10 +33,11 @@ struct ItemTerm {
 
 template <class S>
 __global__ void __launch_bounds__(256)
-k_accumulate(const S* __restrict__ table, uint64_t table_stride, const __grid_constant__ TermMap tm,
-             const uint64_t* __restrict__ xors, const double* __restrict__ coefs, const int32_t* __restrict__ item_begin,
-             double log_shift, dcs_scale* __restrict__ scale, const unsigned long long* __restrict__ maxbits_final,
-             uint64_t mstride, int is64, double2* __restrict__ total) {
+k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ TermMap tm, const uint64_t* xors,
+             const double* coefs, const int32_t* item_begin, double log_shift, dcs_scale* scale,
+             const unsigned long long* maxbits_final, uint64_t mstride, int is64, double2* total) {
+    let_next_start();
+    after_previous();
     // grid.y = output block; items item_begin[b] .. item_begin[b+1]-1 belong to block b
     constexpr int kTerms = 64;  // items whose terms sit in shared memory at a time
     __shared__ ItemTerm terms[kTerms];
@@ -181,6 +182,8 @@ k_tail(double2* __restrict__ total, const __grid_constant__ TailParams tp, int a
        int tb_hi) {
     extern __shared__ double2 sh[];
     const int k = tp.k;
+    let_next_start();
+    after_previous();
     const int tile_log = a + (b_hi - b_lo);
     const int tsize = 1 << tile_log;
     const uint64_t nblk_elems = 1ull << k;
@@ -235,9 +238,9 @@ int tail_pass(double2* total, const TailParams& tp, int a, int b_lo, int b_hi, i
     }
     // (a swizzled index stays inside its row of eight)
     const size_t smem = sizeof(double2) << (tile_log > 3 ? tile_log : 3);
-    k_tail<MODE><<<(unsigned)tiles, threads, smem, st>>>(total, tp, a, b_lo, b_hi, tb_lo, tb_hi);
-    DCS_CHECK_LAUNCH("k_tail launch");
-    return DCS_OK;
+    return dcs_host::check_cuda(dcs_host::launch_after(k_tail<MODE>, dim3((unsigned)tiles), dim3(threads), smem, st, total, tp, a,
+                                                       b_lo, b_hi, tb_lo, tb_hi),
+                                "k_tail launch");
 }
 
 }  // namespace
@@ -307,24 +310,18 @@ extern "C" int dcs_accumulate_batched(int dtype, const void* table, uint64_t tab
     const uint64_t cap = (uint64_t)dcs_host::sm_count() * 8;
     if (bx > cap) bx = cap;
     dim3 grid((unsigned)bx, (unsigned)nblocks);
-    if (dtype == DCS_C64)
-        k_accumulate<float2><<<grid, 256, 0, st>>>((const float2*)table, table_stride, tm, xors, coefs, item_begin,
-                                                   log_shift, scale, (const unsigned long long*)maxbits_final, mstride,
-                                                   0, (double2*)total);
-    else if (dtype == DCS_C128)
-        k_accumulate<double2><<<grid, 256, 0, st>>>((const double2*)table, table_stride, tm, xors, coefs, item_begin,
-                                                    log_shift, scale, (const unsigned long long*)maxbits_final,
-                                                    mstride, 1, (double2*)total);
-    else if (dtype == DCS_H16)
-        k_accumulate<ushort2><<<grid, 256, 0, st>>>((const ushort2*)table, table_stride, tm, xors, coefs, item_begin,
-                                                    log_shift, scale, (const unsigned long long*)maxbits_final,
-                                                    mstride, 0, (double2*)total);
-    else {
-        dcs_host::set_error("dcs_accumulate: unknown dtype %d", dtype);
-        return DCS_E_ARG;
-    }
-    DCS_CHECK_LAUNCH("k_accumulate launch");
-    return DCS_OK;
+    auto run = [&](auto kernel, auto t) {
+        return dcs_host::check_cuda(
+            dcs_host::launch_after(kernel, grid, dim3(256), 0, st, t, table_stride, tm, xors, coefs, item_begin, log_shift, scale,
+                                   (const unsigned long long*)maxbits_final, mstride, dtype == DCS_C128 ? 1 : 0,
+                                   (double2*)total),
+            "k_accumulate launch");
+    };
+    if (dtype == DCS_C64) return run(k_accumulate<float2>, (const float2*)table);
+    if (dtype == DCS_C128) return run(k_accumulate<double2>, (const double2*)table);
+    if (dtype == DCS_H16) return run(k_accumulate<ushort2>, (const ushort2*)table);
+    dcs_host::set_error("dcs_accumulate: unknown dtype %d", dtype);
+    return DCS_E_ARG;
 }
 
 extern "C" int dcs_block_tail(double* total, int k, const uint32_t* adj_hi, const double* u_open, int nblocks,

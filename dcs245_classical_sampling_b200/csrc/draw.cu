@@ -25,6 +25,9 @@
 
 #include "common.cuh"
 
+using dcs::after_previous;
+using dcs::let_next_start;
+
 namespace {
 
 struct dd { double hi, lo; };
@@ -180,6 +183,7 @@ k_weights(const double2* __restrict__ blocks, int k, double* __restrict__ w, dd*
     double* wb = w + ((uint64_t)b << k);
     dd acc{0.0, 0.0};
     int bad = 0;
+    let_next_start();
 #pragma unroll
     for (int j = 0; j < kPer; ++j) {
         const uint64_t i = start + threadIdx.x + (uint64_t)j * kThreads;
@@ -202,8 +206,10 @@ k_weights(const double2* __restrict__ blocks, int k, double* __restrict__ w, dd*
 // 2. chunk scan + chunk search, one CTA per block.  A 2^20 block has 512 chunks: one thread walking them
 //    took 69 us (a dependent load, store and addition per chunk), the scan takes about 5.
 __global__ void __launch_bounds__(kThreads)
-k_scan_locate(dd* __restrict__ chunk_sum, int nch, const double* __restrict__ uniforms,
-              BlockState* __restrict__ state, dcs_draw_result* __restrict__ res, const double* __restrict__ part) {
+k_scan_locate(dd* chunk_sum, int nch, const double* uniforms, BlockState* state, dcs_draw_result* res,
+              const double* part) {
+    let_next_start();
+    after_previous();
     const int b = blockIdx.x;
     dd* cs = chunk_sum + (uint64_t)b * nch;
     __shared__ int at;
@@ -259,8 +265,7 @@ __device__ __forceinline__ void map_then(long long& a0, long long& a1, long long
 // The maps of one chunk's sub-chunks and of the chunk (all threads of the CTA): thread t owns the
 // weights loc[] of elements kPer t .. kPer t + kPer - 1 and `before`, the prefix sum before them.
 __device__ __forceinline__ void chunk_maps(const double (&loc)[kPer], double before, uint64_t n, uint64_t c,
-                                           uint64_t nch, SeqChunk* __restrict__ chunk_map,
-                                           SeqMap* __restrict__ sub_map) {
+                                           uint64_t nch, SeqChunk* chunk_map, SeqMap* sub_map) {
     constexpr int kGroups = kThreads / kSubThreads;
     __shared__ SeqMap sm[kGroups];
     const int lane = threadIdx.x & 31;
@@ -323,9 +328,10 @@ __device__ __forceinline__ void chunk_maps(const double (&loc)[kPer], double bef
 //    element search with its certification, and on request (maps) the sequential CDF's maps.  The three
 //    need the same prefix sums of the chunk's weights.
 __global__ void __launch_bounds__(kThreads)
-k_chunk(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, int nch,
-        const BlockState* __restrict__ state, dcs_draw_result* __restrict__ res, double* __restrict__ part,
-        double* __restrict__ sq_part, SeqChunk* __restrict__ chunk_map, SeqMap* __restrict__ sub_map, int maps) {
+k_chunk(const double* w, int k, const dd* chunk_sum, int nch, const BlockState* state, dcs_draw_result* res, double* part,
+        double* sq_part, SeqChunk* chunk_map, SeqMap* sub_map, int maps) {
+    let_next_start();
+    after_previous();
     const int b = blockIdx.y;
     const int c = blockIdx.x;
     const uint64_t n = 1ull << k;
@@ -478,7 +484,7 @@ __device__ __forceinline__ int seq_run(long long& S, const SeqMap& m, int pos, i
 // each.  Four consecutive weights per lane; their maps in S's binade are scanned, the first weight that leaves the
 // binade is added itself, and the rest goes on in the new one: two scans where 128 dependent additions (2600
 // cycles) were.
-__device__ __forceinline__ double seq_walk(const double* __restrict__ wb, uint64_t i0, uint64_t i1, double S0, double* out) {
+__device__ __forceinline__ double seq_walk(const double* wb, uint64_t i0, uint64_t i1, double S0, double* out) {
     constexpr int kOwn = kSub / 32;
     const int lane = threadIdx.x & 31;
     const int n = (int)(i1 - i0);
@@ -561,8 +567,7 @@ __device__ __forceinline__ double seq_walk(const double* __restrict__ wb, uint64
 }
 
 // S after chunk c from S before it (one warp); sub_start: optional array for S before each of its sub-chunks
-__device__ __forceinline__ double seq_chunk(const double* __restrict__ wb, uint64_t n, uint64_t c,
-                                            const SeqMap* __restrict__ sub_map, double S0, double* sub_start) {
+__device__ __forceinline__ double seq_chunk(const double* wb, uint64_t n, uint64_t c, const SeqMap* sub_map, double S0, double* sub_start) {
     const int lane = threadIdx.x & 31;
     const uint64_t g0 = c * kSubs;
     const uint64_t left = ((n - c * kChunk) + kSub - 1) / kSub;
@@ -593,10 +598,9 @@ __device__ __forceinline__ double seq_chunk(const double* __restrict__ wb, uint6
 //    selected sub-chunk is replayed.  The compensated interval of the selected index is checked
 //    against u as the reference's independent check does (sampling_protocol.py:67-72).
 __global__ void __launch_bounds__(kThreads)
-k_finish(const double* __restrict__ w, int k, const dd* __restrict__ chunk_sum, int nch,
-         const BlockState* __restrict__ state, dcs_draw_result* __restrict__ res, const double* __restrict__ part,
-         const double* __restrict__ sq_part, SeqChunk* __restrict__ chunk_map, SeqMap* __restrict__ sub_map,
-         int force) {
+k_finish(const double* w, int k, const dd* chunk_sum, int nch, const BlockState* state, dcs_draw_result* res,
+         const double* part, const double* sq_part, SeqChunk* chunk_map, SeqMap* sub_map, int force) {
+    after_previous();
     const int b = blockIdx.x;
     const int lane = threadIdx.x & 31;
     dcs_draw_result& r = res[b];
@@ -732,6 +736,7 @@ constexpr int kOverlapParts = kThreads;  // partial sums, one CTA each: 16 KiB o
 
 __global__ void __launch_bounds__(kThreads)
 k_overlap(const double2* __restrict__ ref, const double2* __restrict__ ap, uint64_t len, dd* __restrict__ part) {
+    let_next_start();
     constexpr int kIn = 4;  // entries in flight per thread: one at a time left the loads' latency exposed
     dd rr{0, 0}, aa{0, 0}, re{0, 0}, im{0, 0};
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
@@ -766,7 +771,8 @@ k_overlap(const double2* __restrict__ ref, const double2* __restrict__ ap, uint6
 
 // A thread per partial sum (four threads walking the 256 of them took 24 us, the first pass 9).
 __global__ void __launch_bounds__(kThreads)
-k_overlap_final(const dd* __restrict__ part, double* __restrict__ out) {
+k_overlap_final(const dd* part, double* out) {
+    after_previous();
 #pragma unroll
     for (int q = 0; q < 4; ++q) {
         const dd s = block_sum_dd(part[4 * threadIdx.x + q]);
@@ -799,13 +805,21 @@ int enqueue_draw(const double* blocks, int k, int nblocks, const double* uniform
     const int force = (flags & DCS_DRAW_SEQUENTIAL) ? 1 : 0;
     k_weights<<<dim3(nch, nblocks), kThreads, 0, s>>>((const double2*)blocks, k, w, cs, part);
     DCS_CHECK_LAUNCH("k_weights");
-    k_scan_locate<<<nblocks, kThreads, 0, s>>>(cs, nch, uniforms, st, results, part);
-    DCS_CHECK_LAUNCH("k_scan_locate");
-    k_chunk<<<dim3(nch, nblocks), kThreads, 0, s>>>(w, k, cs, nch, st, results, part, sq, cm, sm, force);
-    DCS_CHECK_LAUNCH("k_chunk");
-    k_finish<<<nblocks, kThreads, 0, s>>>(w, k, cs, nch, st, results, part, sq, cm, sm, force);
-    DCS_CHECK_LAUNCH("k_finish");
-    return DCS_OK;
+    // (what these read is written by the launch before, which may still run when they start: none of their
+    // pointers is declared read-only)
+    using dcs_host::check_cuda;
+    using dcs_host::launch_after;
+    int rc = check_cuda(launch_after(k_scan_locate, dim3(nblocks), dim3(kThreads), 0, s, cs, nch, uniforms, st, results, part),
+                        "k_scan_locate");
+    if (!rc)
+        rc = check_cuda(launch_after(k_chunk, dim3(nch, nblocks), dim3(kThreads), 0, s, w, k, cs, nch, st, results, part, sq, cm,
+                                     sm, force),
+                        "k_chunk");
+    if (!rc)
+        rc = check_cuda(launch_after(k_finish, dim3(nblocks), dim3(kThreads), 0, s, w, k, cs, nch, st, results, part, sq, cm, sm,
+                                     force),
+                        "k_finish");
+    return rc;
 }
 }  // namespace
 
@@ -833,9 +847,8 @@ extern "C" int dcs_overlap(const double* ref, const double* ap, uint64_t len, do
     cudaStream_t s = (cudaStream_t)stream;
     k_overlap<<<kOverlapParts, kThreads, 0, s>>>((const double2*)ref, (const double2*)ap, len, (dd*)scratch);
     DCS_CHECK_LAUNCH("k_overlap");
-    k_overlap_final<<<1, kThreads, 0, s>>>((const dd*)scratch, out);
-    DCS_CHECK_LAUNCH("k_overlap_final");
-    return DCS_OK;
+    return dcs_host::check_cuda(dcs_host::launch_after(k_overlap_final, dim3(1), dim3(kThreads), 0, s, (const dd*)scratch, out),
+                                "k_overlap_final");
 }
 
 // ---------------------------------------------------------------- draw without allocation
