@@ -12,8 +12,8 @@
 // Bound: instruction issue (72% of the issue slots on 2048 tiles of 2^12 entries, 22 instructions per entry
 // and step); with a tile per SM or less, the latency of a step (two shared-memory accesses, the
 // products and a barrier).  A slice, device work and enqueueing, against one launch per step: 40 qubits (2^22
-// entries, 213 steps in 13 groups) 1320 -> 318 us, 48 qubits (2^24) 1830 -> 603 us, in complex128 2470 ->
-// 738 us; 16 slices of 40 qubits in one batch 4860 -> 1763 us.
+// entries, 213 steps in 13 groups) 911 -> 281 us, 48 qubits (2^24) 1414 -> 560 us, in complex128 2044 ->
+// 703 us; 16 slices of 40 qubits in one batch 4545 -> 1563 us.
 //
 // The orbit formulas are k_step's operation by operation (same products, same fused multiply-adds,
 // same order of additions).  The power of two of the renormalisation is applied once per group (exact).
@@ -35,6 +35,7 @@ namespace {
 
 constexpr int kMaxSteps = 24;
 constexpr int kMaxDim = 12;   // 32 KiB (complex64) or 64 KiB per tile
+constexpr int kManyTiles = 4;  // tiles per SM from which on 128 threads take one (run_groups)
 constexpr int kHalfDim = 13;  // binary16 tables: 32 KiB
 
 struct TileStep {
@@ -522,13 +523,17 @@ int run_groups(S* table, uint64_t table_stride, const dcs_step* steps, int nstep
             dcs_host::set_error("dcs_tile_groups: malformed group %d", gi);
             return DCS_E_ARG;
         }
-        // a tile per SM at most: 512 threads share it (a slice of 2^22 entries 5% faster than with 256); with
-        // more tiles CTAs of 256 threads hide each other's latencies better (512 for them: 2 to 15% slower)
-        const bool few = ((uint64_t)nitems << A.coset_m) <= (uint64_t)sms;
-        const int rc = few ? launch_group<S, 512>(table, table_stride, A, params, param_stride, maxbits, maxbits_stride,
-                                                  scale, nitems, sms, dev, st)
-                           : launch_group<S, 256>(table, table_stride, A, params, param_stride, maxbits, maxbits_stride,
-                                                  scale, nitems, sms, dev, st);
+        // A tile per SM at most: 512 threads share it (a slice of 2^22 entries 5% faster than with 256).  More: CTAs
+        // of 256 hide each other's latencies (512 for them: 2 to 15% slower).  Complex64 with many tiles per SM
+        // is bound by issue slots, and 128 threads spend fewer on each step's preparation (2^22 entries, 16
+        // slices: 1562 us against 1727; 512 tiles of 2^11: 146 against 138); the five 32 KiB tiles that an SM
+        // holds have warps enough then, the three 64 KiB ones of complex128 do not (3014 against 2156).
+        const uint64_t tiles = (uint64_t)nitems << A.coset_m;
+        const auto launch = tiles <= (uint64_t)sms                               ? launch_group<S, 512>
+                            : sizeof(S) == 8 && tiles > (uint64_t)kManyTiles * sms ? launch_group<S, 128>
+                                                                                  : launch_group<S, 256>;
+        const int rc = launch(table, table_stride, A, params, param_stride, maxbits, maxbits_stride, scale, nitems, sms, dev,
+                              st);
         if (rc) return rc;
     }
     return DCS_OK;

@@ -60,8 +60,8 @@ HALF_TILE_DIM = 13  # log2 of the largest binary16 table that one tile holds
 
 def tile_dim(maxslots):
     """log2 of the tile entries of device mode's tile groups for tables of 2^maxslots entries: 12 where
-    the whole table is one tile or there are tiles for many SMs (2^22 entries, 16 slices: 1763 us
-    against 2680 with 11), 11 between (2^16 entries, a slice: 149 against 154 us with 12)."""
+    the whole table is one tile or there are tiles for many SMs (2^22 entries, 16 slices: 1562 us
+    against 1816 with 11), 11 between (2^16 entries, a slice: 115 against 119 us with 12)."""
     return 12 if maxslots <= 12 or maxslots >= 18 else 11
 
 
