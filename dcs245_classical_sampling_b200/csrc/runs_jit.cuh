@@ -378,18 +378,27 @@ __device__ __forceinline__ real_t prologue(const jit_param* __restrict__ params,
     const double m2prev = (double)__uint_as_float((uint32_t)maxbits[group]);
 #endif
     const int e = scale_exponent(m2prev);
-    if (blockIdx.x == 0 && threadIdx.x == 0) {
+    if (blockIdx.x == 0 && threadIdx.x < 32) {
+        // a step factor's logarithm and argument per lane, added up in step order (one thread taking all of them
+        // in a row held every launch of a small table up by up to 15 us)
+        double lgi = 0.0, phi = 0.0;
+        if (threadIdx.x < COUNT) {
+            const double2 c = step_factor(params[FIRST + threadIdx.x], (FIXMASK >> threadIdx.x) & 1u);
+            lgi = 0.5 * log(c.x * c.x + c.y * c.y);
+            phi = atan2(c.y, c.x);
+        }
         double lg = 0.0, ph = 0.0;
         for (int i = 0; i < COUNT; ++i) {
-            const double2 c = step_factor(params[FIRST + i], (FIXMASK >> i) & 1u);
-            lg += 0.5 * log(c.x * c.x + c.y * c.y);
-            ph += atan2(c.y, c.x);
+            lg += __shfl_sync(0xffffffffu, lgi, i);
+            ph += __shfl_sync(0xffffffffu, phi, i);
         }
-        scale->logscale += (double)e * 0.69314718055994530942 + lg;
-        scale->phase += ph;
-        scale->exponent_sum += e;
-        if (!isfinite(m2prev)) scale->flags |= 1u;
-        else if (m2prev == 0.0) scale->flags |= 2u;
+        if (threadIdx.x == 0) {
+            scale->logscale += (double)e * 0.69314718055994530942 + lg;
+            scale->phase += ph;
+            scale->exponent_sum += e;
+            if (!isfinite(m2prev)) scale->flags |= 1u;
+            else if (m2prev == 0.0) scale->flags |= 2u;
+        }
     }
     if (threadIdx.x < COUNT) {
         const jit_param p = params[FIRST + threadIdx.x];
