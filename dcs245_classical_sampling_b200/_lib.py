@@ -17,6 +17,7 @@ LIB_PATH = PKG / "libdcs245.so"
 C64, C128, H16 = 0, 1, 2  # table storage: complex64, complex128, two binary16 components
 MAX_RUNS = 28
 E_ARG, E_CUDA, E_NONFINITE, E_CDF = -1, -2, -3, -4
+ACCUMULATE_FRESH = 1  # dcs_accumulate_ex flag: the blocks need not be zeroed before
 DRAW_SEQUENTIAL = 1  # dcs_draw_ex flag: numpy's sequential CDF pass for every block
 
 STEP_DTYPE = np.dtype([
@@ -76,6 +77,8 @@ SIGNATURES = {
     "dcs_tile_groups": (_I, [_I, _P, _U64, _P, _I, _P, _I, _P, _P, _U64, _P, _U64, _P, _I, _P]),
     "dcs_accumulate_batched": (_I, [_I, _P, _U64, _I, _P, _I, _P, _P, _P, _P, _I, _D, _P, _P, _U64, _P, _I, _I,
                                     _P]),
+    "dcs_accumulate_ex": (_I, [_I, _P, _U64, _I, _P, _I, _P, _P, _P, _P, _I, _D, _P, _P, _U64, _P, _I, _I,
+                               ctypes.c_uint, _P]),
     "dcs_block_tail": (_I, [_P, _I, _P, _P, _I, _P]),
     "dcs_gather_steps": (_I, [_I, _P, _P, _U64, _P, _P, _P, _U64, _I, _I, _P, _U64, _P, _I, _P]),
     "dcs_draw_scratch_bytes": (ctypes.c_size_t, [_I, _I]),

@@ -35,7 +35,7 @@ template <class S>
 __global__ void __launch_bounds__(256)
 k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ TermMap tm, const uint64_t* xors,
              const double* coefs, const int32_t* item_begin, double log_shift, dcs_scale* scale,
-             const unsigned long long* maxbits_final, uint64_t mstride, int is64, double2* total) {
+             const unsigned long long* maxbits_final, uint64_t mstride, int is64, int fresh, double2* total) {
     let_next_start();
     after_previous();
     // grid.y = output block; items item_begin[b] .. item_begin[b+1]-1 belong to block b
@@ -45,7 +45,8 @@ k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ Term
     const int i0 = item_begin[blk], i1 = item_begin[blk + 1];
     double2* out = total + ((uint64_t)blk << tm.k);
     const uint64_t n = 1ull << tm.k;
-    for (int c0 = i0; c0 < i1; c0 += kTerms) {
+    int c0 = i0;
+    do {  // (a block without items is written once, too, when it starts at zero)
         const int cn = i1 - c0 < kTerms ? i1 - c0 : kTerms;
         __syncthreads();
         // an exponential and a sine per item and CTA; per item and entry they were most of the kernel
@@ -65,8 +66,8 @@ k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ Term
             if (sc.phase != 0.0) {  // step factors divided out by the plan-specialised kernels
                 double sp, cp;
                 sincos(sc.phase, &sp, &cp);
-                const double r = cr * cp - ci * sp;
-                ci = cr * sp + ci * cp;
+                const double r = __fma_rn(cr, cp, -__dmul_rn(ci, sp));
+                ci = __fma_rn(cr, sp, __dmul_rn(ci, cp));
                 cr = r;
             }
             t.cr = cr;
@@ -77,7 +78,7 @@ k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ Term
         }
         __syncthreads();
         for (uint64_t t = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; t < n; t += (uint64_t)gridDim.x * blockDim.x) {
-            double2 acc = out[t];
+            double2 acc = fresh && c0 == i0 ? make_double2(0.0, 0.0) : out[t];
             for (int q = 0; q < cn; ++q) {
                 const ItemTerm& term = terms[q];
                 if (!term.on) continue;
@@ -90,13 +91,14 @@ k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ Term
                 const uint64_t c = deposit(i, tm.runs, tm.nruns);
                 const double2 v = entry_f64(table[(uint64_t)(c0 + q) * table_stride + c]);
                 const double vr = v.x * term.p2, vi = v.y * term.p2;  // exact
-                // (roundings fixed: the draws' 53-bit distances depend on every bit of a block)
+                // (roundings fixed here and above: the draws' 53-bit distances depend on every bit of a block)
                 acc.x = __dadd_rn(acc.x, __fma_rn(vr, term.cr, -__dmul_rn(vi, term.ci)));
                 acc.y = __dadd_rn(acc.y, __fma_rn(vi, term.cr, __dmul_rn(vr, term.ci)));
             }
             out[t] = acc;
         }
-    }
+        c0 += kTerms;
+    } while (c0 < i1);
 }
 
 // ---------------------------------------------------------------- tail
@@ -296,8 +298,17 @@ extern "C" int dcs_accumulate_batched(int dtype, const void* table, uint64_t tab
                                       const uint64_t* xors, const double* coefs, const int32_t* item_begin,
                                       int nblocks, double log_shift, dcs_scale* scale, const uint64_t* maxbits_final,
                                       uint64_t mstride, double* total, int k, int nitems, void* stream) {
+    return dcs_accumulate_ex(dtype, table, table_stride, tr, terminal_runs, nruns, tbasis, xors, coefs, item_begin, nblocks,
+                             log_shift, scale, maxbits_final, mstride, total, k, nitems, 0u, stream);
+}
+
+extern "C" int dcs_accumulate_ex(int dtype, const void* table, uint64_t table_stride, int tr,
+                                 const uint32_t* terminal_runs, int nruns, const uint64_t* tbasis, const uint64_t* xors,
+                                 const double* coefs, const int32_t* item_begin, int nblocks, double log_shift,
+                                 dcs_scale* scale, const uint64_t* maxbits_final, uint64_t mstride, double* total, int k,
+                                 int nitems, unsigned flags, void* stream) {
     if (!table || !xors || !coefs || !item_begin || !scale || !maxbits_final || !total || nblocks < 1 ||
-        nblocks > 65535 || nitems < 0) {
+        nblocks > 65535 || nitems < 0 || (flags & ~(unsigned)DCS_ACCUMULATE_FRESH)) {
         dcs_host::set_error("dcs_accumulate: invalid arguments");
         return DCS_E_ARG;
     }
@@ -314,7 +325,7 @@ extern "C" int dcs_accumulate_batched(int dtype, const void* table, uint64_t tab
         return dcs_host::check_cuda(
             dcs_host::launch_after(kernel, grid, dim3(256), 0, st, t, table_stride, tm, xors, coefs, item_begin, log_shift, scale,
                                    (const unsigned long long*)maxbits_final, mstride, dtype == DCS_C128 ? 1 : 0,
-                                   (double2*)total),
+                                   (flags & DCS_ACCUMULATE_FRESH) ? 1 : 0, (double2*)total),
             "k_accumulate launch");
     };
     if (dtype == DCS_C64) return run(k_accumulate<float2>, (const float2*)table);

@@ -75,10 +75,15 @@ k_build_items(const __grid_constant__ BuildArgs B, const uint64_t* __restrict__ 
         const int q = B.xq[j];
         const int b = q >= 0 ? (int)((x >> q) & 1ull) : 0;
         const double* f = B.fsel + 8 * j + 4 * b;
-        const double sgn = B.flip[(uint64_t)l * B.nsteps + j] ? -1.0 : 1.0;
+        const int flip = B.flip[(uint64_t)l * B.nsteps + j];
+        const double sgn = (flip & 0x7f) ? -1.0 : 1.0;
         dcs_param p;
         p.f0r = f[0]; p.f0i = f[1];
         p.f1r = f[2] * sgn; p.f1i = f[3] * sgn;
+        if (flip & 0x80) {  // the product with sgn + 0 i, whose zeros have the signs of NumPy's complex product
+            p.f1r = __dsub_rn(p.f1r, __dmul_rn(f[3], 0.0));
+            p.f1i = __dadd_rn(__dmul_rn(f[2], 0.0), p.f1i);
+        }
         p.ov = 0;
         p.y = 0;
         const int a = B.fixidx[j];

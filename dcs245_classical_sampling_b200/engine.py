@@ -37,6 +37,7 @@ from . import _lib
 from .plan import (KIND_GROW, W_T, build_block_plan, deposit_runs, orbit_kind, slot_mask)
 
 LN2 = math.log(2.0)
+_SCALE_WORDS = _lib.SCALE_DTYPE.itemsize // 8
 
 # Fused plan of complex128 tables (plan-specialised kernels in FP64): 2^12-entry tiles of 16-byte
 # entries (64 KB of shared memory, two CTAs per SM), 3 contiguous low bits (128-byte rows),
@@ -259,6 +260,9 @@ class DeviceCircuit:
         self.xq = dev(xq)
         self.fixidx = dev(fixidx)
         self.flip = dev(np.stack(flips).astype(np.uint8))
+        # the same for items with the bits of the host bookkeeping: a zero's sign decides between a step
+        # factor's argument and one 2 pi away
+        self.flip_host = self.flip | 0x80
         self.F = dev(F)
         self.tail = dev(tail.view(np.int64))
         self.coef = dev(np.array([[c.real, c.imag] for c in coefs], np.float64).reshape(-1))
@@ -273,9 +277,10 @@ class DeviceCircuit:
             return None
         return cls(engine, engine.device) if engine.params.items(np.zeros(engine.n, np.uint8))[1] else None
 
-    def build(self, lib, xbits, nsamples, params, coefs, xors, stream):
+    def build(self, lib, xbits, nsamples, params, coefs, xors, stream, flip=None):
         _lib.check(lib.dcs_build_items(
-            _lib.ptr(self.fsel), _lib.ptr(self.xq), _lib.ptr(self.fixidx), _lib.ptr(self.flip), _lib.ptr(self.F),
+            _lib.ptr(self.fsel), _lib.ptr(self.xq), _lib.ptr(self.fixidx),
+            _lib.ptr(self.flip if flip is None else flip), _lib.ptr(self.F),
             _lib.ptr(self.tail), _lib.ptr(self.coef), _lib.ptr(self.freeflip), self.nsteps, self.nfixed,
             self.nslices, _lib.ptr(xbits), nsamples, _lib.ptr(params), _lib.ptr(coefs), _lib.ptr(xors), stream))
 
@@ -324,7 +329,7 @@ def device_batch(engine, masks):
     dev = torch.empty(o3 + B + words, dtype=torch.int64, device=engine.device)
     dev[o3:].copy_(pinned, non_blocking=True)
     params, coefs, xors = dev[:o1], dev[o1:o2].view(torch.float64), dev[o2:o3]
-    engine.dc.build(engine.lib, dev[o3:], B, params, coefs, xors, engine._stream())
+    engine.dc.build(engine.lib, dev[o3:], B, params, coefs, xors, engine._stream(), engine.dc.flip_host)
     return {"n_items": n, "chunks": chunks, "unit_ok": [True] * len(chunks),
             "counts": [1 << len(engine.plan.slices)] * B, "nblocks": B, "dev": dev, "pinned": pinned,
             "params": params, "coefs": coefs, "xors": xors, "begin": dev[o3 + B:].view(torch.int32),
@@ -748,20 +753,24 @@ class InplaceConditionalBlockGPU:
         nm = self._nmax() + 1
         entry = _lib.PARAM_DTYPE.itemsize
         launches = 0
-        out.zero_()
+        # one chunk that holds every block writes the blocks; several add to zeroed ones
+        chunks = prep["chunks"]
+        fresh = _lib.ACCUMULATE_FRESH if len(chunks) == 1 and chunks[0][2:4] == (0, prep["nblocks"]) else 0
+        if not fresh:
+            out.zero_()
         d_params, d_coefs, d_xors, d_begin = (_lib.ptr(prep[k]) for k in ("params", "coefs", "xors", "begin"))
-        for ci, (c0, cn, b0, nb, boff) in enumerate(prep["chunks"]):
+        for ci, (c0, cn, b0, nb, boff) in enumerate(chunks):
             self._reset_items(cn, st)
             ok = prep["unit_ok"][ci]
             self._run_steps(d_params + c0 * self.nsteps * entry, cn, ok, st)
             launches += (len(self.fplan.groups) if self.mode == "fused" else
                          self.tile_launches if self.tplan is not None and ok else self.nsteps)
-            _lib.check(lib.dcs_accumulate_batched(
+            _lib.check(lib.dcs_accumulate_ex(
                 self.dcode, _lib.ptr(self.table), self.table_stride, self.plan.terminal_rank,
                 self.term_runs.ctypes.data, self.term_nruns, self.tbasis.ctypes.data,
                 d_xors + 8 * c0, d_coefs + 16 * c0,
                 d_begin + 4 * boff, nb, self.params.shift, _lib.ptr(self.scale),
-                _lib.ptr(self.maxbits) + 8 * (nm - 1), nm, _lib.ptr(out) + (b0 << (self.k + 4)), self.k, cn, st))
+                _lib.ptr(self.maxbits) + 8 * (nm - 1), nm, _lib.ptr(out) + (b0 << (self.k + 4)), self.k, cn, fresh, st))
             launches += 2
             if flags is not None:
                 if flags.dtype != torch.int64 or not flags.is_cuda or not flags.is_contiguous() or flags.numel() < cn:
@@ -783,9 +792,14 @@ class InplaceConditionalBlockGPU:
     def _run(self, x_list, w=None, part=0, parts=1):
         prep = self.prepare(x_list, w, part, parts)
         out = torch.empty((len(x_list), 1 << self.k), dtype=torch.complex128, device=self.device)
-        flags = self._flags_tensor()
+        # one small device->host read per call: the scale records of a single chunk, or the collected flags
+        flags = None if len(prep["chunks"]) == 1 else self._flags_tensor()
         self.enqueue(prep, out, flags)
-        raise_for_flags(flags.cpu().numpy())  # one small device->host read per call
+        if flags is None:
+            cn = prep["chunks"][0][1]
+            raise_for_flags(self.scale[: cn * _SCALE_WORDS].cpu().numpy().view(_lib.SCALE_DTYPE)["flags"])
+        else:
+            raise_for_flags(flags.cpu().numpy())
         return out, prep
 
     def block(self, x_bits, w=None, part=0, parts=1):

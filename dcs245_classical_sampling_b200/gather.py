@@ -148,8 +148,10 @@ class ConditionalBlockGPU:
         start = time.perf_counter()
         count, chunks, keep = self._prepare(x_bits, w, part, parts)
         lib, st = self.lib, self._stream()
-        out = torch.zeros((1, 1 << self.k), dtype=torch.complex128, device=self.device)
-        flags = torch.zeros(self.items, dtype=torch.int64, device=self.device)
+        # a single chunk writes the block; several add to a zeroed one
+        fresh = _lib.ACCUMULATE_FRESH if len(chunks) == 1 else 0
+        out = (torch.empty if fresh else torch.zeros)((1, 1 << self.k), dtype=torch.complex128, device=self.device)
+        flags = None if fresh else torch.zeros(self.items, dtype=torch.int64, device=self.device)
         S = len(self.steps)
         final = self.tab[S & 1]  # step s reads table s % 2
         for cn, d_params, d_coefs, d_xors, d_begin in chunks:
@@ -159,14 +161,20 @@ class ConditionalBlockGPU:
             _lib.check(lib.dcs_gather_steps(self.dcode, _lib.ptr(self.tab[0]), _lib.ptr(self.tab[1]), self.stride,
                                             self.dsteps.ctypes.data, _lib.ptr(self.words), d_params, S, 0, S,
                                             _lib.ptr(self.maxbits), self.nm, _lib.ptr(self.scale), cn, st))
-            _lib.check(lib.dcs_accumulate_batched(
+            _lib.check(lib.dcs_accumulate_ex(
                 self.dcode, _lib.ptr(final), self.stride, self.terminal_rank, self.term_runs.ctypes.data,
                 self.term_nruns, self.tbasis.ctypes.data, d_xors, d_coefs, d_begin, 1, self.params.shift,
                 _lib.ptr(self.scale), _lib.ptr(self.maxbits) + 8 * (self.nm - 1), self.nm,
-                _lib.ptr(out.view(torch.float64)), self.k, cn, st))
-            _lib.check(lib.dcs_collect_flags(_lib.ptr(self.scale), _lib.ptr(flags), cn, st))
+                _lib.ptr(out), self.k, cn, fresh, st))
+            if flags is not None:
+                _lib.check(lib.dcs_collect_flags(_lib.ptr(self.scale), _lib.ptr(flags), cn, st))
         _lib.check(lib.dcs_block_tail(_lib.ptr(out), self.k, self.adj_hi.ctypes.data, self.u_open.ctypes.data, 1, st))
-        if np.any(flags.cpu().numpy() & 1):
+        if flags is None:
+            words = _lib.SCALE_DTYPE.itemsize // 8 * chunks[0][0]
+            seen = self.scale[:words].cpu().numpy().view(_lib.SCALE_DTYPE)["flags"]
+        else:
+            seen = flags.cpu().numpy()
+        if np.any(seen & 1):
             raise ArithmeticError("Nonfinite prefix table")
         meta = {"seconds": time.perf_counter() - start, "part": part, "parts": parts, "slices_evaluated": count,
                 "prefix_dtype": "complex128" if self.use_fp64 else "complex64", "rmax": self.rmax,

@@ -209,7 +209,9 @@ class CircuitRunner:
                                            _lib.ptr(self.d_x), _lib.ptr(self.d_u), st))
         self.dc.build(lib, self.d_x, n, self.d_params, self.d_coefs, self.d_xors, st)
         out = self.d_out[:n]
-        out.zero_()
+        fresh = _lib.ACCUMULATE_FRESH if len(chunks) == 1 else 0  # one chunk writes the blocks, several add to them
+        if not fresh:
+            out.zero_()
         entry = _lib.PARAM_DTYPE.itemsize
         nm = eng._nmax() + 1
         for c0, cn, b0, nb, boff in chunks:
@@ -217,12 +219,12 @@ class CircuitRunner:
             # (fused mode: weights that the generated kernels cannot take have switched them off)
             eng._run_steps(_lib.ptr(self.d_params) + c0 * eng.nsteps * entry, cn,
                            self.dc.unit_ok or self.mode == "fused")
-            _lib.check(lib.dcs_accumulate_batched(
+            _lib.check(lib.dcs_accumulate_ex(
                 eng.dcode, _lib.ptr(eng.table), eng.table_stride, eng.plan.terminal_rank,
                 eng.term_runs.ctypes.data, eng.term_nruns, eng.tbasis.ctypes.data,
                 _lib.ptr(self.d_xors) + 8 * c0, _lib.ptr(self.d_coefs) + 16 * c0,
                 _lib.ptr(self.d_begin) + 4 * boff, nb, eng.params.shift, _lib.ptr(eng.scale),
-                _lib.ptr(eng.maxbits[nm - 1:]), nm, _lib.ptr(out[b0:b0 + nb]), self.k, cn, st))
+                _lib.ptr(eng.maxbits[nm - 1:]), nm, _lib.ptr(out[b0:b0 + nb]), self.k, cn, fresh, st))
         _lib.check(lib.dcs_block_tail(_lib.ptr(out), self.k, eng.adj_hi.ctypes.data, eng.u_open.ctypes.data, n, st))
         _lib.check(lib.dcs_draw(_lib.ptr(out), self.k, n, _lib.ptr(self.d_u), _lib.ptr(self.d_scratch),
                                 _lib.ptr(self.d_res), st))

@@ -332,6 +332,15 @@ int dcs_accumulate_batched(int dtype, const void *table, uint64_t table_stride, 
                            double log_shift, dcs_scale *scale, const uint64_t *maxbits_final, uint64_t mstride,
                            double *total, int k, int nitems, void *stream);
 
+/* dcs_accumulate_batched with flags.  DCS_ACCUMULATE_FRESH: total need not be zeroed before (the blocks start
+ * at zero; every one of them is written). */
+#define DCS_ACCUMULATE_FRESH 1u
+int dcs_accumulate_ex(int dtype, const void *table, uint64_t table_stride, int tr, const uint32_t *terminal_runs,
+                      int nruns, const uint64_t *tbasis, const uint64_t *xors, const double *coefs,
+                      const int32_t *item_begin, int nblocks, double log_shift, dcs_scale *scale,
+                      const uint64_t *maxbits_final, uint64_t mstride, double *total, int k, int nitems,
+                      unsigned flags, void *stream);
+
 /* Block tail for nblocks consecutive blocks of 2^k complex128: Walsh-Hadamard over k bits,
  * multiply by (-1)^(sum over open edges of y_a y_b) (adj_hi[a] = mask of b > a adjacent to a),
  * then apply u_open[q] (2x2 complex, row-major re/im interleaved: 8 doubles per bit) on bit q.
@@ -385,7 +394,8 @@ void dcs_philox4x32_10_host(uint32_t ctr[4], uint32_t key0, uint32_t key1);
  * the reference's host bookkeeping (conditional_block_gpu.py:136-157, inplace_gpu.py:111-114).
  * Static per-circuit tables (device): fsel (8 doubles per step: f for x bit 0, f for x bit 1),
  * xq (data qubit selecting the row, -1 for references), fixidx (index among fixed steps or -1),
- * flip (nslices x nsteps bytes), F (nfixed x ceil(nsteps/32) words: later-neighbour masks of
+ * flip (nslices x nsteps bytes: the second weight changes its sign where bits 0-6 are not all zero; bit 7: its
+ * zeros get the signs that a complex product with +-1 gives them, as in the host bookkeeping), F (nfixed x ceil(nsteps/32) words: later-neighbour masks of
  * fixed steps), tail (nfixed terminal-offset xors), coef (2 doubles per slice), freeflip (per
  * slice).  Output item i = sample * nslices + slice: params[i * nsteps + j], coefs[2i..2i+1],
  * xors[i]. */

@@ -6,17 +6,28 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 
+def _workload(name):
+    from dcs245_classical_sampling_b200.workloads import build_workload, choose_reference_slices, sweep_order
+    if isinstance(name, str):
+        return build_workload(name)
+    from dcs245_classical_sampling_b200.circuits import build_ring_instance  # weights with negative zeros
+    inst, opened = build_ring_instance(33, 40, 120, 947276), list(range(23, 33))
+    order = sweep_order(inst, opened)
+    ops = choose_reference_slices(inst["graph"], 33, order, 1, opened)
+    return {"graph": inst["graph"], "unitaries": inst["unitaries"], "n": 33, "order": order,
+            "parity_operations": [list(op) for op in ops], "open_vertices": opened}
+
+
 def _engine(name="ring24_d24_t60_k10", items=3, **kw):
     from dcs245_classical_sampling_b200.engine import InplaceConditionalBlockGPU
-    from dcs245_classical_sampling_b200.workloads import build_workload
-    w = build_workload(name)
+    w = _workload(name)
     eng = InplaceConditionalBlockGPU(w["graph"], w["unitaries"], w["n"], w["order"], w["parity_operations"],
                                      w["open_vertices"])
     eng.alloc(items=items, **kw)
     return eng
 
 
-@pytest.mark.parametrize("name", ["ring16_d20_t24_k8", "ring24_d24_t60_k10", "ring32_d37_t79_k14"])
+@pytest.mark.parametrize("name", ["ring16_d20_t24_k8", "ring24_d24_t60_k10", "ring32_d37_t79_k14", "ring40_d45_t190_k16", 33])
 @pytest.mark.parametrize("count,items", [(1, 1), (1, 8), (5, 3), (7, 4), (64, 256)])
 def test_items_equal_the_hosts(name, count, items):
     from dcs245_classical_sampling_b200 import _lib
@@ -31,7 +42,7 @@ def test_items_equal_the_hosts(name, count, items):
     assert (got["n_items"], got["nblocks"]) == (want["n_items"], want["nblocks"])
     a, b = (p["params"].cpu().numpy().view(_lib.PARAM_DTYPE) for p in (got, want))
     for f in _lib.PARAM_DTYPE.names:
-        assert np.array_equal(a[f], b[f]), f
+        assert a[f].tobytes() == b[f].tobytes(), f  # the signs of zeros, too
     for key in ("coefs", "xors"):
         assert np.array_equal(got[key].cpu().numpy(), want[key].cpu().numpy())
     n = sum(1 + c[3] for c in want["chunks"])
