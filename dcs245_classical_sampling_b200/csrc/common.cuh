@@ -112,9 +112,19 @@ __device__ __forceinline__ int scale_exponent(double m2) {
 // [2^floor(E/2), 2^(floor(E/2)+1)).  For m2 whose square root is not within half an ulp of a power of two from
 // below, as every float and every double with 32 zero low bits; subnormal m2 take the general way.
 __device__ __forceinline__ int scale_exponent_fast(double m2) {
+    if (!(m2 > 0.0)) return 0;
     const int h = __double2hiint(m2) >> 20;  // m2 >= 0
     if (h == 0 || h == 0x7ff) return scale_exponent(m2);
     return ((h - 1023) >> 1) + 1;
+}
+
+// e of a maximum whose running type is Q, and 2^-e: maxima of floats take the short way (the long one, a square root
+// in FP64 and library calls ahead of every step, is 1% of a 40-qubit block and 1.5% of a 48-qubit one)
+template <class Q> __device__ __forceinline__ int exponent_of_max(double m2) {
+    return sizeof(Q) == 4 ? scale_exponent_fast(m2) : scale_exponent(m2);
+}
+__device__ __forceinline__ double exp2_neg(int e) {  // 2^-e, |e| < 1000
+    return __hiloint2double((1023 - e) << 20, 0);
 }
 
 // block-wide max of an unsigned 64-bit value; result valid in thread 0

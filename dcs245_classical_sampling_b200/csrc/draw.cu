@@ -860,7 +860,7 @@ extern "C" int dcs_overlap(const double* ref, const double* ap, uint64_t len, do
 // in a file-scope device array of fixed size, so this entry point allocates nothing.
 //
 // Limit: one block of up to 2^20 amplitudes per call (DCS_DRAW_STATIC_MAX_K); every GPU that
-// loads the library holds the array (about 8.4 MiB) until the process exits.
+// loads the library holds the array (about 8.3 MiB) until the process exits.
 namespace {
 constexpr size_t kStaticDrawBytes = layout(DCS_DRAW_STATIC_MAX_K, 1).bytes;
 static __device__ __align__(256) unsigned char g_draw_scratch[kStaticDrawBytes];

@@ -66,8 +66,8 @@ k_gather(const S* Ein, S* Eout, uint64_t stride, const __grid_constant__ dcs_gat
     const dcs_param p = params[(uint64_t)item * param_stride + s];
     unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
     const double m2prev = (double)bits_to_m2<R>(mb[s]);
-    const int e = scale_exponent(m2prev);
-    const double sc = ldexp(1.0, -e);
+    const int e = exponent_of_max<R>(m2prev);
+    const double sc = exp2_neg(e);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         dcs_scale* sp = scale + item;
         sp->logscale += (double)e * 0.69314718055994530942;
@@ -147,7 +147,7 @@ k_gather_small(const S* Ein, S* Eout, uint64_t stride, const __grid_constant__ G
         if (i + 1 < G.count) fetch(i + 1);
         const dcs_param p = prm[i];
         const int e = scale_exponent_fast(m2);
-        const double sc = __hiloint2double((1023 - e) << 20, 0);  // 2^-e
+        const double sc = exp2_neg(e);
         rec.logscale += (double)e * 0.69314718055994530942;
         rec.exponent_sum += e;
         if (!isfinite(m2)) rec.flags |= 1u;

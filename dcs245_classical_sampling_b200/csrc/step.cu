@@ -64,8 +64,8 @@ k_step(M* __restrict__ table, uint64_t table_stride, const __grid_constant__ dcs
     const dcs_param p = params[(uint64_t)item * param_stride + s];
     unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
     const double m2prev = (double)bits_to_m2<R>(mb[s]);
-    const int e = scale_exponent(m2prev);
-    const R sc = (R)ldexp(1.0, -e);
+    const int e = exponent_of_max<Q>(m2prev);  // |e| <= 513
+    const R sc = (R)exp2_neg(e);
     if (blockIdx.x == 0 && threadIdx.x == 0) {
         dcs_scale* sp = scale + item;
         sp->logscale += (double)e * 0.69314718055994530942;  // ln 2, as the reference's e*log(2.)

@@ -174,7 +174,7 @@ __device__ __forceinline__ int add_exponents(const unsigned long long* mb, int l
     const int lane = threadIdx.x & 31;
     double m2 = 1.0;
     if (lane < n) m2 = (double)bits_to_m2<R>(__ldcg(mb + lo + lane));
-    const int x = scale_exponent(m2);
+    const int x = exponent_of_max<R>(m2);
     int e = x - __shfl_up_sync(0xffffffffu, x, 1);
     if (lane == 0) e = x;
     const unsigned bad = __ballot_sync(0xffffffffu, !isfinite(m2)), zero = __ballot_sync(0xffffffffu, m2 == 0.0);
@@ -237,7 +237,7 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     let_next_start();
     fill_tables<NT, kMaxDim, SH>(A, tab, hi_tab);
     after_previous();  // the tables above are the plan's
-    const int e = scale_exponent((double)bits_to_m2<R>(mb[A.first]));
+    const int e = exponent_of_max<R>((double)bits_to_m2<R>(mb[A.first]));
     if (blockIdx.x == 0 && threadIdx.x < 32) {
         const int lo = kStepMax<S> ? A.prev_first + 1 : A.first;
         add_exponents<R>(mb, lo, A.first - lo + 1, scale + item);
@@ -245,7 +245,7 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     if (threadIdx.x < A.count) {
         const dcs_param p = params[(uint64_t)item * param_stride + A.first + threadIdx.x];
         // the pass's power of two goes into the first step's weights (exact)
-        const R sc = threadIdx.x ? (R)1 : (R)ldexp(1.0, -e);
+        const R sc = threadIdx.x ? (R)1 : (R)exp2_neg(e);
         Weights<S> w;
         w.f0 = cscale(Store<S>::make((R)p.f0r, (R)p.f0i), sc);
         w.f1 = cscale(Store<S>::make((R)p.f1r, (R)p.f1i), sc);
@@ -394,12 +394,12 @@ k_tile_half(ushort2* __restrict__ table, uint64_t table_stride, const __grid_con
     for (int s = 0; s < A.count; ++s) {
         const TileStep& st = A.st[s];
         const dcs_param p = prm[s];
-        const int e = scale_exponent(m2);
+        const int e = exponent_of_max<float>(m2);
         sc.logscale += (double)e * 0.69314718055994530942;  // ln 2, as the reference's e*log(2.)
         sc.exponent_sum += e;
         if (!isfinite(m2)) sc.flags |= 1u;
         else if (m2 == 0.0) sc.flags |= 2u;
-        const double f = ldexp(1.0, -e);
+        const double f = exp2_neg(e);
         Weights<double2> w;
         w.f0 = cscale(make_double2(p.f0r, p.f0i), f);
         w.f1 = cscale(make_double2(p.f1r, p.f1i), f);

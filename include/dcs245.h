@@ -369,7 +369,7 @@ int dcs_draw_ex(const double *blocks, int k, int nblocks, const double *uniforms
  * For callers that cannot allocate device memory where they sample: code running while a
  * stream is captured, host runtimes that lend the library only their own buffers, loops where
  * an allocation would synchronise the device.  Same computation and result as dcs_draw for
- * one block, with the scratch in a fixed device array inside the library (about 8.4 MiB per
+ * one block, with the scratch in a fixed device array inside the library (about 8.3 MiB per
  * GPU that loads the library, held until the process exits).  Limit: one block of at most
  * 2^DCS_DRAW_STATIC_MAX_K amplitudes per call; larger blocks are rejected with DCS_E_ARG.
  * The first call on each device looks the array up (cudaGetSymbolAddress) with that device
