@@ -353,6 +353,8 @@ class DeviceBlock(torch.Tensor):
 class InplaceConditionalBlockGPU:
     """Drop-in for the reference engine of the same name (see module docstring)."""
 
+    half = False  # binary16 tables (alloc)
+
     def __init__(self, graph, unitaries, n, order, parity_operations, open_vertices):
         self.plan = plan = build_block_plan(graph, unitaries, n, order, parity_operations, open_vertices)
         # reference attribute surface (conditional_block_gpu.py:25-69)
