@@ -354,6 +354,12 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     if (threadIdx.x == 0) sp->table_exp = rest;
 }
 
+// Bytes of a binary16 tile, with its end where 8-byte words can follow (a plan that starts with fixed or isolated
+// vertices has tiles of one 4-byte entry).
+__host__ __device__ constexpr size_t half_tile_bytes(int tile_dim) {
+    return tile_dim ? sizeof(ushort2) << tile_dim : sizeof(uint64_t);
+}
+
 // A group whose table is one tile, on binary16 tables with FP64 arithmetic (the half-storage tier): one CTA
 // per item.  Every step rounds what it stores, scaled by the exponent of the maximum before it, so the
 // scale is taken step by step here, too; the CTA holds the whole table, so its maximum is at hand.
@@ -370,7 +376,7 @@ k_tile_half(ushort2* __restrict__ table, uint64_t table_stride, const __grid_con
     const int item = blockIdx.y;
     const int T = 1 << A.tile_dim;
     const int low = A.low_bits;
-    uint64_t* hi_tab = reinterpret_cast<uint64_t*>(smem + ((size_t)T << 2));
+    uint64_t* hi_tab = reinterpret_cast<uint64_t*>(smem + half_tile_bytes(A.tile_dim));
     ushort2* E = table + (uint64_t)item * table_stride;
     unsigned long long* mb = maxbits + (uint64_t)item * maxbits_stride;
     let_next_start();
@@ -570,7 +576,7 @@ int run_half_groups(ushort2* table, uint64_t table_stride, const dcs_step* steps
                 dcs_host::set_error("dcs_tile_groups: malformed group %d", gi);
                 return DCS_E_ARG;
             }
-            const size_t smem = sizeof(ushort2) * ((size_t)1 << A.tile_dim) + sizeof(uint64_t) * ((size_t)1 << (A.tile_dim - A.low_bits));
+            const size_t smem = half_tile_bytes(A.tile_dim) + sizeof(uint64_t) * ((size_t)1 << (A.tile_dim - A.low_bits));
             rc = dcs_host::check_cuda(
                 dcs_host::launch_after(k_tile_half<NT>, dim3(1, (unsigned)nitems), dim3(NT), smem, st, table, table_stride, A,
                                        params, param_stride, (unsigned long long*)maxbits, mstride, scale),

@@ -1,0 +1,50 @@
+"""Tile groups at the edges of their range: tiles of one entry, tables whose maximum leaves the range of its
+square in storage precision, step weights at the ends of what they take, single steps where they cannot run."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+def _engine(graph, unitaries, n, order, opened, dtype=np.complex64, **kw):
+    from dcs245_classical_sampling_b200.engine import InplaceConditionalBlockGPU
+    eng = InplaceConditionalBlockGPU(np.asarray(graph, np.uint8), np.asarray(unitaries, complex), n, order, [], opened)
+    eng.alloc(dtype, mode="device", **kw)
+    return eng
+
+
+def _random_case(seed, p):
+    """A random graph state with Clifford-like and diagonal frames: tiles of one entry where `p` is small."""
+    rng = np.random.default_rng(seed)
+    n = int(rng.integers(2, 10))
+    N = n + int(rng.integers(0, 10))
+    A = np.triu(rng.random((N, N)) < p, 1).astype(np.uint8)
+    U = [np.eye(2) if rng.random() < 0.3 else np.linalg.qr(rng.standard_normal((2, 2)) + 1j * rng.standard_normal((2, 2)))[0]
+         for _ in range(N)]
+    opened = sorted(rng.choice(n, int(rng.integers(0, n)), replace=False).tolist())
+    order = [int(v) for v in rng.permutation(N) if v not in opened] + opened
+    return (A + A.T, np.stack(U).astype(complex), n, order, opened), rng.integers(0, 2, n).astype(np.uint8)
+
+
+@pytest.mark.parametrize("storage", [None, "float16"])
+@pytest.mark.parametrize("p", [0.0, 0.1, 0.3])
+def test_small_tiles(p, storage):
+    """Tables of one, two and a few entries (a group of isolated or fixed vertices has tiles of one): the bits of
+    one launch per step, and in complex64 the oracle's block."""
+    from oracle.block_ref import OracleEngine
+    one_entry = 0
+    for seed in range(12):
+        (A, U, n, order, opened), x = _random_case(seed, p)
+        eng = _engine(A, U, n, order, opened, storage=storage)
+        one_entry += sum(int(g["tile_dim"]) == 0 for g in eng.tplan.groups)
+        got = eng.block(x)[0].cpu().numpy()
+        eng.tplan = None
+        assert np.array_equal(got, eng.block(x)[0].cpu().numpy()), seed
+        if storage:
+            continue
+        want, _ = OracleEngine(A, U, n, order, [], opened).block(x)
+        # a step rounds weights, products and sums (5 roundings of 2^-24 of the largest entry that it can have, a
+        # factor |f0| + |f1| <= sqrt 2 (data rows) or 2 (bras) per step, less the block's factor 2^(-1/2) per bra)
+        largest = 2.0 ** ((len(A) - len(opened)) / 2)
+        assert np.abs(got - want).max() <= 5 * 2.0 ** -24 * eng.nsteps * largest, seed
+    assert one_entry or p
