@@ -599,6 +599,13 @@ extern "C" int dcs_tile_groups(int dtype, void* table, uint64_t table_stride, co
         dcs_host::set_error("dcs_tile_groups: invalid arguments");
         return DCS_E_ARG;
     }
+    // rows of complex64 entries move in 16-byte words
+    const bool aligned = ((uintptr_t)table & 15) == 0 && (nitems == 1 || !(table_stride & 1));
+    for (int gi = 0; gi < ngroups && dtype == DCS_C64 && !aligned; ++gi)
+        if (groups[gi].low_bits >= 1) {
+            dcs_host::set_error("dcs_tile_groups: complex64 tables must be 16-byte aligned (an even table_stride)");
+            return DCS_E_ARG;
+        }
     if (dtype == DCS_H16)
         return run_half_groups((ushort2*)table, table_stride, steps, nsteps, groups, ngroups, tile_steps, params,
                                param_stride, maxbits, scale, nitems, (cudaStream_t)stream);

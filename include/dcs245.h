@@ -293,7 +293,8 @@ int dcs_fused_runs(void *table, const dcs_step *steps, int nsteps, const dcs_gro
  * a complex64 table still has is in table_exp.  DCS_H16: groups of one tile (2^13 entries at most) run
  * in one launch with every step's own renormalisation, the others a launch per step; maxbits_stride is
  * nsteps + 1.  Steps 0 .. nsteps - 1
- * in groups that follow one another; steps, groups, tile_steps: host arrays. */
+ * in groups that follow one another; steps, groups, tile_steps: host arrays.  Complex64 tables whose groups have
+ * low_bits >= 1 are 16-byte aligned, with an even table_stride for more than one item (else DCS_E_ARG). */
 int dcs_tile_groups(int dtype, void *table, uint64_t table_stride, const dcs_step *steps, int nsteps,
                     const dcs_group *groups, int ngroups, const dcs_tile_step *tile_steps, const dcs_param *params,
                     uint64_t param_stride, uint64_t *maxbits, uint64_t maxbits_stride, dcs_scale *scale, int nitems,
