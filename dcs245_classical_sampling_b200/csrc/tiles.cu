@@ -23,8 +23,9 @@
 // have goes into table_exp: a block has the bits of the per-step executor's (13% of a group's time), and
 // so have the draws and the 53-bit distances that depend on every bit of it.  In complex128 a group takes one
 // maximum (per-step ones cost 18%); the logscale then is a shorter sum of the same numbers, and the block
-// differs from the per-step executor's in that factor's rounding only.  The host keeps
-// step weights out of here whose size could overflow or underflow a group (engine.tile_weights_ok).
+// differs from the per-step executor's in that factor's rounding only.  The host keeps step weights out of
+// here that could let a group's entries, or in complex64 their squares, overflow (engine.tile_weights_ok,
+// tile_growth_ok).
 #include <string.h>
 
 #include "common.cuh"

@@ -51,9 +51,13 @@ FP64_FALLBACK_CONFIGS = ({"low": 4, "grouping": "greedy"}, {"variant": 4}, {"var
 
 TILE_STEPS = 24  # steps of a tile group: the most that one launch takes
 # Step weights that a tile group may run without a renormalisation inside: the larger weight of a free
-# step (the selected one of a fixed step) in [2^-3, 2^2].  A step then grows the largest entry by 2^4
-# at most, 24 of them by 2^96, inside the FP32 range.
+# step (the selected one of a fixed step) in [2^-3, 2^2].
 TILE_WEIGHT_RANGE = (0.125, 4.0)
+# A group starts with entries below 1.  complex64 takes every step's maximum as |x|^2 in FP32, which
+# overflows from |x| = 2^64 on, so the steps of a group may let entries grow by 2^63 together
+# (step_growth).  Bras and frames of unitary matrices have |f0| + |f1| <= 2 and reach 2^48 at most.  (In FP64
+# the range above holds 24 steps to 2^96, whose square is far inside.)
+TILE_GROWTH_LOG2 = 63
 
 
 HALF_TILE_DIM = 13  # log2 of the largest binary16 table that one tile holds
@@ -253,7 +257,7 @@ class DeviceCircuit:
             rows["f0r"][b::2], rows["f0i"][b::2] = fsel[:, 4 * b], fsel[:, 4 * b + 1]
             rows["f1r"][b::2], rows["f1i"][b::2] = fsel[:, 4 * b + 2], fsel[:, 4 * b + 3]
         rows["y"] = np.hypot(rows["f0r"], rows["f0i"]) <= 1e-12  # the value that a fixed step's row selects
-        self.unit_ok = all(engine.weights_ok(rows[b::2]) for b in (0, 1))
+        self.unit_ok = engine.weights_ok(rows.reshape(S, 2).T, any_row=True)
         self.nsteps, self.nfixed = S, nfixed
         dev = lambda a: torch.from_numpy(np.ascontiguousarray(a)).to(device)
         self.fsel = dev(fsel)
@@ -682,13 +686,15 @@ class InplaceConditionalBlockGPU:
                 "pinned": pinned, "params": dev[:o1], "coefs": dev[o1:o2].view(torch.float64),
                 "xors": dev[o2:o3], "begin": dev[o3:].to(torch.int32), "h2d_bytes": blob.nbytes}
 
-    def weights_ok(self, params):
-        """Whether an item's step weights can run the kernels of several steps per launch of this mode
-        (generated kernels, tile groups); else its batch runs the library kernels / single steps."""
+    def weights_ok(self, params, any_row=False):
+        """Whether an item's step weights (or several items', the plan's steps on the last axis) can run the
+        kernels of several steps per launch of this mode (generated kernels, tile groups); else its batch
+        runs the library kernels / single steps.  any_row: an item takes each step's weights from any row."""
         if self.mode == "fused":
             return self.unit_weights_ok(params)
-        # (binary16 tables renormalise after every step in both forms)
-        return self.tile_weights_ok(params) if self.tplan is not None and not self.half else True
+        if self.tplan is None or self.half:  # (binary16 tables renormalise after every step in both forms)
+            return True
+        return self.tile_weights_ok(params) and (self.use_fp64 or self.tile_growth_ok(params, any_row))
 
     def tile_weights_ok(self, params):
         """Whether step weights (dcs_param arrays, the plan's steps on the last axis) stay inside
@@ -698,11 +704,27 @@ class InplaceConditionalBlockGPU:
         big = np.where(self.free_steps, np.maximum(a0, a1), np.where(params["y"] != 0, a1, a0))
         return bool(np.all((big >= TILE_WEIGHT_RANGE[0]) & (big <= TILE_WEIGHT_RANGE[1])))
 
+    def step_growth(self, params):
+        """Bound of the factor by which each step can enlarge the largest |entry|."""
+        a0 = np.hypot(params["f0r"], params["f0i"])
+        a1 = np.hypot(params["f1r"], params["f1i"])
+        big, both, sel = np.maximum(a0, a1), a0 + a1, np.where(params["y"] != 0, a1, a0)
+        # by kind: grow, mix, diag, replace, fixed, fixed shrink, four- and two-entry shrink
+        return np.choose(self.dsteps["kind"], [big, both, both, 2 * big, sel, 2 * sel, 2 * both, 2 * both])
+
+    def tile_growth_ok(self, params, any_row=False):
+        """Whether no group of the tile plan can let an entry grow by more than 2^TILE_GROWTH_LOG2."""
+        lg = np.log2(self.step_growth(params))
+        if any_row:
+            lg = lg.max(axis=0)
+        return all(bool(np.all(lg[..., g["first"]:g["first"] + g["count"]].sum(axis=-1) <= TILE_GROWTH_LOG2))
+                   for g in self.tplan.groups)
+
     def unit_weights_ok(self, params):
         """Whether an item's step weights (a dcs_param array) can run the plan-specialised kernels,
         which divide f0 out of every free step: f0 != 0 there, and |f1 / f0| <= 2^32 so that a
         group of steps stays inside the FP32 range between renormalisations."""
-        p = params[self.free_steps]
+        p = params[..., self.free_steps]
         a0 = np.hypot(p["f0r"], p["f0i"])
         return bool(np.all(a0 > 0) and np.all(np.hypot(p["f1r"], p["f1i"]) <= 2.0 ** 32 * a0))
 

@@ -107,7 +107,7 @@ class ConditionalBlockGPU:
         self.dc = DeviceCircuit.of(self)
         self._alloc = True
 
-    def weights_ok(self, params):
+    def weights_ok(self, params, any_row=False):
         """Every step weight runs the gather kernel."""
         return True
 

@@ -289,7 +289,8 @@ int dcs_fused_runs(void *table, const dcs_step *steps, int nsteps, const dcs_gro
  * [0, ngroups) in order, tiles of at most 2^12 entries.  Item i uses table + i*table_stride entries,
  * params + i*param_stride, maxbits + i*maxbits_stride (word s + 1 receives the max of step s, for
  * complex128 of a group's last step s only; word 0 holds the bits of 1.0) and scale + i (all zero on entry).  The table is renormalised once per group, so
- * the weights of a group must not overflow or underflow the storage precision; the power of two that
+ * the weights of a group must not let an entry leave the storage precision's range, nor in complex64 |entry|^2 that
+ * of FP32 (entries below 2^63); the power of two that
  * a complex64 table still has is in table_exp.  DCS_H16: groups of one tile (2^13 entries at most) run
  * in one launch with every step's own renormalisation, the others a launch per step; maxbits_stride is
  * nsteps + 1.  Steps 0 .. nsteps - 1

@@ -48,3 +48,24 @@ def test_small_tiles(p, storage):
         largest = 2.0 ** ((len(A) - len(opened)) / 2)
         assert np.abs(got - want).max() <= 5 * 2.0 ** -24 * eng.nsteps * largest, seed
     assert one_entry or p
+
+
+def _star(leaves):
+    """Reference vertices on one open vertex: a growing step, then diagonal ones, which multiply an entry by f0 + f1."""
+    A = np.zeros((1 + leaves, 1 + leaves), np.uint8)
+    A[0, 1:] = A[1:, 0] = 1
+    return A, np.stack([np.eye(2, dtype=complex)] * (1 + leaves)), 1, list(range(1, 1 + leaves)) + [0], [0]
+
+
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+@pytest.mark.parametrize("leaves", [5, 24, 30, 60])
+@pytest.mark.parametrize("weight", [0.125, 3.0, 4.0])
+def test_weights_at_the_ends_of_the_range(weight, leaves, dtype):
+    """Entries grow by up to 8 a step (2^72 in a group of 24): squares past the FP32 range, the block is right."""
+    from oracle.block_ref import OracleEngine
+    args, x, w = _star(leaves), np.zeros(1, np.uint8), np.array([weight, weight])
+    eng = _engine(*args, dtype=dtype)
+    assert all(eng.prepare([x], w)["unit_ok"]) == (dtype == np.complex128 or weight < 3.1 or leaves < 24)
+    want, _ = OracleEngine(*args[:4], [], args[4]).block(x, w)
+    got = eng.block(x, w)[0].cpu().numpy()
+    assert np.linalg.norm(got - want) <= 4 * leaves * 2.0 ** -24 * np.linalg.norm(want)
