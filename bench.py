@@ -333,13 +333,14 @@ def gpu_arm(args):
     res = torch.empty((total, _lib.DRAW_DTYPE.itemsize), dtype=torch.uint8, device=dev)
     lib = _lib.load()
     scratch = torch.empty(lib.dcs_draw_scratch_bytes(k, 1), dtype=torch.uint8, device=dev)
+    flags = device_flags(eng)
     torch.cuda.synchronize(dev)
 
     def one(i, record=False):
         ev0 = torch.cuda.Event(enable_timing=True) if record else None
         if record:
             ev0.record(stream)
-        launches = eng.enqueue(preps[i], outs[i:i + 1])
+        launches = eng.enqueue(preps[i], outs[i:i + 1], flags)
         _lib.check(lib.dcs_draw(_lib.ptr(outs[i]), k, 1, _lib.ptr(d_us[i:i + 1]), _lib.ptr(scratch),
                                 _lib.ptr(res[i]), stream.cuda_stream))
         ev1 = None
@@ -372,6 +373,7 @@ def gpu_arm(args):
         t = torch.tensor([elapsed], device=dev)
         torch.distributed.all_reduce(t, op=torch.distributed.ReduceOp.MAX)
         elapsed = float(t.item())
+    check_flags(eng, preps[0], flags)
     lat = sorted(a.elapsed_time(b) for a, b in lat_events)
     draws = res.cpu().numpy().view(_lib.DRAW_DTYPE).reshape(-1)
     value = args.steps * world / elapsed
@@ -582,6 +584,21 @@ def run_audit(args, a64, local):
             "rows": rows}
 
 
+def device_flags(eng):
+    """The scale flags that device mode's tile groups report through (None in the other modes)."""
+    import torch
+    return torch.zeros(eng.items, dtype=torch.int64, device=eng.device) if eng.tplan is not None else None
+
+
+def check_flags(eng, prep, flags):
+    from dcs245_classical_sampling_b200.engine import raise_for_flags
+    if flags is not None:
+        seen = flags.cpu().numpy()
+        raise_for_flags(seen)
+        if eng.out_of_range(prep, seen):
+            raise RuntimeError("a timed sample left the range of the tile groups")
+
+
 def gpu_small_configs(args, local):
     """The small workloads measured completely on the GPU: device-resident samples/s (inputs
     prepared and uploaded first), end to end through sampling.sample_checked, and c_y of a few
@@ -613,18 +630,20 @@ def gpu_small_configs(args, local):
         res = torch.empty((len(xs), _lib.DRAW_DTYPE.itemsize), dtype=torch.uint8, device=dev)
         lib = _lib.load()
         scratch = torch.empty(lib.dcs_draw_scratch_bytes(k, 1), dtype=torch.uint8, device=dev)
+        flags = device_flags(eng)
         for i in range(min(3, len(xs))):
-            eng.enqueue(preps[i], outs[i:i + 1])
+            eng.enqueue(preps[i], outs[i:i + 1], flags)
         torch.cuda.synchronize(dev)
         a = torch.cuda.Event(enable_timing=True)
         b = torch.cuda.Event(enable_timing=True)
         a.record(stream)
         for i in range(len(xs)):
-            eng.enqueue(preps[i], outs[i:i + 1])
+            eng.enqueue(preps[i], outs[i:i + 1], flags)
             _lib.check(lib.dcs_draw(_lib.ptr(outs[i]), k, 1, _lib.ptr(d_us[i:i + 1]), _lib.ptr(scratch),
                                     _lib.ptr(res[i]), stream.cuda_stream))
         b.record(stream)
         torch.cuda.synchronize(dev)
+        check_flags(eng, preps[0], flags)
         value = len(xs) / (a.elapsed_time(b) / 1000.0)
         sample_checked(eng, xs[:3], us[:3], hashes=True, exact_cdf=True)
         torch.cuda.synchronize(dev)

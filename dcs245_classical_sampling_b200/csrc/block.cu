@@ -60,7 +60,10 @@ k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ Term
             t.on = !(sc.flags & 3u) && mf != 0 && isfinite(m2);
             // the reference checks every step's max, including the last (every other reader of the flags in
             // this launch takes the maximum itself)
-            if (blockIdx.x == 0 && !isfinite(m2)) scale[it].flags = sc.flags | 1u;
+            if (blockIdx.x == 0) {
+                if (!isfinite(m2)) scale[it].flags = sc.flags | 1u;
+                else if (m2 > 0.0 && m2 < (is64 ? kLeastMax<double> : kLeastMax<float>)) scale[it].flags = sc.flags | kFlagRange;
+            }
             const double m = exp(sc.logscale - log_shift);
             double cr = coefs[2 * it] * m, ci = coefs[2 * it + 1] * m;
             if (sc.phase != 0.0) {  // step factors divided out by the plan-specialised kernels

@@ -127,6 +127,11 @@ __device__ __forceinline__ double exp2_neg(int e) {  // 2^-e, |e| < 1000
     return __hiloint2double((1023 - e) << 20, 0);
 }
 
+// |x|^2 of a table's largest entry below this has lost bits, or all of them (its exponent, and whether the table is
+// zero, are then not known): the least normal number of the maximum's type.
+template <class R> constexpr double kLeastMax = sizeof(R) == 4 ? 0x1p-126 : 0x1p-1022;
+constexpr uint32_t kFlagRange = 8u;  // dcs_scale.flags: such a maximum was seen
+
 // block-wide max of an unsigned 64-bit value; result valid in thread 0
 __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v) {
     __shared__ unsigned long long red[32];

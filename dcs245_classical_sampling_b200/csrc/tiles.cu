@@ -23,7 +23,9 @@
 // have goes into table_exp: a block has the bits of the per-step executor's (13% of a group's time), and
 // so have the draws and the 53-bit distances that depend on every bit of it.  In complex128 a group takes one
 // maximum (per-step ones cost 18%); the logscale then is a shorter sum of the same numbers, and the block
-// differs from the per-step executor's in that factor's rounding only.  The host keeps step weights out of
+// differs from the per-step executor's in that factor's rounding only.  Cancellation in a group can take the
+// squares of a table that is not zero below their type's range: that sets kFlagRange, and the host runs the batch
+// again with a launch per step.  The host keeps step weights out of
 // here that could let a group's entries, or in complex64 their squares, overflow (engine.tile_weights_ok,
 // tile_growth_ok).
 #include <string.h>
@@ -91,6 +93,11 @@ __device__ __forceinline__ double sign_of(uint32_t x, double) { return __hiloint
 __device__ __forceinline__ float flip1(float a, uint32_t m) { return __uint_as_float(__float_as_uint(a) ^ m); }
 __device__ __forceinline__ double flip1(double a, uint32_t m) {
     return __hiloint2double(__double2hiint(a) ^ (int)m, __double2loint(a));
+}
+// zero only for +-0
+__device__ __forceinline__ uint32_t nonzero_bits(float2 v) { return (__float_as_uint(v.x) | __float_as_uint(v.y)) & ~kSign; }
+__device__ __forceinline__ uint32_t nonzero_bits(double2 v) {
+    return ((uint32_t)(__double2hiint(v.x) | __double2hiint(v.y)) & ~kSign) | (uint32_t)(__double2loint(v.x) | __double2loint(v.y));
 }
 template <class S> __device__ __forceinline__ S flip(S a, uint32_t m) { return c2(flip1(a.x, m), flip1(a.y, m)); }
 
@@ -168,17 +175,24 @@ __device__ __forceinline__ typename Mem<S, M>::Q run_step(unsigned char* __restr
     return lm;
 }
 
-// Adds the exponents of steps lo .. lo + n - 1 to the item's scale (one warp, n <= 32): word t is the
-// maximum before step t, in one scale for all of them, in which the word before lo is 1.
+// Adds the exponents of steps lo .. lo + n - 1 to the item's scale (one warp, n <= look <= 32): word t is the
+// maximum before step t, in one scale for all of them, in which the word before lo is 1.  Words lo .. lo + look - 1
+// are looked at for maxima that left the range of their type: a group is renormalised at its start only, so
+// cancellation in its steps can take squares of entries that are not zero below it.
 template <class R>
-__device__ __forceinline__ int add_exponents(const unsigned long long* mb, int lo, int n, dcs_scale* sp) {
+__device__ __forceinline__ int add_exponents(const unsigned long long* mb, int lo, int n, int look, dcs_scale* sp) {
     const int lane = threadIdx.x & 31;
     double m2 = 1.0;
-    if (lane < n) m2 = (double)bits_to_m2<R>(__ldcg(mb + lo + lane));
+    if (lane < look) m2 = (double)bits_to_m2<R>(__ldcg(mb + lo + lane));
     const int x = exponent_of_max<R>(m2);
     int e = x - __shfl_up_sync(0xffffffffu, x, 1);
     if (lane == 0) e = x;
-    const unsigned bad = __ballot_sync(0xffffffffu, !isfinite(m2)), zero = __ballot_sync(0xffffffffu, m2 == 0.0);
+    const unsigned none = __ballot_sync(0xffffffffu, m2 == 0.0);
+    const unsigned some = __ballot_sync(0xffffffffu, lane < look && m2 != 0.0);
+    const unsigned bad = __ballot_sync(0xffffffffu, lane < n && !isfinite(m2)), zero = n < 32 ? none & ((1u << n) - 1u) : none;
+    // (a table of zeros stays one: a maximum after a zero one means that only the squares were zero)
+    const bool lost = __any_sync(0xffffffffu, m2 > 0.0 && m2 < kLeastMax<R>) ||
+                      (some && none & ((1u << (31 - __clz(some))) - 1u));
     double lg = sp->logscale;
     int sum = 0;
     for (int j = 0; j < n; ++j) {
@@ -191,6 +205,7 @@ __device__ __forceinline__ int add_exponents(const unsigned long long* mb, int l
         sp->exponent_sum += sum;
         if (bad) sp->flags |= 1u;
         if (zero) sp->flags |= 2u;
+        if (lost) sp->flags |= kFlagRange;
     }
     return sum;
 }
@@ -239,10 +254,6 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     fill_tables<NT, kMaxDim, SH>(A, tab, hi_tab);
     after_previous();  // the tables above are the plan's
     const int e = exponent_of_max<R>((double)bits_to_m2<R>(mb[A.first]));
-    if (blockIdx.x == 0 && threadIdx.x < 32) {
-        const int lo = kStepMax<S> ? A.prev_first + 1 : A.first;
-        add_exponents<R>(mb, lo, A.first - lo + 1, scale + item);
-    }
     if (threadIdx.x < A.count) {
         const dcs_param p = params[(uint64_t)item * param_stride + A.first + threadIdx.x];
         // the pass's power of two goes into the first step's weights (exact)
@@ -265,6 +276,7 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     const bool pair = sizeof(S) == 8 && low >= 1;
     const bool pair_in = pair && !(A.in_inactive & 1), pair_out = pair && !(A.out_inactive & 1);
     R gm = 0;
+    uint32_t left = 0;  // zero if every entry written is
     for (uint64_t tile = blockIdx.x; tile < ntiles; tile += gridDim.x) {
         const uint64_t base = deposit(tile, A.coset_runs, A.ncoset_runs);
         auto addr = [&](int t) { return base ^ hi_tab[t >> low] ^ ((uint64_t)t & lowmask); };
@@ -286,6 +298,10 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
                 else
                     asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(dst), "l"(E + a) : "memory");
             }
+        }
+        if (tile == 0 && threadIdx.x < 32) {  // (one CTA, once, while its entries are on their way)
+            const int lo = kStepMax<S> ? A.prev_first + 1 : A.first;
+            add_exponents<R>(mb, lo, A.first - lo + 1, A.first - lo + 1, scale + item);
         }
         asm volatile("cp.async.wait_all;\n" ::: "memory");
         __syncthreads();
@@ -320,7 +336,9 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
             for (int t = 2 * threadIdx.x; t < T; t += 2 * NT) {
                 const uint64_t a = addr(t);
                 if (a & A.out_inactive) continue;
-                *reinterpret_cast<float4*>(E + a) = *reinterpret_cast<const float4*>(smem + ((size_t)t << SH));
+                const uint4 v = *reinterpret_cast<const uint4*>(smem + ((size_t)t << SH));
+                left |= (v.x | v.y | v.z | v.w) & ~kSign;
+                *reinterpret_cast<uint4*>(E + a) = v;
             }
         } else {
             for (int t = threadIdx.x; t < T; t += NT) {
@@ -328,16 +346,19 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
                 if (a & A.out_inactive) continue;
                 const S v = *reinterpret_cast<const S*>(smem + ((size_t)t << SH));
                 if constexpr (!kStepMax<S>) gm = fmax(gm, v.x * v.x + v.y * v.y);
+                left |= nonzero_bits(v);
                 E[a] = v;
             }
         }
         __syncthreads();
     }
+    // (a maximum that is zero although entries are not gets the least number there is, which sets kFlagRange)
     if constexpr (!kStepMax<S>) {
-        const unsigned long long bm = block_max_u64(max_bits(gm));
+        const unsigned long long bm = block_max_u64(gm == 0 && left ? 1ull : max_bits(gm));
         if (threadIdx.x == 0 && bm) atomicMax(&mb[A.first + A.count], bm);
         return;
     }
+    if (left && !smax[A.count - 1]) atomicMax(&mb[A.first + A.count], 1ull);
     if (threadIdx.x < A.count && smax[threadIdx.x])
         atomicMax(&mb[A.first + threadIdx.x + 1], (unsigned long long)smax[threadIdx.x]);
     if (!A.last) return;
@@ -351,7 +372,7 @@ k_tiles(S* __restrict__ table, uint64_t table_stride, const __grid_constant__ Ti
     __syncthreads();
     if (!s_end || threadIdx.x >= 32) return;
     __threadfence();
-    const int rest = add_exponents<R>(mb, A.first + 1, A.count - 1, sp);
+    const int rest = add_exponents<R>(mb, A.first + 1, A.count - 1, A.count, sp);
     if (threadIdx.x == 0) sp->table_exp = rest;
 }
 

@@ -15,8 +15,10 @@ Execution modes (``alloc(..., mode=...)``):
 * ``"device"`` — the renormalisation stays on the device; all steps of all slices are
   enqueued without host synchronisation, several slices (work items) per launch when the
   HBM budget allows (default).  complex64 and complex128 tables take up to 24 steps per launch,
-  tile by tile in shared memory (csrc/tiles.cu); step weights outside ``TILE_WEIGHT_RANGE``, and
-  binary16 tables of more than one tile, one step per launch;
+  tile by tile in shared memory (csrc/tiles.cu); step weights outside ``TILE_WEIGHT_RANGE`` or of too
+  much growth (``weights_ok``), batches whose entries cancel below the range of a group
+  (``out_of_range``: they run a second time), and binary16 tables of more than one tile, one step per
+  launch;
 * ``"fused"``  — like ``device`` but several vertex steps per pass over the table
   (coset-tiled fused kernels; complex128 tables run the plan-specialised register-run kernels
   compiled in FP64, which is how the complex128 audit recontraction runs at full size).
@@ -87,6 +89,9 @@ def device_steps(steps):
         for j, (src, dst, ln) in enumerate(runs):
             r["runs"][j] = src | (dst << 8) | (ln << 16)
     return out
+
+
+FLAG_RANGE = 8  # scale flag: a table's maximum left the range of its square (see out_of_range)
 
 
 def raise_for_flags(flags):
@@ -772,7 +777,26 @@ class InplaceConditionalBlockGPU:
         """Device work for a prepared batch into `out` ((nblocks, 2^k) complex128): contraction of
         every work item, accumulation, tail.  No host synchronisation (except in "plain" mode).
         flags: optional (self.items,) int64 device tensor that collects the items' scale flags
-        (bit 0: a nonfinite table).  Returns the number of library kernel launches."""
+        (bit 0: a nonfinite table; bit 3: see out_of_range).  Returns the number of library kernel
+        launches.
+
+        Tile groups of complex64 and complex128 tables run only where the caller takes the flags, since
+        they can report that a batch needs single steps; without flags it takes those at once."""
+        return self._enqueue(prep, out, flags, flags is not None)
+
+    def out_of_range(self, prep, flags):
+        """Whether a batch that enqueue ran on tile groups, with these flags (host), has to run again with
+        single_steps(prep): its entries cancelled so far inside a group that the squares of a maximum left
+        the storage precision's range."""
+        return (self.tplan is not None and not self.half and any(prep["unit_ok"])
+                and bool(np.any(np.asarray(flags) & FLAG_RANGE)))
+
+    @staticmethod
+    def single_steps(prep):
+        """The same batch with a launch per step."""
+        return {**prep, "unit_ok": [False] * len(prep["chunks"])}
+
+    def _enqueue(self, prep, out, flags, tiles):
         lib, st = self.lib, self._stream()
         nm = self._nmax() + 1
         entry = _lib.PARAM_DTYPE.itemsize
@@ -785,7 +809,7 @@ class InplaceConditionalBlockGPU:
         d_params, d_coefs, d_xors, d_begin = (_lib.ptr(prep[k]) for k in ("params", "coefs", "xors", "begin"))
         for ci, (c0, cn, b0, nb, boff) in enumerate(chunks):
             self._reset_items(cn, st)
-            ok = prep["unit_ok"][ci]
+            ok = prep["unit_ok"][ci] and (tiles or self.tplan is None or self.half)
             self._run_steps(d_params + c0 * self.nsteps * entry, cn, ok, st)
             launches += (len(self.fplan.groups) if self.mode == "fused" else
                          self.tile_launches if self.tplan is not None and ok else self.nsteps)
@@ -817,13 +841,19 @@ class InplaceConditionalBlockGPU:
         prep = self.prepare(x_list, w, part, parts)
         out = torch.empty((len(x_list), 1 << self.k), dtype=torch.complex128, device=self.device)
         # one small device->host read per call: the scale records of a single chunk, or the collected flags
-        flags = None if len(prep["chunks"]) == 1 else self._flags_tensor()
-        self.enqueue(prep, out, flags)
-        if flags is None:
-            cn = prep["chunks"][0][1]
-            raise_for_flags(self.scale[: cn * _SCALE_WORDS].cpu().numpy().view(_lib.SCALE_DTYPE)["flags"])
-        else:
-            raise_for_flags(flags.cpu().numpy())
+        single = len(prep["chunks"]) == 1
+        while True:
+            flags = None if single else self._flags_tensor()
+            self._enqueue(prep, out, flags, True)
+            if single:
+                cn = prep["chunks"][0][1]
+                seen = self.scale[: cn * _SCALE_WORDS].cpu().numpy().view(_lib.SCALE_DTYPE)["flags"]
+            else:
+                seen = flags.cpu().numpy()
+            if not self.out_of_range(prep, seen):
+                break
+            prep = self.single_steps(prep)
+        raise_for_flags(seen)
         return out, prep
 
     def block(self, x_bits, w=None, part=0, parts=1):

@@ -199,24 +199,7 @@ def sample_checked(engine, x_list, uniforms, hashes=True, exact_cdf=False, strad
     copied = [None, None]
     out, blocks = [], []
 
-    def finish(i, slot):
-        copied[slot].synchronize()
-        from .engine import raise_for_flags
-        raise_for_flags(host_flags[slot].numpy())
-        rec = record_dict(host_res[slot].numpy().view(_lib.DRAW_DTYPE)[0], straddle_rel_l2)
-        if hashes:
-            rec.update(block_hashes(host_blk[slot].numpy()))
-        rec["replay_scope"] = REPLAY_SCOPE
-        out.append(rec)
-        if keep_host_blocks:
-            blocks.append(host_blk[slot].numpy().copy())
-
-    prep = engine.prepare([x_list[0]])
-    pending = None
-    for i in range(n):
-        slot = i & 1
-        if copied[slot] is not None:  # sample i - 2's copies out of this slot are done
-            stream.wait_event(copied[slot])
+    def contract_and_draw(i, slot, prep):
         flags[slot].zero_()
         engine.enqueue(prep, outs[slot], flags=flags[slot])
         _lib.check(lib.dcs_draw_ex(_lib.ptr(outs[slot]), k, 1, _lib.ptr(d_u[i:i + 1]),
@@ -233,11 +216,35 @@ def sample_checked(engine, x_list, uniforms, hashes=True, exact_cdf=False, strad
         ev = torch.cuda.Event()
         ev.record(copy_stream)
         copied[slot] = ev
+
+    def finish(i, slot, prep):
+        copied[slot].synchronize()
+        from .engine import raise_for_flags
+        if engine.out_of_range(prep, host_flags[slot].numpy()):
+            contract_and_draw(i, slot, engine.single_steps(prep))
+            copied[slot].synchronize()
+        raise_for_flags(host_flags[slot].numpy())
+        rec = record_dict(host_res[slot].numpy().view(_lib.DRAW_DTYPE)[0], straddle_rel_l2)
+        if hashes:
+            rec.update(block_hashes(host_blk[slot].numpy()))
+        rec["replay_scope"] = REPLAY_SCOPE
+        out.append(rec)
+        if keep_host_blocks:
+            blocks.append(host_blk[slot].numpy().copy())
+
+    prep = engine.prepare([x_list[0]])
+    pending = None
+    for i in range(n):
+        slot = i & 1
+        if copied[slot] is not None:  # sample i - 2's copies out of this slot are done
+            stream.wait_event(copied[slot])
+        contract_and_draw(i, slot, prep)
+        ran = prep
         if i + 1 < n:
             prep = engine.prepare([x_list[i + 1]])
         if pending is not None:
             finish(*pending)
-        pending = (i, slot)
+        pending = (i, slot, ran)
     finish(*pending)
     return (out, blocks) if keep_host_blocks else out
 

@@ -37,7 +37,7 @@ import numpy as np
 import torch
 
 from . import _lib
-from .engine import DeviceCircuit, InplaceConditionalBlockGPU, item_chunks
+from .engine import FLAG_RANGE, DeviceCircuit, InplaceConditionalBlockGPU, item_chunks
 
 
 class TablePool:
@@ -110,6 +110,7 @@ class Batch:
     xbits: torch.Tensor      # pinned prefix masks
     launched: float
     region: tuple = None     # pool region holding the batch's tables
+    flags: torch.Tensor = None  # pinned scale flags, where the batch ran on tile groups
 
 
 class CircuitRunner:
@@ -171,6 +172,9 @@ class CircuitRunner:
         self.d_begin = torch.empty(4 * M * L + 8, dtype=torch.int32, device=dev)
         self.d_out = torch.empty((M, 1 << self.k), dtype=torch.complex128, device=dev)
         self.d_res = torch.empty(M * _lib.DRAW_DTYPE.itemsize, dtype=torch.uint8, device=dev)
+        # tile groups report through the flags whether a batch has to run again with single steps
+        self.tiles = self.engine.tplan is not None and self.dc.unit_ok
+        self.d_flags = torch.zeros(items, dtype=torch.int64, device=dev) if self.tiles else None
         self.d_scratch = torch.empty(self.lib.dcs_draw_scratch_bytes(self.k, M), dtype=torch.uint8, device=dev)
 
     def table_bytes(self):
@@ -199,9 +203,10 @@ class CircuitRunner:
         """Launch chunks of engine.items work items and, per chunk, the item ranges of its blocks."""
         return item_chunks(n, self.dc.nslices, self.engine.items)
 
-    def _device_work(self, n, chunks):
+    def _device_work(self, n, chunks, tiles):
         """Every device step of a batch of n samples after the id upload, on self.stream, with
-        fixed buffers only (so that it can be captured as a CUDA graph)."""
+        fixed buffers only (so that it can be captured as a CUDA graph).  tiles: in device mode, on
+        tile groups (else a launch per step)."""
         eng, lib = self.engine, self.lib
         st = self.stream.cuda_stream
         _lib.check(lib.dcs_philox_prefixes(_lib.ptr(self.d_ids), _lib.ptr(self.d_ids) + 4 * n, n, self.key,
@@ -212,19 +217,22 @@ class CircuitRunner:
         fresh = _lib.ACCUMULATE_FRESH if len(chunks) == 1 else 0  # one chunk writes the blocks, several add to them
         if not fresh:
             out.zero_()
+        if tiles:
+            self.d_flags.zero_()
         entry = _lib.PARAM_DTYPE.itemsize
         nm = eng._nmax() + 1
         for c0, cn, b0, nb, boff in chunks:
             eng._reset_items(cn)
             # (fused mode: weights that the generated kernels cannot take have switched them off)
-            eng._run_steps(_lib.ptr(self.d_params) + c0 * eng.nsteps * entry, cn,
-                           self.dc.unit_ok or self.mode == "fused")
+            eng._run_steps(_lib.ptr(self.d_params) + c0 * eng.nsteps * entry, cn, tiles or self.mode == "fused")
             _lib.check(lib.dcs_accumulate_ex(
                 eng.dcode, _lib.ptr(eng.table), eng.table_stride, eng.plan.terminal_rank,
                 eng.term_runs.ctypes.data, eng.term_nruns, eng.tbasis.ctypes.data,
                 _lib.ptr(self.d_xors) + 8 * c0, _lib.ptr(self.d_coefs) + 16 * c0,
                 _lib.ptr(self.d_begin) + 4 * boff, nb, eng.params.shift, _lib.ptr(eng.scale),
                 _lib.ptr(eng.maxbits[nm - 1:]), nm, _lib.ptr(out[b0:b0 + nb]), self.k, cn, fresh, st))
+            if tiles:
+                _lib.check(lib.dcs_collect_flags(_lib.ptr(eng.scale), _lib.ptr(self.d_flags), cn, st))
         _lib.check(lib.dcs_block_tail(_lib.ptr(out), self.k, eng.adj_hi.ctypes.data, eng.u_open.ctypes.data, n, st))
         _lib.check(lib.dcs_draw(_lib.ptr(out), self.k, n, _lib.ptr(self.d_u), _lib.ptr(self.d_scratch),
                                 _lib.ptr(self.d_res), st))
@@ -233,11 +241,11 @@ class CircuitRunner:
         g = self._graph.get(n)
         if g is None:
             # one direct run first (kernel attributes, allocator), then the capture
-            self._device_work(n, chunks)
+            self._device_work(n, chunks, self.tiles)
             self.stream.synchronize()
             g = torch.cuda.CUDAGraph()
             with torch.cuda.graph(g, stream=self.stream):
-                self._device_work(n, chunks)
+                self._device_work(n, chunks, self.tiles)
             self._graph[n] = g
         g.replay()
 
@@ -255,9 +263,10 @@ class CircuitRunner:
                 self._replay(n, chunks)
         self.stream.synchronize()
 
-    def launch(self, samples, region=()):
+    def launch(self, samples, region=(), tiles=None):
         """Enqueue one batch (list of (request id, sample index)) on the tables of `region` (from
-        grant); returns a Batch."""
+        grant); returns a Batch.  tiles=False: with a launch per step (see out_of_range)."""
+        tiles = self.tiles if tiles is None else tiles
         n = len(samples)
         assert 0 < n <= self.max_samples
         chunks, begins = self._chunks(n)
@@ -266,18 +275,28 @@ class CircuitRunner:
                                dtype=torch.int32).pin_memory()
             self.d_begin[:len(begins)].copy_(ids[2 * n:], non_blocking=True)
             self.d_ids[:2 * n].copy_(ids[:2 * n], non_blocking=True)
-            if self.graphs:
+            if self.graphs and tiles == self.tiles:
                 self._replay(n, chunks)
             else:
-                self._device_work(n, chunks)
+                self._device_work(n, chunks, tiles)
             host = torch.empty(n * _lib.DRAW_DTYPE.itemsize, dtype=torch.uint8).pin_memory()
             host.copy_(self.d_res[:n * _lib.DRAW_DTYPE.itemsize], non_blocking=True)
             hx = torch.empty(n, dtype=torch.int64).pin_memory()
             hx.copy_(self.d_x[:n], non_blocking=True)
+            hf = None
+            if tiles:
+                hf = torch.empty(self.d_flags.numel(), dtype=torch.int64).pin_memory()
+                hf.copy_(self.d_flags, non_blocking=True)
             ev = torch.cuda.Event()
             ev.record(self.stream)
             self._hold = ids  # the pinned upload must outlive its copy
-        return Batch(list(samples), ev, host, hx, time.perf_counter(), region or None)
+        return Batch(list(samples), ev, host, hx, time.perf_counter(), region or None, hf)
+
+    @staticmethod
+    def out_of_range(batch):
+        """Whether a finished batch has to be launched again, on the same tables, with tiles=False
+        (InplaceConditionalBlockGPU.out_of_range)."""
+        return batch.flags is not None and bool(np.any(batch.flags.numpy() & FLAG_RANGE))
 
 
 @dataclass
@@ -336,6 +355,10 @@ class Server:
             for c, run in self.runners.items():
                 b = inflight[c]
                 if b is not None and b.event.query():
+                    if run.out_of_range(b):
+                        inflight[c] = run.launch(b.samples, b.region or (), tiles=False)
+                        progressed = True
+                        continue
                     recs = b.host.numpy().view(_lib.DRAW_DTYPE)
                     xs = b.xbits.numpy()
                     tnow = time.perf_counter() - t0

@@ -103,7 +103,9 @@ typedef struct dcs_param {
 typedef struct dcs_scale {
     double logscale;
     int64_t exponent_sum;
-    uint32_t flags; /* bit 0: a nonfinite maximum was seen; bit 1: the table became zero */
+    uint32_t flags; /* bit 0: a nonfinite maximum was seen; bit 1: the table became zero; bit 2: a generated
+                       kernel's bounded wait gave up; bit 3: a maximum |entry|^2 fell below the normal range of
+                       its type (after dcs_tile_groups the item has to run again with a launch per step) */
     int32_t table_exp; /* the entries are the table's times 2^-table_exp (dcs_tile_groups; else 0) */
     double phase;   /* radians: the argument of the step factors the plan-specialised kernels divide
                        out of the weights (the table is e^{logscale + i phase} times its entries) */
@@ -290,7 +292,8 @@ int dcs_fused_runs(void *table, const dcs_step *steps, int nsteps, const dcs_gro
  * params + i*param_stride, maxbits + i*maxbits_stride (word s + 1 receives the max of step s, for
  * complex128 of a group's last step s only; word 0 holds the bits of 1.0) and scale + i (all zero on entry).  The table is renormalised once per group, so
  * the weights of a group must not let an entry leave the storage precision's range, nor in complex64 |entry|^2 that
- * of FP32 (entries below 2^63); the power of two that
+ * of FP32 (entries below 2^63); an item whose entries cancel so far inside a group that their squares leave the
+ * range at the lower end has bit 3 of its flags set, and no valid table; the power of two that
  * a complex64 table still has is in table_exp.  DCS_H16: groups of one tile (2^13 entries at most) run
  * in one launch with every step's own renormalisation, the others a launch per step; maxbits_stride is
  * nsteps + 1.  Steps 0 .. nsteps - 1

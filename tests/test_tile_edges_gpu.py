@@ -69,3 +69,118 @@ def test_weights_at_the_ends_of_the_range(weight, leaves, dtype):
     want, _ = OracleEngine(*args[:4], [], args[4]).block(x, w)
     got = eng.block(x, w)[0].cpu().numpy()
     assert np.linalg.norm(got - want) <= 4 * leaves * 2.0 ** -24 * np.linalg.norm(want)
+
+
+def _with_isolated(shape, before, factors, seed=3):
+    """A ring circuit's graph with isolated reference vertices, which multiply the table by f0 + f1, in the middle of
+    the order: a product of small factors, as an improbable outcome of many vertices gives one."""
+    from dcs245_classical_sampling_b200.circuits import build_ring_instance
+    from dcs245_classical_sampling_b200.workloads import sweep_order
+    n, depth, t, k = shape
+    inst = build_ring_instance(n, depth, t, seed)
+    opened = list(range(n - k, n))
+    order = [int(v) for v in sweep_order(inst, opened)]
+    g = np.asarray(inst["graph"], np.uint8)
+    N, m = len(g), len(factors)
+    A = np.zeros((N + m, N + m), np.uint8)
+    A[:N, :N] = g
+    # the default bra takes the first row: f = (1, factor - 1), exact for the factors used here
+    U = np.concatenate([np.asarray(inst["unitaries"], complex), np.array([[[1, f - 1], [0, 0]] for f in factors], complex)])
+    at = int(before * (len(order) - k))
+    return A, U, n, order[:at] + list(range(N, N + m)) + order[at:], opened
+
+
+SMALL, GROW = 2.0 ** -7, 2.0  # f0 + f1
+# 2^-49 .. 2^-280: squares normal, below the normal range, zero; zero inside a group and then not; one group and more
+FACTORS = {"7": [SMALL] * 7, "9": [SMALL] * 9, "10": [SMALL] * 10, "11": [SMALL] * 11, "20": [SMALL] * 20,
+           "40": [SMALL] * 40, "12 and back": [SMALL] * 12 + [GROW] * 10, "10 and back": [SMALL] * 10 + [GROW] * 3}
+
+
+@pytest.mark.parametrize("factors", FACTORS)
+@pytest.mark.parametrize("shape,before", [((6, 6, 9, 3), 0.0), ((6, 6, 9, 3), 1.0), ((14, 15, 50, 5), 0.5), ((34, 38, 150, 11), 0.4)])
+def test_small_products_are_not_lost(shape, before, factors):
+    """Maxima whose squares leave the FP32 range inside a group: the block of a launch per step, not zero."""
+    args = _with_isolated(shape, before, FACTORS[factors])
+    x = np.random.default_rng(shape[0]).integers(0, 2, shape[0]).astype(np.uint8)
+    eng = _engine(*args, items=2)
+    got = eng.blocks([x, x]).cpu().numpy()
+    plan, eng.tplan = eng.tplan, None
+    want = eng.blocks([x, x]).cpu().numpy()
+    eng.tplan = plan
+    assert np.linalg.norm(want) > 0 and np.array_equal(got, want)
+    one = eng.block(x)[0].cpu().numpy()
+    assert np.array_equal(one, want[0])
+    ref = _engine(*args, dtype=np.complex128).block(x)[0].cpu().numpy()
+    assert np.linalg.norm(one - ref) <= 1e-5 * np.linalg.norm(ref)  # complex64 against complex128 tables
+
+
+@pytest.mark.parametrize("count", [24, 30])
+def test_small_products_in_complex128(count):
+    """24 factors of 2^-22 (2^-528) leave the range of an FP64 square."""
+    args = _with_isolated((14, 15, 50, 5), 0.5, [2.0 ** -22] * count)
+    x = np.random.default_rng(14).integers(0, 2, 14).astype(np.uint8)
+    eng = _engine(*args, dtype=np.complex128)
+    got = eng.block(x)[0].cpu().numpy()
+    eng.tplan = None
+    want = eng.block(x)[0].cpu().numpy()
+    size = np.abs(want).max()
+    assert size > 0 and np.abs(got - want).max() <= 1e-12 * size
+
+
+def test_zero_tables_take_no_second_run(monkeypatch):
+    """A table that is zero (f0 + f1 = 0 exactly) stays a zero block, and is not taken for a lost one."""
+    from dcs245_classical_sampling_b200.engine import InplaceConditionalBlockGPU
+    args = _with_isolated((14, 15, 50, 5), 0.5, [0.0] * 3)
+    again = []
+    monkeypatch.setattr(InplaceConditionalBlockGPU, "single_steps", staticmethod(lambda prep: again.append(1)))
+    for dtype in (np.complex64, np.complex128):
+        assert not _engine(*args, dtype=dtype).block(np.zeros(14, np.uint8))[0].cpu().numpy().any()
+    assert not again
+
+
+def _spy(monkeypatch):
+    from dcs245_classical_sampling_b200.engine import InplaceConditionalBlockGPU
+    calls, plain = [], InplaceConditionalBlockGPU.single_steps
+    monkeypatch.setattr(InplaceConditionalBlockGPU, "single_steps", staticmethod(lambda prep: calls.append(1) or plain(prep)))
+    return calls
+
+
+def test_checked_samples_and_enqueue_of_small_products(monkeypatch):
+    import torch
+
+    from dcs245_classical_sampling_b200.sampling import sample_checked
+    args = _with_isolated((14, 15, 50, 5), 0.5, [SMALL] * 20)
+    rng = np.random.default_rng(5)
+    xs, us = [rng.integers(0, 2, 14).astype(np.uint8) for _ in range(5)], rng.random(5).tolist()
+    eng = _engine(*args)
+    calls = _spy(monkeypatch)
+    recs, blocks = sample_checked(eng, xs, us, keep_host_blocks=True)
+    assert len(calls) == 5
+    plain = _engine(*args, dtype=np.complex64)
+    plain.tplan = None
+    recs2, blocks2 = sample_checked(plain, xs, us, keep_host_blocks=True)
+    assert recs == recs2 and all(np.array_equal(a, b) for a, b in zip(blocks, blocks2))
+    prep, out = eng.prepare([xs[0]]), torch.empty((1, 32), dtype=torch.complex128, device="cuda")
+    eng.enqueue(prep, out)  # nobody looks at flags: single steps
+    assert np.array_equal(out[0].cpu().numpy(), blocks[0])
+    flags = torch.zeros(eng.items, dtype=torch.int64, device="cuda")
+    eng.enqueue(prep, out, flags)
+    assert eng.out_of_range(prep, flags.cpu().numpy())
+
+
+@pytest.mark.parametrize("graphs", [False, True])
+def test_served_samples_of_small_products(graphs):
+    from dcs245_classical_sampling_b200.sampling import draw_many
+    from dcs245_classical_sampling_b200.serve import CircuitRunner, Request, Server
+    A, U, n, order, opened = _with_isolated((14, 15, 50, 5), 0.5, [SMALL] * 20)
+    w = {"graph": A, "unitaries": U, "n": n, "order": order, "parity_operations": [], "open_vertices": opened}
+    run = CircuitRunner("c", w, 11, 4, graphs=graphs)
+    reqs = Server({"c": run}).run([Request(i, "c", 3, 0.0) for i in range(4)], realtime=False)
+    ref = _engine(A, U, n, order, opened, dtype=np.complex128)
+    for r in reqs:
+        for i in range(3):
+            rec, mask = r.records[i]
+            x = np.array([mask >> q & 1 for q in range(n)], np.uint8)
+            want = draw_many(ref.block(x)[0], [float(rec["uniform"])])[0]
+            assert rec["status"] == 0 and rec["total_exact"] > 0
+            assert abs(rec["total_exact"] / want["total_exact"] - 1) <= 2e-5  # squares of amplitudes within 1e-5
