@@ -327,7 +327,7 @@ extern "C" int dcs_accumulate_ex(int dtype, const void* table, uint64_t table_st
     auto run = [&](auto kernel, auto t) {
         return dcs_host::check_cuda(
             dcs_host::launch_after(kernel, grid, dim3(256), 0, st, t, table_stride, tm, xors, coefs, item_begin, log_shift, scale,
-                                   (const unsigned long long*)maxbits_final, mstride, dtype == DCS_C128 ? 1 : 0,
+                                   (const unsigned long long*)maxbits_final, mstride, dtype != DCS_C64 ? 1 : 0,  // (binary16: FP64 arithmetic)
                                    (flags & DCS_ACCUMULATE_FRESH) ? 1 : 0, (double2*)total),
             "k_accumulate launch");
     };

@@ -85,7 +85,8 @@ def _with_isolated(shape, before, factors, seed=3):
     A = np.zeros((N + m, N + m), np.uint8)
     A[:N, :N] = g
     # the default bra takes the first row: f = (1, factor - 1), exact for the factors used here
-    U = np.concatenate([np.asarray(inst["unitaries"], complex), np.array([[[1, f - 1], [0, 0]] for f in factors], complex)])
+    rows = np.array([[[1, f - 1], [0, 0]] for f in factors], complex).reshape(m, 2, 2)
+    U = np.concatenate([np.asarray(inst["unitaries"], complex), rows])
     at = int(before * (len(order) - k))
     return A, U, n, order[:at] + list(range(N, N + m)) + order[at:], opened
 
@@ -184,3 +185,18 @@ def test_served_samples_of_small_products(graphs):
             want = draw_many(ref.block(x)[0], [float(rec["uniform"])])[0]
             assert rec["status"] == 0 and rec["total_exact"] > 0
             assert abs(rec["total_exact"] / want["total_exact"] - 1) <= 2e-5  # squares of amplitudes within 1e-5
+
+
+@pytest.mark.parametrize("shape,tiles", [((6, 6, 9, 3), False), ((30, 33, 120, 15), True)])
+@pytest.mark.parametrize("storage", [None, "float16"])
+def test_overflow_in_the_last_step_is_reported(shape, tiles, storage):
+    """A weight past the storage's range at the last vertex: no block with infinities in it, on one tile or many."""
+    A, U, n, order, opened = _with_isolated(shape, 0.5, [])
+    x = np.random.default_rng(1).integers(0, 2, n).astype(np.uint8)
+    eng = _engine(A, U, n, order, opened, storage=storage)
+    assert (int(eng.tplan.groups[-1]["coset_m"]) > 0) == tiles
+    last = int(eng.params.keep[eng.plan.steps[-1].v])
+    eng.block(x)
+    U[last] *= 1e6 if storage else 1e30  # entries up to 65504, |entry|^2 up to 3.4e38
+    with pytest.raises(ArithmeticError):
+        _engine(A, U, n, order, opened, storage=storage).block(x)
