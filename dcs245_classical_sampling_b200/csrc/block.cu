@@ -56,12 +56,13 @@ k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ Term
             const unsigned long long mf = maxbits_final[(uint64_t)it * mstride];
             const double m2 = is64 ? __longlong_as_double((long long)mf) : (double)__uint_as_float((uint32_t)mf);
             ItemTerm t;
-            // a zero table (skipped slice: at some step, or after the last one) or a nonfinite one adds nothing
-            t.on = !(sc.flags & 3u) && mf != 0 && isfinite(m2);
-            // the reference checks every step's max, including the last (every other reader of the flags in
-            // this launch takes the maximum itself)
+            // a zero table (skipped slice: at some step, or after the last one) or one that was nonfinite before the
+            // last step adds nothing; one that the last step made nonfinite shows in the block, too
+            t.on = mf != 0 && (!(sc.flags & 3u) || (sc.flags & kFlagLast));
+            // the reference checks every step's max, including the last (kFlagLast: the launch's other CTAs may
+            // read the flags before or after this)
             if (blockIdx.x == 0) {
-                if (!isfinite(m2)) scale[it].flags = sc.flags | 1u;
+                if (!isfinite(m2)) scale[it].flags = sc.flags | (sc.flags & 1u ? 0u : 1u | kFlagLast);
                 else if (m2 > 0.0 && m2 < (is64 ? kLeastMax<double> : kLeastMax<float>)) scale[it].flags = sc.flags | kFlagRange;
             }
             const double m = exp(sc.logscale - log_shift);

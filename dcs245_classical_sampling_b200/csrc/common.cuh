@@ -131,6 +131,7 @@ __device__ __forceinline__ double exp2_neg(int e) {  // 2^-e, |e| < 1000
 // zero, are then not known): the least normal number of the maximum's type.
 template <class R> constexpr double kLeastMax = sizeof(R) == 4 ? 0x1p-126 : 0x1p-1022;
 constexpr uint32_t kFlagRange = 8u;  // dcs_scale.flags: such a maximum was seen
+constexpr uint32_t kFlagLast = 16u;  // with bit 0: the nonfinite maximum is the last step's
 
 // block-wide max of an unsigned 64-bit value; result valid in thread 0
 __device__ __forceinline__ unsigned long long block_max_u64(unsigned long long v) {

@@ -105,7 +105,8 @@ typedef struct dcs_scale {
     int64_t exponent_sum;
     uint32_t flags; /* bit 0: a nonfinite maximum was seen; bit 1: the table became zero; bit 2: a generated
                        kernel's bounded wait gave up; bit 3: a maximum |entry|^2 fell below the normal range of
-                       its type (after dcs_tile_groups the item has to run again with a launch per step) */
+                       its type (after dcs_tile_groups the item has to run again with a launch per step); bit 4:
+                       with bit 0, the nonfinite maximum is the last step's (the table is in the block) */
     int32_t table_exp; /* the entries are the table's times 2^-table_exp (dcs_tile_groups; else 0) */
     double phase;   /* radians: the argument of the step factors the plan-specialised kernels divide
                        out of the weights (the table is e^{logscale + i phase} times its entries) */

@@ -200,3 +200,25 @@ def test_overflow_in_the_last_step_is_reported(shape, tiles, storage):
     U[last] *= 1e6 if storage else 1e30  # entries up to 65504, |entry|^2 up to 3.4e38
     with pytest.raises(ArithmeticError):
         _engine(A, U, n, order, opened, storage=storage).block(x)
+
+
+@pytest.mark.parametrize("storage,weight", [(None, 1e36), ("float16", 1e6)])
+def test_overflow_in_the_last_step_shows_in_the_block(storage, weight):
+    """A caller that takes no flags does not get a finite block without the overflowed table."""
+    import torch
+    A, U, n, order, opened = _with_isolated((14, 15, 50, 5), 0.5, [])
+    xs = np.random.default_rng(1).integers(0, 2, (3, n)).astype(np.uint8)
+    eng = _engine(A, U, n, order, opened, storage=storage)
+    last = int(eng.params.keep[eng.plan.steps[-1].v])
+    U[last] *= weight  # |entry|^2 past FP32, entries past binary16
+    eng = _engine(A, U, n, order, opened, storage=storage, items=2)
+    out = torch.zeros((3, 32), dtype=torch.complex128, device="cuda")
+    flags = torch.zeros(2, dtype=torch.int64, device="cuda")
+    eng.enqueue(eng.prepare(list(xs)), out, flags)
+    got = out.cpu().numpy()
+    assert np.all(flags.cpu().numpy() & 1)
+    if storage:  # infinite entries
+        assert not np.isfinite(got).all(axis=1).any()
+    else:  # entries whose squares are infinite: the block itself is right
+        want = _engine(A, U, n, order, opened, dtype=np.complex128).blocks(list(xs)).cpu().numpy()
+        assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
