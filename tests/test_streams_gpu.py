@@ -1,0 +1,72 @@
+"""Audits and draws that run at the same time on several streams of one GPU: no workspace is shared."""
+import threading
+
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+
+class _Recorder:
+    """The library with one entry point's calls recorded."""
+
+    def __init__(self, lib, name, arg):
+        self.lib, self.name, self.arg, self.seen = lib, name, arg, []
+
+    def __getattr__(self, attr):
+        fn = getattr(self.lib, attr)
+        if attr != self.name:
+            return fn
+
+        def call(*args):
+            self.seen.append(args[self.arg])
+            return fn(*args)
+        return call
+
+
+def _pairs(count, bits):
+    import torch
+    g = torch.Generator(device="cuda")
+    g.manual_seed(bits)
+    v = torch.view_as_complex(torch.randn((count, 2, 1 << bits, 2), generator=g, dtype=torch.float64, device="cuda"))
+    torch.cuda.synchronize()
+    return v
+
+
+def _in_streams(run, count):
+    """run(i) on a stream and a thread of its own, all at once, twenty times each; the last results."""
+    import torch
+    out, errors = [None] * count, []
+    gate = threading.Barrier(count)
+
+    def work(i):
+        try:
+            with torch.cuda.stream(torch.cuda.Stream()):
+                gate.wait()
+                for _ in range(20):
+                    got = run(i)
+                    assert out[i] is None or repr(out[i]) == repr(got)
+                    out[i] = got
+        except Exception as e:  # a thread's failure fails the test
+            errors.append(e)
+    threads = [threading.Thread(target=work, args=(i,)) for i in range(count)]
+    for t in threads:
+        t.start()
+    for t in threads:
+        t.join()
+    assert not errors, errors
+    return out
+
+
+def test_audits_on_streams(monkeypatch):
+    import torch
+
+    from dcs245_classical_sampling_b200 import _lib, audit
+    rec = _Recorder(_lib.load(), "dcs_overlap", 4)
+    monkeypatch.setattr(audit._lib, "load", lambda: rec)
+    pairs = _pairs(4, 17)
+    want = [audit.overlap_sums(p[0], p[1]) for p in pairs]
+    with torch.cuda.stream(torch.cuda.Stream()):
+        audit.overlap_sums(pairs[0][0], pairs[0][1])
+    assert abs(rec.seen[-1] - rec.seen[0]) >= 16384
+    assert repr(_in_streams(lambda i: audit.overlap_sums(pairs[i][0], pairs[i][1]), 4)) == repr(want)
