@@ -53,20 +53,9 @@ def straddle_margin(weight_l2, rel_l2=COMPLEX64_REL_L2):
     return min(2.0 * rel_l2, STRADDLE_SIGMAS * 2.0 * rel_l2 * float(np.sqrt(max(weight_l2, 0.0))))
 
 
-class _Scratch:
-    def __init__(self):
-        self.buf = {}
-
-    def get(self, device, nbytes):
-        key = (device, 0)
-        t = self.buf.get(key)
-        if t is None or t.numel() < nbytes:
-            t = torch.empty(max(nbytes, 1 << 20), dtype=torch.uint8, device=device)
-            self.buf[key] = t
-        return t
-
-
-_scratch = _Scratch()
+def _draw_scratch(lib, k, nblocks, device):
+    """Workspace of one draw (a call's own: draws of other threads and streams may run at the same time)."""
+    return torch.empty(lib.dcs_draw_scratch_bytes(k, nblocks), dtype=torch.uint8, device=device)
 
 
 def _as_device_blocks(amplitudes, device=None):
@@ -97,7 +86,7 @@ def draw_many(blocks, uniforms, device=None, exact_cdf=False):
     k = n.bit_length() - 1
     u = torch.as_tensor(np.asarray(uniforms, dtype=np.float64).reshape(B), device=v.device)
     res = torch.empty(B * _lib.DRAW_DTYPE.itemsize, dtype=torch.uint8, device=v.device)
-    scratch = _scratch.get(v.device, lib.dcs_draw_scratch_bytes(k, B))
+    scratch = _draw_scratch(lib, k, B, v.device)
     stream = torch.cuda.current_stream(v.device).cuda_stream
     _lib.check(lib.dcs_draw_ex(_lib.ptr(v), k, B, _lib.ptr(u), _lib.DRAW_SEQUENTIAL if exact_cdf else 0,
                                _lib.ptr(scratch), _lib.ptr(res), stream))
@@ -191,7 +180,7 @@ def sample_checked(engine, x_list, uniforms, hashes=True, exact_cdf=False, strad
     outs = [torch.empty((1, 1 << k), dtype=torch.complex128, device=dev) for _ in range(2)]
     res = torch.empty((2, _lib.DRAW_DTYPE.itemsize), dtype=torch.uint8, device=dev)
     flags = torch.zeros((2, engine.items), dtype=torch.int64, device=dev)
-    scratch = _scratch.get(dev, lib.dcs_draw_scratch_bytes(k, 1))
+    scratch = _draw_scratch(lib, k, 1, dev)
     host_blk = [torch.empty(1 << k, dtype=torch.complex128).pin_memory() if hashes or keep_host_blocks else None
                 for _ in range(2)]
     host_res = [torch.empty(_lib.DRAW_DTYPE.itemsize, dtype=torch.uint8).pin_memory() for _ in range(2)]

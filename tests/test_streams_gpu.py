@@ -70,3 +70,22 @@ def test_audits_on_streams(monkeypatch):
         audit.overlap_sums(pairs[0][0], pairs[0][1])
     assert abs(rec.seen[-1] - rec.seen[0]) >= 16384
     assert repr(_in_streams(lambda i: audit.overlap_sums(pairs[i][0], pairs[i][1]), 4)) == repr(want)
+
+
+@pytest.mark.parametrize("exact_cdf", [False, True])
+def test_draws_on_streams(monkeypatch, exact_cdf):
+    import torch
+
+    from dcs245_classical_sampling_b200 import _lib, sampling
+    rec = _Recorder(_lib.load(), "dcs_draw_ex", 5)
+    monkeypatch.setattr(sampling._lib, "load", lambda: rec)
+    blocks = [p.contiguous() for p in _pairs(4, 14)]
+
+    def draw(i):
+        return sampling.draw_many(blocks[i], [0.3, 0.7], exact_cdf=exact_cdf).tolist()
+
+    want = [draw(i) for i in range(4)]
+    with torch.cuda.stream(torch.cuda.Stream()):
+        draw(0)
+    assert abs(rec.seen[-1] - rec.seen[0]) >= rec.lib.dcs_draw_scratch_bytes(14, 2)
+    assert repr(_in_streams(draw, 4)) == repr(want)
