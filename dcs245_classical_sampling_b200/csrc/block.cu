@@ -35,7 +35,7 @@ template <class S>
 __global__ void __launch_bounds__(256)
 k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ TermMap tm, const uint64_t* xors,
              const double* coefs, const int32_t* item_begin, double log_shift, dcs_scale* scale,
-             const unsigned long long* maxbits_final, uint64_t mstride, int is64, int fresh, double2* total) {
+             const unsigned long long* maxbits_final, uint64_t mstride, int is64, int fresh, int use_exp, double2* total) {
     let_next_start();
     after_previous();
     // grid.y = output block; items item_begin[b] .. item_begin[b+1]-1 belong to block b
@@ -76,7 +76,7 @@ k_accumulate(const S* table, uint64_t table_stride, const __grid_constant__ Term
             }
             t.cr = cr;
             t.ci = ci;
-            t.p2 = ldexp(1.0, -sc.table_exp);
+            t.p2 = use_exp ? ldexp(1.0, -sc.table_exp) : 1.0;
             t.xor_ = xors[it];
             terms[threadIdx.x] = t;
         }
@@ -297,20 +297,10 @@ static int build_termmap(TermMap& tm, int tr, const uint32_t* runs, int nruns, c
     return DCS_OK;
 }
 
-extern "C" int dcs_accumulate_batched(int dtype, const void* table, uint64_t table_stride, int tr,
-                                      const uint32_t* terminal_runs, int nruns, const uint64_t* tbasis,
-                                      const uint64_t* xors, const double* coefs, const int32_t* item_begin,
-                                      int nblocks, double log_shift, dcs_scale* scale, const uint64_t* maxbits_final,
-                                      uint64_t mstride, double* total, int k, int nitems, void* stream) {
-    return dcs_accumulate_ex(dtype, table, table_stride, tr, terminal_runs, nruns, tbasis, xors, coefs, item_begin, nblocks,
-                             log_shift, scale, maxbits_final, mstride, total, k, nitems, 0u, stream);
-}
-
-extern "C" int dcs_accumulate_ex(int dtype, const void* table, uint64_t table_stride, int tr,
-                                 const uint32_t* terminal_runs, int nruns, const uint64_t* tbasis, const uint64_t* xors,
-                                 const double* coefs, const int32_t* item_begin, int nblocks, double log_shift,
-                                 dcs_scale* scale, const uint64_t* maxbits_final, uint64_t mstride, double* total, int k,
-                                 int nitems, unsigned flags, void* stream) {
+static int accumulate(int dtype, const void* table, uint64_t table_stride, int tr, const uint32_t* terminal_runs, int nruns,
+                      const uint64_t* tbasis, const uint64_t* xors, const double* coefs, const int32_t* item_begin,
+                      int nblocks, double log_shift, dcs_scale* scale, const uint64_t* maxbits_final, uint64_t mstride,
+                      double* total, int k, int nitems, unsigned flags, bool use_exp, void* stream) {
     if (!table || !xors || !coefs || !item_begin || !scale || !maxbits_final || !total || nblocks < 1 ||
         nblocks > 65535 || nitems < 0 || (flags & ~(unsigned)DCS_ACCUMULATE_FRESH)) {
         dcs_host::set_error("dcs_accumulate: invalid arguments");
@@ -329,7 +319,7 @@ extern "C" int dcs_accumulate_ex(int dtype, const void* table, uint64_t table_st
         return dcs_host::check_cuda(
             dcs_host::launch_after(kernel, grid, dim3(256), 0, st, t, table_stride, tm, xors, coefs, item_begin, log_shift, scale,
                                    (const unsigned long long*)maxbits_final, mstride, dtype != DCS_C64 ? 1 : 0,  // (binary16: FP64 arithmetic)
-                                   (flags & DCS_ACCUMULATE_FRESH) ? 1 : 0, (double2*)total),
+                                   (flags & DCS_ACCUMULATE_FRESH) ? 1 : 0, use_exp ? 1 : 0, (double2*)total),
             "k_accumulate launch");
     };
     if (dtype == DCS_C64) return run(k_accumulate<float2>, (const float2*)table);
@@ -337,6 +327,25 @@ extern "C" int dcs_accumulate_ex(int dtype, const void* table, uint64_t table_st
     if (dtype == DCS_H16) return run(k_accumulate<ushort2>, (const ushort2*)table);
     dcs_host::set_error("dcs_accumulate: unknown dtype %d", dtype);
     return DCS_E_ARG;
+}
+
+extern "C" int dcs_accumulate_batched(int dtype, const void* table, uint64_t table_stride, int tr,
+                                      const uint32_t* terminal_runs, int nruns, const uint64_t* tbasis,
+                                      const uint64_t* xors, const double* coefs, const int32_t* item_begin,
+                                      int nblocks, double log_shift, dcs_scale* scale, const uint64_t* maxbits_final,
+                                      uint64_t mstride, double* total, int k, int nitems, void* stream) {
+    // (callers of the step and fused kernels need not set table_exp)
+    return accumulate(dtype, table, table_stride, tr, terminal_runs, nruns, tbasis, xors, coefs, item_begin, nblocks, log_shift,
+                      scale, maxbits_final, mstride, total, k, nitems, 0u, false, stream);
+}
+
+extern "C" int dcs_accumulate_ex(int dtype, const void* table, uint64_t table_stride, int tr,
+                                 const uint32_t* terminal_runs, int nruns, const uint64_t* tbasis, const uint64_t* xors,
+                                 const double* coefs, const int32_t* item_begin, int nblocks, double log_shift,
+                                 dcs_scale* scale, const uint64_t* maxbits_final, uint64_t mstride, double* total, int k,
+                                 int nitems, unsigned flags, void* stream) {
+    return accumulate(dtype, table, table_stride, tr, terminal_runs, nruns, tbasis, xors, coefs, item_begin, nblocks, log_shift,
+                      scale, maxbits_final, mstride, total, k, nitems, flags, true, stream);
 }
 
 extern "C" int dcs_block_tail(double* total, int k, const uint32_t* adj_hi, const double* u_open, int nblocks,

@@ -107,7 +107,9 @@ typedef struct dcs_scale {
                        kernel's bounded wait gave up; bit 3: a maximum |entry|^2 fell below the normal range of
                        its type (after dcs_tile_groups the item has to run again with a launch per step); bit 4:
                        with bit 0, the nonfinite maximum is the last step's (the table is in the block) */
-    int32_t table_exp; /* the entries are the table's times 2^-table_exp (dcs_tile_groups; else 0) */
+    int32_t table_exp; /* the entries are the table's times 2^-table_exp.  Written by dcs_begin_items (0) and
+                          dcs_tile_groups (which wants 0 on entry), read by dcs_accumulate_ex; no other entry
+                          point reads or needs it */
     double phase;   /* radians: the argument of the step factors the plan-specialised kernels divide
                        out of the weights (the table is e^{logscale + i phase} times its entries) */
 } dcs_scale;
@@ -338,8 +340,9 @@ int dcs_accumulate_batched(int dtype, const void *table, uint64_t table_stride, 
                            double log_shift, dcs_scale *scale, const uint64_t *maxbits_final, uint64_t mstride,
                            double *total, int k, int nitems, void *stream);
 
-/* dcs_accumulate_batched with flags.  DCS_ACCUMULATE_FRESH: total need not be zeroed before (the blocks start
- * at zero; every one of them is written). */
+/* dcs_accumulate_batched with flags, and with the power of two that dcs_tile_groups leaves in scale's table_exp
+ * (so table_exp is set, 0 after other kernels).  DCS_ACCUMULATE_FRESH: total need not be zeroed before (the
+ * blocks start at zero; every one of them is written). */
 #define DCS_ACCUMULATE_FRESH 1u
 int dcs_accumulate_ex(int dtype, const void *table, uint64_t table_stride, int tr, const uint32_t *terminal_runs,
                       int nruns, const uint64_t *tbasis, const uint64_t *xors, const double *coefs,
