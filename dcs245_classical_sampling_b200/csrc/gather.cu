@@ -116,7 +116,7 @@ k_gather_small(const S* Ein, S* Eout, uint64_t stride, const __grid_constant__ G
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ uint64_t T[2][kSmallBytes * 256];
     __shared__ uint64_t C[2][kMaxCombos];
-    __shared__ uint32_t smax[kSmallSteps];
+    __shared__ uint32_t smax[kSmallSteps], slow[kSmallSteps];
     __shared__ dcs_param prm[kSmallSteps];
     const int item = blockIdx.y;
     S* tab[2] = {reinterpret_cast<S*>(smem), reinterpret_cast<S*>(smem) + ((size_t)1 << G.rank)};
@@ -133,7 +133,7 @@ k_gather_small(const S* Ein, S* Eout, uint64_t stride, const __grid_constant__ G
     };
     let_next_start();
     fetch(0);
-    if (threadIdx.x < kSmallSteps) smax[threadIdx.x] = 0;
+    if (threadIdx.x < kSmallSteps) smax[threadIdx.x] = slow[threadIdx.x] = 0;
     after_previous();
     if (threadIdx.x < G.count) prm[threadIdx.x] = params[(uint64_t)item * param_stride + G.s0 + threadIdx.x];
     for (uint32_t i = threadIdx.x; i < (1u << G.st[0].r_in); i += kSmallThreads)
@@ -162,12 +162,18 @@ k_gather_small(const S* Ein, S* Eout, uint64_t stride, const __grid_constant__ G
             out[cp] = o;
             lm = fmax(lm, o.x * o.x + o.y * o.y);
         }
-        // 32 bits that order like the maximum and keep its exponent, all that the scale takes from it
+        // 32 bits that order like the maximum and keep its exponent, all that the scale takes from it; in FP64 the
+        // low half counts only for a maximum below 2^-1042, whose high half is zero
         uint32_t key = sizeof(R) == 4 ? __float_as_uint((float)lm) : (uint32_t)__double2hiint((double)lm);
         key = __reduce_max_sync(0xffffffffu, key);
         if ((threadIdx.x & 31) == 0 && key) atomicMax(&smax[i], key);
+        if (sizeof(R) == 8 && !key) {
+            key = __reduce_max_sync(0xffffffffu, (uint32_t)__double2loint((double)lm));
+            if ((threadIdx.x & 31) == 0 && key) atomicMax(&slow[i], key);
+        }
         __syncthreads();
-        const unsigned long long word = sizeof(R) == 4 ? (unsigned long long)smax[i] : (unsigned long long)smax[i] << 32;
+        const unsigned long long word = sizeof(R) == 4 ? (unsigned long long)smax[i]
+                                        : smax[i]      ? (unsigned long long)smax[i] << 32 : slow[i];
         m2 = (double)bits_to_m2<R>(word);
         if (threadIdx.x == 0) mb[G.s0 + i + 1] = word;
     }
