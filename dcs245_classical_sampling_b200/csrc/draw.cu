@@ -355,8 +355,15 @@ k_chunk(const double* w, int k, const dd* chunk_sum, int nch, const BlockState* 
                    sub_map + (uint64_t)b * (n >= (uint64_t)kSub ? n / kSub : 1));
     dd run = before;
     const double two53 = 9007199254740992.0;
-    const double inv = 1.0 / T.hi;  // T.hi > 0
-    double prev_end = ceil(dd_div(run, T, inv) * two53);
+    // quotients by the total (> 0); totals whose reciprocal is infinite, subnormal or near it are scaled, exactly
+    const double up = T.hi < 0x1p-900 ? 0x1p600 : T.hi > 0x1p900 ? 0x1p-600 : 1.0;
+    const dd Ts{T.hi * up, T.lo * up};
+    const double inv = 1.0 / Ts.hi;
+    auto share = [&](dd a) {
+        if (up != 1.0) a = dd{a.hi * up, a.lo * up};
+        return dd_div(a, Ts, inv);
+    };
+    double prev_end = ceil(share(run) * two53);
     if (start + (uint64_t)threadIdx.x * kPer == 0) prev_end = 0.0;
     double s = 0.0, q = 0.0;
 #pragma unroll
@@ -364,7 +371,7 @@ k_chunk(const double* w, int k, const dd* chunk_sum, int nch, const BlockState* 
         const uint64_t i = start + (uint64_t)threadIdx.x * kPer + j;
         if (i >= n) break;
         run = dd_add(run, loc[j]);
-        const double ci = (i == n - 1) ? 1.0 : dd_div(run, T, inv);
+        const double ci = (i == n - 1) ? 1.0 : share(run);
         const double end = ceil(ci * two53);
         const double p = loc[j] / mass;
         s += fabs((end - prev_end) / two53 - p);
