@@ -83,7 +83,8 @@ struct BlockState {  // per block scratch (device)
 // additions inside one binade is a map (parity of k) -> increment of k, two maps in a row are again
 // such a map, and stretches are composed in parallel, exactly.  A stretch is a sub-chunk of kSub elements
 // and a chunk; S of its ends is known beforehand to (n + 16) 2^-52 relative from the compensated
-// prefix sums (Higham, Accuracy and Stability, Sec. 4.2), which decides whether it lies in one binade.
+// prefix sums (Higham, Accuracy and Stability, Sec. 4.2), which decides whether it lies in one binade.  Zero and the
+// subnormal numbers are one more such stretch of whole multiples (e = -1023), in which additions are exact.
 constexpr int kSub = 128;                       // elements per sub-chunk: 16 threads of kPer
 constexpr int kSubs = kChunk / kSub;            // sub-chunks per chunk
 constexpr int kSubThreads = kSub / kPer;
@@ -280,7 +281,7 @@ __device__ __forceinline__ void chunk_maps(const double (&loc)[kPer], double bef
     const double rel = ((double)n + 16.0) * 2.220446049250313e-16;  // twice the bound, in ulps of 2^-53
     const double s0 = lo * (1.0 - rel), s1 = hi * (1.0 + rel);
     const int e0 = (__double2hiint(s0) >> 20) - 1023, e1 = (__double2hiint(s1) >> 20) - 1023;
-    const bool inside = some && e0 == e1 && e0 > -900 && e0 < 1000;
+    const bool inside = some && e0 == e1 && e0 < 1000;
     long long d0 = 0, d1 = 0;
     if (inside) {
         // increments from an even and from an odd k of the same binade, 2^e and 2^e + q (inside a binade an
@@ -517,7 +518,7 @@ __device__ __forceinline__ double seq_walk(const double* wb, uint64_t i0, uint64
     while (pos < n) {
         const int es = exponent_of(S);
         int at = pos;  // the weight to add itself
-        if (es > -900 && es < 1000) {
+        if (es < 1000) {
             const double even = __hiloint2double((es + 1023) << 20, 0), odd = __hiloint2double((es + 1023) << 20, 1);
             long long c0[kOwn], c1[kOwn], d0 = 0, d1 = 0;
 #pragma unroll
@@ -538,7 +539,7 @@ __device__ __forceinline__ double seq_walk(const double* wb, uint64_t i0, uint64
             for (int r = kOwn - 1; r >= 0; --r) {
                 k[r] = before + ((before & 1) ? c1[r] : c0[r]);
                 const int i = lane * kOwn + r;
-                if (i >= pos && i < n && (v[r] >= even || exponent_of(k[r]) != es)) first = r;
+                if (i >= pos && i < n && ((v[r] >= even && even > 0.0) || exponent_of(k[r]) != es)) first = r;
             }
             const unsigned any = __ballot_sync(0xffffffffu, first < kOwn);
             const int who = any ? __ffs(any) - 1 : 31;
