@@ -328,7 +328,7 @@ __device__ __forceinline__ void chunk_maps(const double (&loc)[kPer], double bef
 // 3. per chunk: 53-bit grid TV and sum of squared weights (partial sums), in the located chunk the
 //    element search with its certification, and on request (maps) the sequential CDF's maps.  The three
 //    need the same prefix sums of the chunk's weights.
-__global__ void __launch_bounds__(kThreads)
+__global__ void __launch_bounds__(kThreads, 3)  // (3 of them per SM: 64 blocks of 2^14 take 4 us longer with 2)
 k_chunk(const double* w, int k, const dd* chunk_sum, int nch, const BlockState* state, dcs_draw_result* res, double* part,
         double* sq_part, SeqChunk* chunk_map, SeqMap* sub_map, int maps) {
     let_next_start();
