@@ -13,8 +13,9 @@ import numpy as np
 import torch
 
 from . import _lib
+from .sampling import workspaces
 
-_PARTIALS = 2048  # dcs_overlap's scratch in doubles (16 KiB)
+_PARTIALS = 16384  # bytes of dcs_overlap's partial sums
 
 
 def _dev(v, device):
@@ -33,11 +34,11 @@ def overlap_sums(reference_scaled, approximate_vector, device=None):
     ap = _dev(approximate_vector, device)
     if ref.dim() != 1 or ref.shape != ap.shape or not ref.numel():
         raise ValueError("Need two nonempty full vectors with identical shape")
-    # (a call's own partial sums: calls of other threads and streams may run at the same time)
-    out = torch.empty(4 + _PARTIALS, dtype=torch.float64, device=ref.device)
-    _lib.check(lib.dcs_overlap(_lib.ptr(ref), _lib.ptr(ap), ref.numel(), _lib.ptr(out), _lib.ptr(out) + 32,
-                               torch.cuda.current_stream(ref.device).cuda_stream))
-    rr, aa, re, im = out[:4].cpu().tolist()
+    stream = torch.cuda.current_stream(ref.device).cuda_stream
+    out = torch.empty(4, dtype=torch.float64, device=ref.device)
+    _lib.check(lib.dcs_overlap(_lib.ptr(ref), _lib.ptr(ap), ref.numel(), _lib.ptr(out),
+                               _lib.ptr(workspaces.get(ref.device, stream, _PARTIALS)), stream))
+    rr, aa, re, im = out.cpu().tolist()
     return rr, aa, complex(re, im)
 
 

@@ -24,6 +24,7 @@
 from __future__ import annotations
 
 import hashlib
+import threading
 
 import numpy as np
 import torch
@@ -53,9 +54,28 @@ def straddle_margin(weight_l2, rel_l2=COMPLEX64_REL_L2):
     return min(2.0 * rel_l2, STRADDLE_SIGMAS * 2.0 * rel_l2 * float(np.sqrt(max(weight_l2, 0.0))))
 
 
-def _draw_scratch(lib, k, nblocks, device):
-    """Workspace of one draw (a call's own: draws of other threads and streams may run at the same time)."""
-    return torch.empty(lib.dcs_draw_scratch_bytes(k, nblocks), dtype=torch.uint8, device=device)
+class Workspaces(threading.local):
+    """Scratch memory of library calls, kept per thread and stream: calls of other threads and streams may run at the
+    same time, those of one thread on one stream follow one another.  At most KEEP buffers of KEEP_BYTES a thread
+    are kept, and end with it; larger ones are the call's own."""
+
+    KEEP, KEEP_BYTES = 4, 32 << 20
+
+    def __init__(self):
+        self.buf = {}
+
+    def get(self, device, stream, nbytes):
+        t = self.buf.get((device, stream))
+        if t is None or t.numel() < nbytes:
+            t = torch.empty(nbytes, dtype=torch.uint8, device=device)
+            if nbytes <= self.KEEP_BYTES:
+                if len(self.buf) >= self.KEEP:
+                    self.buf.clear()
+                self.buf[device, stream] = t
+        return t
+
+
+workspaces = Workspaces()
 
 
 def _as_device_blocks(amplitudes, device=None):
@@ -86,8 +106,8 @@ def draw_many(blocks, uniforms, device=None, exact_cdf=False):
     k = n.bit_length() - 1
     u = torch.as_tensor(np.asarray(uniforms, dtype=np.float64).reshape(B), device=v.device)
     res = torch.empty(B * _lib.DRAW_DTYPE.itemsize, dtype=torch.uint8, device=v.device)
-    scratch = _draw_scratch(lib, k, B, v.device)
     stream = torch.cuda.current_stream(v.device).cuda_stream
+    scratch = workspaces.get(v.device, stream, lib.dcs_draw_scratch_bytes(k, B))
     _lib.check(lib.dcs_draw_ex(_lib.ptr(v), k, B, _lib.ptr(u), _lib.DRAW_SEQUENTIAL if exact_cdf else 0,
                                _lib.ptr(scratch), _lib.ptr(res), stream))
     return res.cpu().numpy().view(_lib.DRAW_DTYPE)
@@ -180,7 +200,7 @@ def sample_checked(engine, x_list, uniforms, hashes=True, exact_cdf=False, strad
     outs = [torch.empty((1, 1 << k), dtype=torch.complex128, device=dev) for _ in range(2)]
     res = torch.empty((2, _lib.DRAW_DTYPE.itemsize), dtype=torch.uint8, device=dev)
     flags = torch.zeros((2, engine.items), dtype=torch.int64, device=dev)
-    scratch = _draw_scratch(lib, k, 1, dev)
+    scratch = workspaces.get(dev, stream.cuda_stream, lib.dcs_draw_scratch_bytes(k, 1))
     host_blk = [torch.empty(1 << k, dtype=torch.complex128).pin_memory() if hashes or keep_host_blocks else None
                 for _ in range(2)]
     host_res = [torch.empty(_lib.DRAW_DTYPE.itemsize, dtype=torch.uint8).pin_memory() for _ in range(2)]

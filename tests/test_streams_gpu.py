@@ -89,3 +89,22 @@ def test_draws_on_streams(monkeypatch, exact_cdf):
         draw(0)
     assert abs(rec.seen[-1] - rec.seen[0]) >= rec.lib.dcs_draw_scratch_bytes(14, 2)
     assert repr(_in_streams(draw, 4)) == repr(want)
+
+
+def test_kept_workspaces_are_bounded():
+    import torch
+
+    from dcs245_classical_sampling_b200.sampling import Workspaces
+    ws, dev = Workspaces(), torch.device("cuda", 0)
+    first = ws.get(dev, 1, 1 << 20)
+    assert ws.get(dev, 1, 1 << 10) is first and ws.get(dev, 2, 1 << 10) is not first
+    big = ws.get(dev, 1, ws.KEEP_BYTES + 1)
+    assert big.numel() > ws.KEEP_BYTES and ws.get(dev, 1, 1 << 20) is first
+    for stream in range(3, 20):
+        ws.get(dev, stream, 1 << 10)
+    assert len(ws.buf) <= ws.KEEP
+    seen = []
+    t = threading.Thread(target=lambda: seen.append(ws.get(dev, 19, 1 << 10)))
+    t.start()
+    t.join()
+    assert seen[0] is not ws.get(dev, 19, 1 << 10)
