@@ -776,7 +776,7 @@ class InplaceConditionalBlockGPU:
     def enqueue(self, prep, out, flags=None):
         """Device work for a prepared batch into `out` ((nblocks, 2^k) complex128): contraction of
         every work item, accumulation, tail.  No host synchronisation (except in "plain" mode).
-        flags: optional (self.items,) int64 device tensor that collects the items' scale flags
+        flags: optional (self.items,) integer device tensor that collects the items' scale flags
         (bit 0: a nonfinite table; bit 3: see out_of_range).  Returns the number of library kernel
         launches.
 
@@ -821,9 +821,11 @@ class InplaceConditionalBlockGPU:
                 _lib.ptr(self.maxbits) + 8 * (nm - 1), nm, _lib.ptr(out) + (b0 << (self.k + 4)), self.k, cn, fresh, st))
             launches += 2
             if flags is not None:
-                if flags.dtype != torch.int64 or not flags.is_cuda or not flags.is_contiguous() or flags.numel() < cn:
-                    raise ValueError("flags must be a contiguous int64 device tensor of engine.items elements")
-                _lib.check(lib.dcs_collect_flags(_lib.ptr(self.scale), _lib.ptr(flags), cn, st))
+                if (flags.dtype == torch.int64 and flags.device == out.device and flags.dim() == 1 and flags.is_contiguous()
+                        and flags.numel() >= cn):
+                    _lib.check(lib.dcs_collect_flags(_lib.ptr(self.scale), _lib.ptr(flags), cn, st))
+                else:  # strided, or of another integer type
+                    flags[:cn] |= self._sc()[:cn, 2] & 0xffffffff  # (the word's other half is table_exp)
                 launches += 1
         _lib.check(lib.dcs_block_tail(_lib.ptr(out), self.k, self.adj_hi.ctypes.data, self.u_open.ctypes.data,
                                       prep["nblocks"], st))
