@@ -801,9 +801,13 @@ class InplaceConditionalBlockGPU:
         nm = self._nmax() + 1
         entry = _lib.PARAM_DTYPE.itemsize
         launches = 0
-        # one chunk that holds every block writes the blocks; several add to zeroed ones
         chunks = prep["chunks"]
-        fresh = _lib.ACCUMULATE_FRESH if len(chunks) == 1 and chunks[0][2:4] == (0, prep["nblocks"]) else 0
+        if chunks:
+            out.view(torch.float64)  # refuses entries that do not follow one another
+        # one chunk that holds every block writes the blocks; several add to zeroed ones (as do fewer blocks than `out`
+        # has room for: the rest is zero)
+        fresh = (_lib.ACCUMULATE_FRESH if len(chunks) == 1 and chunks[0][2:4] == (0, prep["nblocks"])
+                 and out.numel() == prep["nblocks"] << self.k else 0)
         if not fresh:
             out.zero_()
         d_params, d_coefs, d_xors, d_begin = (_lib.ptr(prep[k]) for k in ("params", "coefs", "xors", "begin"))

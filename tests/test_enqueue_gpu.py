@@ -47,3 +47,23 @@ def test_forms_of_the_flags(items):
         assert torch.equal(flags[:items].long(), want), flags.dtype
     with pytest.raises(Exception):
         eng.enqueue(prep, out, torch.zeros(items - 2, dtype=torch.int64, device="cuda"))
+
+
+@pytest.mark.parametrize("items", [4, 1])
+def test_forms_of_the_blocks(items):
+    import torch
+    eng, xs = _engine(items)
+    n = 1 << eng.k
+    want = eng.block(xs[0])[0].cpu().numpy()
+    prep = eng.prepare([xs[0]])
+    roomy = torch.full((3, n), 7.0, dtype=torch.complex128, device="cuda")
+    eng.enqueue(prep, roomy, eng._flags_tensor())  # the rows that the batch does not have are zero
+    assert np.array_equal(roomy[0].cpu().numpy(), want) and not roomy[1:].cpu().numpy().any()
+    flat = torch.full((1, 2 * n), 7.0, dtype=torch.float64, device="cuda")
+    eng.enqueue(prep, flat, eng._flags_tensor())
+    assert np.array_equal(torch.view_as_complex(flat.view(n, 2)).cpu().numpy(), want)
+    strided = torch.zeros((1, 2 * n), dtype=torch.complex128, device="cuda")
+    with pytest.raises(RuntimeError):
+        eng.enqueue(prep, strided[:, ::2], eng._flags_tensor())
+    torch.cuda.synchronize()
+    assert not strided.cpu().numpy().any()
