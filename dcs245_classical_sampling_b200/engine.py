@@ -28,6 +28,7 @@ offset bits), vectorised over slices; the device does every pass over the tables
 """
 from __future__ import annotations
 
+import functools
 import itertools
 import math
 import time
@@ -94,13 +95,18 @@ def device_steps(steps):
 FLAG_RANGE = 8  # scale flag: a table's maximum left the range of its square (see out_of_range)
 
 
+def flags_seen(flags):
+    """The union of items' flags (an array, or a union already)."""
+    return flags if isinstance(flags, int) else int(np.bitwise_or.reduce(np.asarray(flags).reshape(-1)))
+
+
 def raise_for_flags(flags):
     """The errors an item's scale flags report: bit 2, a generated kernel's bounded wait between
     tiles gave up (the block is invalid); bit 0, a nonfinite table (the reference's error)."""
-    flags = np.asarray(flags)
-    if np.any(flags & 4):
+    seen = flags_seen(flags)
+    if seen & 4:
         raise RuntimeError("a group kernel's wait between tiles gave up; the block is invalid")
-    if np.any(flags & 1):
+    if seen & 1:
         raise ArithmeticError("Nonfinite in-place environment")
 
 
@@ -209,6 +215,7 @@ class DeviceCircuit:
     """Static tables of one circuit for dcs_build_items (from the engine's host bookkeeping)."""
 
     MAX_QUBITS = 64  # dcs_build_items takes a prefix as a 64-bit mask
+    MAX_FIXED = 4096  # fixed steps that it holds
 
     def __init__(self, engine, device):
         sp = engine.params
@@ -237,24 +244,12 @@ class DeviceCircuit:
             for t in np.flatnonzero(sp.F[a]):
                 F[a, t >> 5] |= np.uint32(1 << (t & 31))
         tail = np.array([int(x) for x in sp.tail] + [0], np.uint64)
-        # slices: x-independent coefficients (slices are reference vertices) and flips
-        _, items = sp.items(np.zeros(p.n, np.uint8))
-        # items skip zero coefficients; recover each kept slice's flips from its bits
-        flips, coefs, freeflips = [], [], []
-        ff = ffull_ref
-        for bits in itertools.product((0, 1), repeat=sp.nslice):
-            bits = np.array(bits, np.int64)
-            coef = complex(np.prod([ff[s][b] for s, b in zip(p.slices, bits)])) if sp.nslice else 1 + 0j
-            par = sum(int(bits[p.slices.index(a)]) * int(bits[p.slices.index(b)]) for a, b in p.slice_edges)
-            coef *= (-1) ** par
-            if not coef:
-                continue
-            fl = (bits @ sp.nbr) & 1 if sp.nslice else np.zeros(p.N, np.int64)
-            flips.append(fl[sp.vert].astype(np.uint8))
-            coefs.append(coef)
-            freeflips.append(sum(int(fl[q]) << jj for jj, q in enumerate(sp.open_red)))
+        kept, coefs = self.slice_coefs(sp, ffull_ref)
+        flips = slice_flips(sp)[kept]
+        self._flips = flips[:, sp.vert]
+        freeflips = (flips[:, sp.open_red].astype(np.uint64) << np.arange(len(sp.open_red), dtype=np.uint64)).sum(
+            axis=1, dtype=np.uint64)
         self.nslices = len(coefs)
-        assert self.nslices == len(items)
         # the plan-specialised kernels divide f0 out of the free steps' weights: every weight row
         # a prefix can select (slices flip only f1) must pass the engine's check
         rows = np.zeros(2 * S, _lib.PARAM_DTYPE)
@@ -268,23 +263,48 @@ class DeviceCircuit:
         self.fsel = dev(fsel)
         self.xq = dev(xq)
         self.fixidx = dev(fixidx)
-        self.flip = dev(np.stack(flips).astype(np.uint8))
-        # the same for items with the bits of the host bookkeeping: a zero's sign decides between a step
-        # factor's argument and one 2 pi away
-        self.flip_host = self.flip | 0x80
+        self._dev = dev
         self.F = dev(F)
         self.tail = dev(tail.view(np.int64))
         self.coef = dev(np.array([[c.real, c.imag] for c in coefs], np.float64).reshape(-1))
-        self.freeflip = dev(np.array(freeflips, np.uint64).view(np.int64))
+        self.freeflip = dev(freeflips.view(np.int64))
         self.closed = dev(np.array([q for q in range(p.n) if q not in set(p.open_full)], np.int32))
+
+    @functools.cached_property
+    def flip(self):
+        """1 where a slice flips a step's vertex."""
+        return self._dev(self._flips)
+
+    @functools.cached_property
+    def flip_host(self):
+        """The same for items with the bits of the host bookkeeping: a zero's sign decides between a step factor's
+        argument and one 2 pi away."""
+        return self._dev(self._flips | 0x80)
+
+    @staticmethod
+    def slice_coefs(sp, f):
+        """Indices and coefficients of the slices whose coefficient is not zero, as SliceParams.items makes them
+        (they are reference vertices: f, the local vectors, are the same for every prefix)."""
+        p = sp.plan
+        edges = [(p.slices.index(a), p.slices.index(b)) for a, b in p.slice_edges]
+        kept, coefs = [], []
+        for idx, bits in enumerate(itertools.product((0, 1), repeat=sp.nslice)):
+            coef = complex(np.prod([f[s][b] for s, b in zip(p.slices, bits)])) if sp.nslice else 1 + 0j
+            coef *= (-1) ** sum(bits[a] * bits[b] for a, b in edges)
+            if coef:
+                kept.append(idx)
+                coefs.append(coef)
+        return np.array(kept, np.int64), coefs
 
     @classmethod
     def of(cls, engine):
         """The tables of an engine's circuit, or None where dcs_build_items cannot build its items: more
-        qubits than a mask has bits, or no slice with a nonzero coefficient."""
-        if engine.n > cls.MAX_QUBITS or not engine.params.nsteps:
+        qubits than a mask has bits, more fixed steps than it takes, or no slice with a nonzero coefficient."""
+        sp = engine.params
+        if engine.n > cls.MAX_QUBITS or not sp.nsteps or len(sp.fixed_pos) > cls.MAX_FIXED:
             return None
-        return cls(engine, engine.device) if engine.params.items(np.zeros(engine.n, np.uint8))[1] else None
+        dc = cls(engine, engine.device)
+        return dc if dc.nslices else None
 
     def build(self, lib, xbits, nsamples, params, coefs, xors, stream, flip=None):
         _lib.check(lib.dcs_build_items(
@@ -292,6 +312,38 @@ class DeviceCircuit:
             _lib.ptr(self.flip if flip is None else flip), _lib.ptr(self.F),
             _lib.ptr(self.tail), _lib.ptr(self.coef), _lib.ptr(self.freeflip), self.nsteps, self.nfixed,
             self.nslices, _lib.ptr(xbits), nsamples, _lib.ptr(params), _lib.ptr(coefs), _lib.ptr(xors), stream))
+
+
+def slice_flips(sp):
+    """(2^slices, vertices) uint8: whether a slice, in the order of SliceParams.items, flips a vertex."""
+    flips = np.zeros((1, sp.plan.N), np.uint8)
+    for row in sp.nbr:
+        flips = np.stack([flips, flips ^ row], axis=1).reshape(-1, sp.plan.N)
+    return flips
+
+
+class DeviceItems:
+    """The device tables of an engine's work items (`dc`; None: the host builds the items), made when a call first
+    wants them: alloc need not walk the slices for a worker that evaluates one part of many."""
+
+    _dc = None
+    _dc_pending = False
+
+    @property
+    def dc(self):
+        if self._dc_pending:
+            self.dc = DeviceCircuit.of(self)
+        return self._dc
+
+    @dc.setter
+    def dc(self, value):
+        self._dc, self._dc_pending = value, False
+
+    def _plan_items(self):
+        """After alloc: make the tables at once if that is quick, else at the first whole batch."""
+        self._dc, self._dc_pending = None, True
+        if len(self.slices) <= 4:
+            self.dc  # noqa: B018
 
 
 def prefix_masks(x_list, n):
@@ -325,7 +377,8 @@ def item_chunks(nblocks, nslices, cap):
 def device_batch(engine, masks):
     """The work items of whole prefixes (masks), built on the device by dcs_build_items: one upload of the
     masks and the chunks' block ranges, no host work per item."""
-    B, L = len(masks), engine.dc.nslices
+    dc = engine.dc
+    B, L = len(masks), dc.nslices
     n = B * L
     chunks, begins = item_chunks(B, L, engine.items)
     words = (len(begins) + 1) // 2
@@ -333,12 +386,12 @@ def device_batch(engine, masks):
     host = pinned.numpy()
     host[:B] = masks.view(np.int64)
     host[B:].view(np.int32)[:len(begins)] = begins
-    o1 = n * engine.dc.nsteps * (_lib.PARAM_DTYPE.itemsize // 8)
+    o1 = n * dc.nsteps * (_lib.PARAM_DTYPE.itemsize // 8)
     o2, o3 = o1 + 2 * n, o1 + 3 * n
     dev = torch.empty(o3 + B + words, dtype=torch.int64, device=engine.device)
     dev[o3:].copy_(pinned, non_blocking=True)
     params, coefs, xors = dev[:o1], dev[o1:o2].view(torch.float64), dev[o2:o3]
-    engine.dc.build(engine.lib, dev[o3:], B, params, coefs, xors, engine._stream(), engine.dc.flip_host)
+    dc.build(engine.lib, dev[o3:], B, params, coefs, xors, engine._stream(), dc.flip_host)
     return {"n_items": n, "chunks": chunks, "unit_ok": [True] * len(chunks),
             "counts": [1 << len(engine.plan.slices)] * B, "nblocks": B, "dev": dev, "pinned": pinned,
             "params": params, "coefs": coefs, "xors": xors, "begin": dev[o3 + B:].view(torch.int32),
@@ -359,7 +412,7 @@ class DeviceBlock(torch.Tensor):
         return host if dtype is None else host.astype(dtype, copy=False)
 
 
-class InplaceConditionalBlockGPU:
+class InplaceConditionalBlockGPU(DeviceItems):
     """Drop-in for the reference engine of the same name (see module docstring)."""
 
     half = False  # binary16 tables (alloc)
@@ -501,7 +554,7 @@ class InplaceConditionalBlockGPU:
             u[q] = [m[0, 0].real, m[0, 0].imag, m[0, 1].real, m[0, 1].imag,
                     m[1, 0].real, m[1, 0].imag, m[1, 1].real, m[1, 1].imag]
         self.u_open = u
-        self.dc = DeviceCircuit.of(self)
+        self._plan_items()
         self._alloc = True
         self.buf = True
 
@@ -789,7 +842,7 @@ class InplaceConditionalBlockGPU:
         single_steps(prep): its entries cancelled so far inside a group that the squares of a maximum left
         the storage precision's range."""
         return (self.tplan is not None and not self.half and any(prep["unit_ok"])
-                and bool(np.any(np.asarray(flags) & FLAG_RANGE)))
+                and bool(flags_seen(flags) & FLAG_RANGE))
 
     @staticmethod
     def single_steps(prep):
@@ -856,6 +909,7 @@ class InplaceConditionalBlockGPU:
                 seen = self.scale[: cn * _SCALE_WORDS].cpu().numpy().view(_lib.SCALE_DTYPE)["flags"]
             else:
                 seen = flags.cpu().numpy()
+            seen = flags_seen(seen)
             if not self.out_of_range(prep, seen):
                 break
             prep = self.single_steps(prep)

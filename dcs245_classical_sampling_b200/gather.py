@@ -21,11 +21,11 @@ import numpy as np
 import torch
 
 from . import _lib
-from .engine import DeviceBlock, DeviceCircuit, SliceParams, device_batch, pack_runs, prefix_masks
+from .engine import DeviceBlock, DeviceItems, SliceParams, device_batch, pack_runs, prefix_masks
 from .plan import build_block_plan, build_gather_plan
 
 
-class ConditionalBlockGPU:
+class ConditionalBlockGPU(DeviceItems):
     """Drop-in for the reference's gather engine (see the module docstring)."""
 
     def __init__(self, graph, unitaries, n, order, parity_operations, open_vertices):
@@ -89,8 +89,6 @@ class ConditionalBlockGPU:
         self.nm = S + 1
         self.maxbits = torch.zeros(self.items * self.nm, dtype=torch.int64, device=self.device)
         self.scale = torch.zeros(self.items * _lib.SCALE_DTYPE.itemsize // 8, dtype=torch.int64, device=self.device)
-        self.one_bits = (int(np.array([1.0], np.float64).view(np.int64)[0]) if self.use_fp64
-                         else int(np.array([1.0], np.float32).view(np.uint32)[0]))
         self.term_runs, self.term_nruns = pack_runs(list(range(self.terminal_rank)))
         self.tbasis = np.array(self.terminal_basis + [0], dtype=np.uint64)
         adj = np.zeros(max(1, self.k), dtype=np.uint32)
@@ -104,7 +102,7 @@ class ConditionalBlockGPU:
             u[q] = [m[0, 0].real, m[0, 0].imag, m[0, 1].real, m[0, 1].imag,
                     m[1, 0].real, m[1, 0].imag, m[1, 1].real, m[1, 1].imag]
         self.u_open = u
-        self.dc = DeviceCircuit.of(self)
+        self._plan_items()
         self._alloc = True
 
     def weights_ok(self, params, any_row=False):

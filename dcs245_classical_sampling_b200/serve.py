@@ -155,6 +155,7 @@ class CircuitRunner:
         self.lib = _lib.load()
         self.dc = self.engine.dc or DeviceCircuit(self.engine, self.device)
         assert self.dc.nslices == L
+        self.dc.flip  # uploaded before the first batch  # noqa: B018
         if self.mode == "fused" and self.engine.jit and not self.dc.unit_ok:
             self.engine.set_fused_config(jit=False)  # weights the plan-specialised kernels cannot take
         self.max_samples = max_samples if self.mode == "fused" else max(1, min(max_samples, items // L) or 1)
