@@ -87,3 +87,28 @@ def test_tiny_weights_cost_no_walk():
             torch.cuda.synchronize()
         times.append(t0.elapsed_time(t1))
     assert max(times) < 8 * times[0] + 1.0  # (milliseconds; one by one: 33 against 0.1)
+
+
+@pytest.mark.parametrize("k", [4, 11, 14, 17])
+def test_ties_are_decided_as_the_reference_does(k):
+    """u on an edge of numpy's CDF, and one place beside it: numpy's index where the reference's compensated check
+    accepts it, an error where it does not, by a sequential pass that makes its maps itself."""
+    import torch
+
+    from dcs245_classical_sampling_b200.sampling import draw_many
+    rng = np.random.default_rng(k)
+    v = rng.standard_normal(1 << k) + 1j * rng.standard_normal(1 << k)
+    w = v.real * v.real + v.imag * v.imag
+    cdf = np.cumsum(w) / np.cumsum(w)[-1]
+    accepted = 0
+    for at in (0.1, 0.4, 0.7):
+        edge = cdf[int(at * len(v))]
+        for u in (edge, np.nextafter(edge, 0), np.nextafter(edge, 1)):
+            sums, want, i, ok = _reference(w, u)
+            r = draw_many(torch.from_numpy(v).cuda(), [u])[0]
+            assert r["tie"] and float(r["total_cdf"]) == float(sums[-1])
+            assert (r["status"] == 0) == ok
+            if ok:
+                assert (int(r["index"]), float(r["cdf_upper"])) == (i, float(want[i]))
+            accepted += ok
+    assert accepted

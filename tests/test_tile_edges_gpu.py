@@ -222,3 +222,38 @@ def test_overflow_in_the_last_step_shows_in_the_block(storage, weight):
     else:  # entries whose squares are infinite: the block itself is right
         want = _engine(A, U, n, order, opened, dtype=np.complex128).blocks(list(xs)).cpu().numpy()
         assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("w", [[300.0, 200.0], [1e-3, 2e-3], [2.0 ** 20, 1.0]])
+def test_weights_outside_the_range(w):
+    """Bras that tile groups do not take: single steps, and the block of complex128 tables."""
+    A, U, n, order, opened = _with_isolated((18, 20, 60, 7), 0.5, [])
+    x = np.random.default_rng(2).integers(0, 2, n).astype(np.uint8)
+    eng = _engine(A, U, n, order, opened)
+    assert not any(eng.prepare([x], np.array(w))["unit_ok"])
+    got = eng.block(x, np.array(w))[0].cpu().numpy()
+    ref = _engine(A, U, n, order, opened, dtype=np.complex128)
+    ref.tplan = None
+    want = ref.block(x, np.array(w))[0].cpu().numpy()
+    if w[0] == 2.0 ** 20:  # the amplitudes themselves are past the FP64 range
+        assert not np.isfinite(want).any() and not np.isfinite(got).any()
+    else:
+        assert np.linalg.norm(got - want) <= 1e-5 * np.linalg.norm(want)
+
+
+@pytest.mark.parametrize("dtype", [np.complex64, np.complex128])
+@pytest.mark.parametrize("w", [[0.3, 0.125], [0.2, 0.2j], [2.5, 1.5j], [1.0, 1e-3]])
+def test_other_bras_inside_the_range(w, dtype):
+    """Bras other than the default, towards both ends of what tile groups take: one launch per step's bits."""
+    A, U, n, order, opened = _with_isolated((18, 20, 60, 7), 0.5, [])
+    U[n:] = np.eye(2)  # the bras are the references' weights
+    x = np.random.default_rng(2).integers(0, 2, n).astype(np.uint8)
+    eng = _engine(A, U, n, order, opened, dtype=dtype)
+    assert all(eng.prepare([x], np.array(w))["unit_ok"])
+    got = eng.block(x, np.array(w))[0].cpu().numpy()
+    eng.tplan = None
+    want = eng.block(x, np.array(w))[0].cpu().numpy()
+    assert np.linalg.norm(want) > 0
+    if dtype == np.complex64:
+        assert np.array_equal(got, want)
+    assert np.linalg.norm(got - want) <= 1e-12 * np.linalg.norm(want)  # the scale factor's rounding
