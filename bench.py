@@ -347,7 +347,7 @@ def gpu_arm(args):
         if record:
             ev1 = torch.cuda.Event(enable_timing=True)
             ev1.record(stream)
-        return launches + 6, (ev0, ev1)
+        return launches + 4, (ev0, ev1)  # (the draw: weights, chunk scan, chunks, finish)
 
     for i in range(args.warmup):
         one(i)
@@ -683,7 +683,8 @@ def eng_maxslots(w):
 
 def kernel_roofline(eng, prep, out, stream):
     """Average duration and algorithmic bytes of the dominant contraction kernel, from CUDA
-    events around each of its launches (one slice of one sample)."""
+    events around each of its launches (one slice of one sample; device mode: one chunk of its
+    slices, whose tile groups are one call)."""
     import torch
     from dcs245_classical_sampling_b200 import _lib
     lib = eng.lib
@@ -706,7 +707,20 @@ def kernel_roofline(eng, prep, out, stream):
             evs.append((a, b, alg))
         kernel = ("dcs_g (plan-specialised k_runs)" if f.jit is not None else "k_runs") \
             if f.tile_runs is not None and bool((f.groups["variant"] & 4).any()) else "k_fused"
+        spans, launches = f.spans, len(f.groups)
+    elif eng.tplan is not None and prep["unit_ok"][0]:
+        a = torch.cuda.Event(enable_timing=True)
+        b = torch.cuda.Event(enable_timing=True)
+        a.record(stream)
+        eng._run_steps(params_ptr, cn, True, stream.cuda_stream)
+        b.record(stream)
+        entry = 16 if eng.use_fp64 else (4 if eng.half else 8)
+        evs.append((a, b, cn * entry * sum((1 << len(plan.steps[s0].active_in)) + (1 << len(plan.steps[s0 + c - 1].active_out))
+                                           for s0, c in eng.tplan.spans)))
+        kernel = "k_tile_half, k_step (half storage)" if eng.half else "k_tiles"
+        spans, launches = [(0, eng.nsteps)], eng.tile_launches
     else:
+        spans, launches = [(s, 1) for s in range(eng.nsteps)], eng.nsteps
         for s in range(eng.nsteps):
             a = torch.cuda.Event(enable_timing=True)
             b = torch.cuda.Event(enable_timing=True)
@@ -718,20 +732,19 @@ def kernel_roofline(eng, prep, out, stream):
             b.record(stream)
             st = plan.steps[s]
             entry = 16 if eng.use_fp64 else (4 if eng.half else 8)
-            evs.append((a, b, ((1 << len(st.active_in)) + (1 << len(st.active_out))) * entry))
+            evs.append((a, b, ((1 << len(st.active_in)) + (1 << len(st.active_out))) * entry * cn))
         kernel = "k_step"
     torch.cuda.synchronize()
     tot_t = sum(a.elapsed_time(b) for a, b, _ in evs) / 1000.0
     tot_b = sum(x for _, _, x in evs)
-    n = len(evs)
+    items = 1 if eng.mode == "fused" else cn
     # entry-steps of each launch: every vertex step touches 2^max(|in|, |out|) table entries
-    spans = eng.fplan.spans if eng.mode == "fused" else [(s, 1) for s in range(eng.nsteps)]
-    entry_steps = [sum(1 << max(len(st.active_in), len(st.active_out)) for st in plan.steps[f0:f0 + c])
+    entry_steps = [items * sum(1 << max(len(st.active_in), len(st.active_out)) for st in plan.steps[f0:f0 + c])
                    for f0, c in spans]
     prm = prep["params"][:eng.nsteps * _lib.PARAM_DTYPE.itemsize // 8].cpu().numpy().view(_lib.PARAM_DTYPE)
-    ops = [sum(step_fp32_ops(st, int(prm[f0 + i]["y"])) for i, st in enumerate(plan.steps[f0:f0 + c]))
+    ops = [items * sum(step_fp32_ops(st, int(prm[f0 + i]["y"])) for i, st in enumerate(plan.steps[f0:f0 + c]))
            for f0, c in spans]
-    return {"kernel": kernel, "launches": n, "avg_launch_s": tot_t / n, "alg_bytes_per_launch": tot_b / n,
+    return {"kernel": kernel, "launches": launches, "avg_launch_s": tot_t / launches, "alg_bytes_per_launch": tot_b / launches,
             "launch_ms": [a.elapsed_time(b) for a, b, _ in evs], "launch_bytes": [x for _, _, x in evs],
             "launch_entry_steps": entry_steps, "launch_fp32_ops": ops}
 
@@ -923,7 +936,9 @@ def profile_case(argv):
 
     ap = argparse.ArgumentParser(prog="bench.py --profile-case")
     ap.add_argument("--workload", default="ring64_d73_t314_k20")
-    ap.add_argument("--mode", default="fused", choices=["fused", "device"])
+    ap.add_argument("--mode", default="fused", choices=["fused", "device", "tiles"],
+                    help="groups of the fused plan, a launch per step, or device mode's tile groups")
+    ap.add_argument("--items", type=int, default=1, help="tiles: work items in the batch (copies of one slice)")
     ap.add_argument("--max-slots", type=int, default=28)
     ap.add_argument("--iters", type=int, default=3)
     ap.add_argument("--max-dim", type=int, default=13)
@@ -967,6 +982,9 @@ def profile_case(argv):
     if a.fp64 and (a.mode != "fused" or not a.jit or half):
         raise SystemExit("--fp64 takes --mode fused --jit (the complex128 generated kernels)")
     entry = 4 if half else (16 if a.fp64 else 8)
+    if a.mode == "tiles":
+        profile_tiles(a, lib, P.BlockPlan(**{**bp.__dict__, "steps": steps}), params)
+        return
     if half:
         table = torch.zeros(2 << a.max_slots, dtype=torch.float16, device=dev)
     else:
@@ -1036,6 +1054,34 @@ def profile_case(argv):
                       "alg_gb": tot_b / 1e9, "alg_gbs": tot_b / tot_ms / 1e6,
                       "big_launch_gbs": (sum(b for _, b in big) / sum(t for t, _ in big) / 1e6) if big else None,
                       "per_launch_ms": [round(t, 3) for t, _ in per_launch]}))
+
+
+def profile_tiles(a, lib, plan, params):
+    """The tile groups of a plan (complex64) on --items copies of one slice, --iters times."""
+    import torch
+    from dcs245_classical_sampling_b200 import _lib
+    from dcs245_classical_sampling_b200.engine import TILE_STEPS, device_steps, tile_dim
+    from dcs245_classical_sampling_b200.fused import build_fused_plan
+    slots = max(max(st.active_in + st.active_out + (st.pivot if st.kind == "grow" else 0,)) for st in plan.steps) + 1
+    fp = build_fused_plan(plan, max_dim=tile_dim(slots), low=3, max_steps=TILE_STEPS)
+    n, m = len(plan.steps), a.items
+    dsteps = device_steps(plan.steps)
+    table = torch.zeros(m << slots, dtype=torch.complex64, device="cuda")
+    maxbits = torch.zeros(m * (n + 1), dtype=torch.int64, device="cuda")
+    scale = torch.zeros(m * _lib.SCALE_DTYPE.itemsize // 8, dtype=torch.int64, device="cuda")
+    prm = params.repeat(m)
+    st = torch.cuda.current_stream().cuda_stream
+    e0, e1 = (torch.cuda.Event(enable_timing=True) for _ in range(2))
+    for _ in range(a.iters):
+        e0.record()
+        _lib.check(lib.dcs_begin_items(_lib.C64, _lib.ptr(table), 1 << slots, _lib.ptr(maxbits), n + 1, _lib.ptr(scale), m, st))
+        _lib.check(lib.dcs_tile_groups(_lib.C64, _lib.ptr(table), 1 << slots, dsteps.ctypes.data, n, fp.groups.ctypes.data,
+                                       len(fp.groups), fp.tile_steps.ctypes.data, _lib.ptr(prm), n, _lib.ptr(maxbits), n + 1,
+                                       _lib.ptr(scale), m, st))
+        e1.record()
+        torch.cuda.synchronize()
+    print(json.dumps({"mode": "tiles", "items": m, "steps": n, "launches": len(fp.groups), "spans": fp.spans,
+                      "tile_dims": fp.dims, "slots": slots, "total_ms": e0.elapsed_time(e1)}))
 
 
 def main():

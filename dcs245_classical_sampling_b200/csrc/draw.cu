@@ -601,10 +601,11 @@ __device__ __forceinline__ double seq_chunk(const double* wb, uint64_t n, uint64
 //    chunks by scanning their maps; chunks that cross a binade (about log2 of the block size of them) go through
 //    their sub-chunks' maps, and the one or two sub-chunks that cross through their weights'.
 //    The chain of n dependent additions this replaces took 10.9 ms for 2^20 weights; chunk by chunk, with
-//    dependent additions in the sub-chunks that cross, the kernel took 93 us, so 53.  The selected chunk (and sub-chunk) is the last one whose
-//    starting value satisfies fl(start / S_n) <= u (fl(x / S_n) is non-decreasing in x), and only the
-//    selected sub-chunk is replayed.  The compensated interval of the selected index is checked
-//    against u as the reference's independent check does (sampling_protocol.py:67-72).
+//    dependent additions in the sub-chunks that cross, the kernel took 93 us, and by runs and scans 53.  The
+//    selected chunk (and sub-chunk) is the last one whose starting value satisfies fl(start / S_n) <= u
+//    (fl(x / S_n) is non-decreasing in x), and only the selected sub-chunk is replayed.  The compensated
+//    interval of the selected index is checked against u as the reference's independent check does
+//    (sampling_protocol.py:67-72).
 __global__ void __launch_bounds__(kThreads)
 k_finish(const double* w, int k, const dd* chunk_sum, int nch, const BlockState* state, dcs_draw_result* res,
          const double* part, const double* sq_part, SeqChunk* chunk_map, SeqMap* sub_map, int force) {

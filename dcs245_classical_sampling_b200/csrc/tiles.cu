@@ -9,8 +9,8 @@
 // next one for each of the 30 to 400 steps of a plan, and most plans' tables are so small that the
 // launch and the gap are most of it.
 //
-// Bound: instruction issue (72% of the issue slots on 2048 tiles of 2^12 entries, 22 instructions per entry
-// and step); with a tile per SM or less, the latency of a step (two shared-memory accesses, the
+// Bound: instruction issue (68% of the issue slots on 16 items of 1024 tiles of 2^12 entries, 22 instructions per
+// active entry and step); with a tile per SM or less, the latency of a step (two shared-memory accesses, the
 // products and a barrier).  A slice, device work and enqueueing, against one launch per step: 40 qubits (2^22
 // entries, 213 steps in 13 groups) 911 -> 281 us, 48 qubits (2^24) 1414 -> 560 us, in complex128 2044 ->
 // 703 us; 16 slices of 40 qubits in one batch 4545 -> 1563 us.
