@@ -43,7 +43,9 @@ template <class S> struct Mem<S, S> {
     static __device__ __forceinline__ S ld(const S& m) { return m; }
     static __device__ __forceinline__ Q st(S* E, uint64_t c, S v) {
         E[c] = v;
-        return v.x * v.x + v.y * v.y;
+        // (rounded alike in every kernel: the maxima of complex64 tables decide the exponents)
+        if constexpr (sizeof(Q) == 4) return __fmaf_rn(v.x, v.x, __fmul_rn(v.y, v.y));
+        else return v.x * v.x + v.y * v.y;
     }
 };
 template <> struct Mem<double2, ushort2> {

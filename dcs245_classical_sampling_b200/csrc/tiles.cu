@@ -77,6 +77,10 @@ template <class S, class R> __device__ __forceinline__ S zaddg(S a, R g, S b) { 
 template <class S> __device__ __forceinline__ S zmul(S f, S x) {
     return c2(rfma(f.x, x.x, -rmul(f.y, x.y)), rfma(f.y, x.x, rmul(f.x, x.y)));
 }
+// the same for a fixed step without a sum, whose product k_step rounds the other way round in the imaginary part
+template <class S> __device__ __forceinline__ S zmulf(S f, S x) {
+    return c2(rfma(f.x, x.x, -rmul(f.y, x.y)), rfma(f.x, x.y, rmul(f.y, x.x)));
+}
 
 template <class S> struct Weights {
     S f0, f1, fp, fm;  // f0 + f1, f0 - f1
@@ -159,7 +163,7 @@ __device__ __forceinline__ typename Mem<S, M>::Q run_step(unsigned char* __restr
             stv(t, zmul(f0, zadd(a, b)));
             stv(t ^ tK, flip(zmul(f1, zaddg(a, gK, b)), x & kSign));
         } else if constexpr (KIND == DCS_KIND_FIXED) {
-            stv(t, flip(zmul(fy, a), x & my));
+            stv(t, flip(zmulf(fy, a), x & my));
         } else if constexpr (KIND == DCS_KIND_FIXED_SHRINK) {
             const S b = ld(t ^ tK);
             stv(t, flip(zmul(fy, zaddg(a, gy, b)), x & my));
