@@ -169,14 +169,22 @@ def test_checked_samples_and_enqueue_of_small_products(monkeypatch):
     assert eng.out_of_range(prep, flags.cpu().numpy())
 
 
-@pytest.mark.parametrize("graphs", [False, True])
-def test_served_samples_of_small_products(graphs):
+@pytest.mark.parametrize("tables", ["owned", "graphs", "pool"])
+def test_served_samples_of_small_products(tables):
     from dcs245_classical_sampling_b200.sampling import draw_many
-    from dcs245_classical_sampling_b200.serve import CircuitRunner, Request, Server
+    from dcs245_classical_sampling_b200.serve import CircuitRunner, Request, Server, TablePool
     A, U, n, order, opened = _with_isolated((14, 15, 50, 5), 0.5, [SMALL] * 20)
     w = {"graph": A, "unitaries": U, "n": n, "order": order, "parity_operations": [], "open_vertices": opened}
-    run = CircuitRunner("c", w, 11, 4, graphs=graphs)
-    reqs = Server({"c": run}).run([Request(i, "c", 3, 0.0) for i in range(4)], realtime=False)
+    pool = TablePool(1 << 20, "cuda:0") if tables == "pool" else None
+    run = CircuitRunner("c", w, 11, 4, graphs=tables == "graphs", pool=pool)
+    again, launch = [], run.launch
+
+    def spy(samples, region=(), tiles=None):
+        again.extend([1] if tiles is False else [])
+        return launch(samples, region, tiles)
+    run.launch = spy
+    reqs = Server({"c": run}, pool).run([Request(i, "c", 3, 0.0) for i in range(4)], realtime=False)
+    assert again and (pool is None or pool.free_bytes() == pool.nbytes)
     ref = _engine(A, U, n, order, opened, dtype=np.complex128)
     for r in reqs:
         for i in range(3):
